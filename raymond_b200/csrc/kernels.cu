@@ -305,6 +305,20 @@ __global__ void k_envmap_normalize(const float *sum, float *pdfs, uint32_t gridS
     pdfs[i] *= scale;
 }
 
+// Clears *uniform if the map is not uniform: a texel of `pdfs` that differs
+// from the first, or a probability of the pyramid (the quads from the second
+// level on) other than 1/4.
+__global__ void k_envmap_uniform(const float *pdfs, uint32_t numPdfs, const float *quads, uint32_t numQuadFloats,
+                                 int *uniform) {
+    const float first = pdfs[0];
+    bool same = true;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < numPdfs; i += gridDim.x * blockDim.x)
+        same = same && pdfs[i] == first;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < numQuadFloats; i += gridDim.x * blockDim.x)
+        same = same && quads[i] == 0.25f;
+    if (!same) *uniform = 0;
+}
+
 // ------------------------------------------------------------- film read-out
 // kernels/utils/normalizeImage.metal:11-59
 __device__ float3 tonemapHablePartial(float3 x) {
@@ -435,6 +449,13 @@ cudaError_t rmdLaunchEnvmapReduce(float *mip, int cur, cudaStream_t s) {
 }
 cudaError_t rmdLaunchEnvmapNormalize(const float *sum, float *pdfs, uint32_t gridSize, cudaStream_t s) {
     k_envmap_normalize<<<(gridSize + 255) / 256, 256, 0, s>>>(sum, pdfs, gridSize);
+    return cudaGetLastError();
+}
+cudaError_t rmdLaunchEnvmapUniform(const float *pdfs, uint32_t numPdfs, const float *quads, uint32_t numQuadFloats,
+                                   int *uniform, cudaStream_t s) {
+    const uint32_t n = std::max(numPdfs, numQuadFloats);
+    k_envmap_uniform<<<std::min<uint32_t>((n + 255) / 256, 148u * 8u), 256, 0, s>>>(pdfs, numPdfs, quads, numQuadFloats,
+                                                                                  uniform);
     return cudaGetLastError();
 }
 cudaError_t rmdLaunchFilmResolve(const float4 *film, const double *film64, int fp64, float *out, uint32_t numPixels,

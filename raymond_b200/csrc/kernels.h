@@ -19,6 +19,9 @@ cudaError_t rmdLaunchTraceShadow(const rmd::WideNode *nodes, const float4 *tris,
                                  rmd::Counters *cnt, uint32_t cur, int blocks, cudaStream_t s);
 cudaError_t rmdLaunchEnvmapReduce(float *mip, int cur, cudaStream_t s);
 cudaError_t rmdLaunchEnvmapNormalize(const float *sum, float *pdfs, uint32_t gridSize, cudaStream_t s);
+// clears *uniform (device, 1 before) unless all texels are equal and all pyramid probabilities are 1/4
+cudaError_t rmdLaunchEnvmapUniform(const float *pdfs, uint32_t numPdfs, const float *quads, uint32_t numQuadFloats,
+                                   int *uniform, cudaStream_t s);
 cudaError_t rmdLaunchFilmResolve(const float4 *film, const double *film64, int fp64, float *out, uint32_t numPixels,
                                  float exposure, float divisor, uint32_t tonemapping, uint32_t channels,
                                  cudaStream_t s);

@@ -334,13 +334,18 @@ rmd_status buildEnvironmentMap(rmd_scene *s, int exponent) {
     const int res = 1 << exponent;
     size_t mipSize = 0;
     for (int e = 0; e <= exponent; e++) mipSize += (size_t)1 << (2 * e);
-    RMD_CUDA(s->envMipmap.alloc(mipSize * sizeof(float)));
+    // three floats ahead of the one-texel level put every later level on 16 bytes (worldLightSample loads quads);
+    // the uniformity flag follows the last level
+    constexpr size_t lead = 3;
+    RMD_CUDA(s->envMipmap.alloc((lead + mipSize + 1) * sizeof(float)));
     RMD_CUDA(s->envPdfs.alloc((size_t)res * res * sizeof(float)));
+    float *mip = s->envMipmap.as<float>() + lead;
     s->dctx.envResolution = res;
-    s->dctx.envMipmap = s->envMipmap.as<float>();
+    s->dctx.envUniform = 0;
+    s->dctx.envMipmap = mip;
     s->dctx.envPdfs = s->envPdfs.as<float>();
     const size_t lastLevel = mipSize - (size_t)res * res;
-    float *finest = s->envMipmap.as<float>() + lastLevel;
+    float *finest = mip + lastLevel;
     float *pdfs = s->envPdfs.as<float>();
     void *args[] = {&s->dctx, &finest, &pdfs, (void *)&res};
     dim3 b(8, 8), g((res + 7) / 8, (res + 7) / 8);
@@ -349,10 +354,16 @@ rmd_status buildEnvironmentMap(rmd_scene *s, int exponent) {
     for (int e = exponent - 1; e >= 0; e--) {
         const int cur = 1 << e;
         off -= (size_t)cur * cur;
-        RMD_CUDA(rmdLaunchEnvmapReduce(s->envMipmap.as<float>() + off, cur, st));
+        RMD_CUDA(rmdLaunchEnvmapReduce(mip + off, cur, st));
     }
-    RMD_CUDA(rmdLaunchEnvmapNormalize(s->envMipmap.as<float>(), pdfs, (uint32_t)res * (uint32_t)res, st));
+    RMD_CUDA(rmdLaunchEnvmapNormalize(mip, pdfs, (uint32_t)res * (uint32_t)res, st));
+    int *flag = reinterpret_cast<int *>(mip + mipSize);
+    int uniform = 1;
+    RMD_CUDA(cudaMemcpyAsync(flag, &uniform, sizeof(int), cudaMemcpyHostToDevice, st));
+    RMD_CUDA(rmdLaunchEnvmapUniform(pdfs, (uint32_t)res * (uint32_t)res, mip + 1, (uint32_t)(mipSize - 1), flag, st));
+    RMD_CUDA(cudaMemcpyAsync(&uniform, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     RMD_CUDA(cudaStreamSynchronize(st));
+    s->dctx.envUniform = uniform;
     return RMD_OK;
 }
 
