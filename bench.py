@@ -635,7 +635,7 @@ def main():
              "film_regen": (tot["paths"] + 0.0, BYTES_FILM_PER_PATH)}
     n_units, bpu = units[dominant]
     achieved = n_units * bpu / (stage_ms[dominant] / 1e3) / 1e9
-    launches = max(1, tot["iterations"])  # one launch of each stage per iteration
+    launches = max(1, tot["iterations"])  # closest hits and shadow rays share a launch: three launches per iteration
     traffic = TRAFFIC_PER_UNIT[dominant] * n_units / launches if dominant in TRAFFIC_PER_UNIT else None
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     peak = peaks.get("hbm_gbs", 6650.0)
@@ -662,7 +662,7 @@ def main():
                              "frac": seg_rate * BYTES_PER_SEGMENT / 1e9 / peak},
         "e2e": None if args.no_e2e else {"value": e2e_value, "unit": "Mpaths/s", "h2d_bytes_per_step": 64 + 40,
                                          "d2h_bytes_per_step": W * H * 3 * 4},
-        "gpu_launches": int(tot["iterations"] * 4 + args.steps),
+        "gpu_launches": int(tot["iterations"] * 3 + args.steps),
         "frame": {"samples": frame_samples, "ranks": world, "reduce_ms": reduce_s * 1e3,
                   "reduce_bytes": W * H * 16 if world > 1 else 0,
                   "mean_radiance": float(r.film(normalize=True).mean())},

@@ -341,7 +341,9 @@ typedef struct rmd_stats {
     uint64_t shadow_rays;      /* shadow rays traced */
     uint64_t iterations;       /* wavefront iterations of the last render */
     double   ms_total;         /* device time of the last render */
-    double   ms_trace;         /* closest-hit traversal */
+    double   ms_trace;         /* closest-hit traversal; one kernel traces closest hits and shadow rays
+                                  (training renders apart), its time is split by the clocks its warps
+                                  spent on each */
     double   ms_shade;         /* shading, NEE and BSDF sampling */
     double   ms_shadow;        /* any-hit traversal + shadow resolve */
     double   ms_film;          /* film accumulation and path regeneration */
@@ -598,7 +600,7 @@ rmd_status rmd_batch_guide_stats(const rmd_batch *batch, rmd_guide_stats *out);
  * allocation, a real-time loop that must not pay allocation latency, a
  * process held to a fixed memory budget): renders like rmd_render but keeps
  * its path pool, queues and counters in one fixed device array compiled into
- * the library (RMD_NOALLOC_MAX_PATHS paths, about 8.1 MB) and never calls
+ * the library (RMD_NOALLOC_MAX_PATHS paths, about 8.7 MB) and never calls
  * cudaMalloc, cudaFree or any other allocating routine.  The array is
  * reserved on a GPU when the first rmd_context for that GPU is created
  * (rmd_context_create looks up its device address, which loads the module

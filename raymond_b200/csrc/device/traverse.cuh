@@ -342,6 +342,155 @@ RMD_HD bool closestHit(const TraversalState &s, const float4 *__restrict__ tris,
     return true;
 }
 
+// Cooperative form: a group of 8 lanes traces one ray, lane k the child slot
+// k ^ octant of each node (so a ballot lists the entered inner children in
+// visiting order) and the node's triangles k, k + 8 and k + 16.  A step's
+// chain of dependent instructions is about a quarter of traverseStep's, which
+// pays where rays are too few to fill the machine.  Box and triangle tests are
+// those of traverseStep, and the closest hit does not depend on the order of
+// the tests (lowest distance, then instance, then primitive), so the hits are
+// the same.
+//
+// All 32 lanes of a warp call it; each group's lanes pass the same ray (have:
+// whether the group has one) and get the finished state.  `stack`: the warp's
+// 4 x TRAVERSAL_STACK entries in shared memory.
+template <bool ANY>
+__device__ __forceinline__ void traverseGroups(TraversalState &s, bool have, const WideNode *__restrict__ nodes,
+                                               const float4 *__restrict__ tris, float3 o, float3 d, float tmin,
+                                               float tmax, uint2 *stack, uint32_t *errors) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, shift = lane & 24u;
+    stack += (shift >> 3) * TRAVERSAL_STACK;
+    beginTraversal(s, have ? nodes : nullptr, o, d, tmin, tmax);
+    have = s.sp >= 0;
+    const uint32_t octant = rayOctant(s.r.idir), slot = sub ^ octant;
+    // byte offsets of the slot's near planes; the far ones lie at the other of the axis's two
+    const uint32_t offX = ((octant & 1u) ? 56u : 32u) + slot;
+    const uint32_t offY = ((octant & 2u) ? 64u : 40u) + slot;
+    const uint32_t offZ = ((octant & 4u) ? 72u : 48u) + slot;
+    while (__any_sync(FULL, have)) {
+        bool inner = false;
+        uint32_t triHits = 0, triBase = 0;
+        if (have) {
+            const uint32_t key = __ffs(s.group.y >> 24) - 1;
+            s.group.y &= ~(1u << (24u + key));
+            const uint32_t index = s.group.x + __popc(s.group.y & ((1u << (key ^ octant)) - 1u) & 0xffu);
+            if (s.group.y > 0x00ffffffu) {
+                if (s.sp < TRAVERSAL_STACK) {
+                    if (sub == 0) stack[s.sp] = s.group;
+                    s.sp++;
+                } else {
+                    atomicOr(errors, 2u);
+                }
+            }
+            const WideNode *np = &nodes[index];
+            const uint8_t *nb = reinterpret_cast<const uint8_t *>(np);
+            const float4 os = __ldg(&np->originScale);
+            const uint2 bases = __ldg(reinterpret_cast<const uint2 *>(&np->bases));
+            const uint32_t meta = __ldg(nb + 24u + slot);
+            const uint32_t nx = __ldg(nb + offX), fx = __ldg(nb + (88u + 2u * slot - offX));
+            const uint32_t ny = __ldg(nb + offY), fy = __ldg(nb + (104u + 2u * slot - offY));
+            const uint32_t nz = __ldg(nb + offZ), fz = __ldg(nb + (120u + 2u * slot - offZ));
+            const uint32_t ew = __float_as_uint(os.w);
+            const float3 idir = s.r.idir;
+            const float ax = __uint_as_float((ew & 0xffu) << 23) * idir.x;
+            const float ay = __uint_as_float(((ew >> 8) & 0xffu) << 23) * idir.y;
+            const float az = __uint_as_float(((ew >> 16) & 0xffu) << 23) * idir.z;
+            const float bx = (os.x - s.r.org.x) * idir.x, by = (os.y - s.r.org.y) * idir.y, bz = (os.z - s.r.org.z) * idir.z;
+            // planes and widening as in intersectChildren
+            const float wx = fmaf(4.0e-7f, fabsf(bx), 0.0078125f * fabsf(ax));
+            const float wy = fmaf(4.0e-7f, fabsf(by), 0.0078125f * fabsf(ay));
+            const float wz = fmaf(4.0e-7f, fabsf(bz), 0.0078125f * fabsf(az));
+            const float Ax = 128.0f * ax, Ay = 128.0f * ay, Az = 128.0f * az;
+            const float t0x = fmaf(bytePlane(nx, 0), Ax, fmaf(-32768.0f, ax, bx - wx));
+            const float t1x = fmaf(bytePlane(fx, 0), Ax, fmaf(-32768.0f, ax, bx + wx));
+            const float t0y = fmaf(bytePlane(ny, 0), Ay, fmaf(-32768.0f, ay, by - wy));
+            const float t1y = fmaf(bytePlane(fy, 0), Ay, fmaf(-32768.0f, ay, by + wy));
+            const float t0z = fmaf(bytePlane(nz, 0), Az, fmaf(-32768.0f, az, bz - wz));
+            const float t1z = fmaf(bytePlane(fz, 0), Az, fmaf(-32768.0f, az, bz + wz));
+            const float enter = fmaxf(fmaxf(t0x, t0y), fmaxf(t0z, s.tmin));
+            const float leave = fminf(fminf(t1x, t1y), fminf(t1z, fmaf(s.tmax, 1.000002f, s.slack)));
+            const uint32_t imask = ew >> 24;
+            if (enter <= leave * 1.0000004f) {
+                inner = ((imask >> slot) & 1u) != 0u;
+                if (!inner) triHits = (meta >> 5) << (meta & 31u);
+            }
+            s.group = make_uint2(bases.x, imask);
+            triBase = bases.y;
+        }
+        const uint32_t innerHits = (__ballot_sync(FULL, inner) >> shift) & 0xffu;
+        s.group.y |= innerHits << 24;
+        bool finished = false;
+        if (__any_sync(FULL, triHits != 0u)) {
+            triHits |= __shfl_xor_sync(FULL, triHits, 1);
+            triHits |= __shfl_xor_sync(FULL, triHits, 2);
+            triHits |= __shfl_xor_sync(FULL, triHits, 4);
+            int bestTri = -1;
+            uint32_t bestInst = 0xffffffffu, bestPrim = 0xffffffffu;
+            float bestT = s.tmax, bestB0 = 0.0f, bestB1 = 0.0f;
+            for (uint32_t bits = triHits >> sub, i = sub; bits != 0u; bits >>= 8, i += 8u) {
+                if (!(bits & 1u)) continue;
+                const int ti = (int)(triBase + i);
+                const float4 *tv = &tris[TRI_FLOAT4 * (size_t)ti + 3 * s.r.wr.kz];
+                const float4 a = __ldg(&tv[0]), b = __ldg(&tv[1]), c = __ldg(&tv[2]);
+                float t, b0, b1;
+                if (intersectTriangle(s.r.wr, xyz(a), xyz(b), xyz(c), s.tmin, bestT, t, b0, b1)) {
+                    const uint32_t inst = __float_as_uint(a.w), prim = __float_as_uint(b.w);
+                    if (t < bestT || bestTri < 0 || inst < bestInst || (inst == bestInst && prim < bestPrim)) {
+                        bestTri = ti;
+                        bestInst = inst;
+                        bestPrim = prim;
+                        bestT = t;
+                        bestB0 = b0;
+                        bestB1 = b1;
+                    }
+                }
+            }
+            const uint32_t found = (__ballot_sync(FULL, bestTri >= 0) >> shift) & 0xffu;
+            if (ANY) {
+                if (found) {
+                    s.hitTri = 0;  // any of them
+                    finished = true;
+                }
+            } else if (__any_sync(FULL, found != 0u)) {
+#pragma unroll
+                for (int m = 1; m < 8; m <<= 1) {
+                    const int tri = __shfl_xor_sync(FULL, bestTri, m);
+                    const uint32_t inst = __shfl_xor_sync(FULL, bestInst, m), prim = __shfl_xor_sync(FULL, bestPrim, m);
+                    const float t = __shfl_xor_sync(FULL, bestT, m), b0 = __shfl_xor_sync(FULL, bestB0, m),
+                                b1 = __shfl_xor_sync(FULL, bestB1, m);
+                    if (tri >= 0 && (bestTri < 0 || t < bestT || (t == bestT && (inst < bestInst || (inst == bestInst && prim < bestPrim))))) {
+                        bestTri = tri;
+                        bestInst = inst;
+                        bestPrim = prim;
+                        bestT = t;
+                        bestB0 = b0;
+                        bestB1 = b1;
+                    }
+                }
+                if (bestTri >= 0 && (bestT < s.tmax || s.hitTri < 0 || bestInst < s.hitInst ||
+                                     (bestInst == s.hitInst && bestPrim < s.hitPrim))) {
+                    s.hitTri = bestTri;
+                    s.hitInst = bestInst;
+                    s.hitPrim = bestPrim;
+                    s.tmax = bestT;
+                    s.b0 = bestB0;
+                    s.b1 = bestB1;
+                }
+            }
+        }
+        __syncwarp();  // the pushed groups
+        if (have) {
+            if (!finished && s.group.y <= 0x00ffffffu) {
+                if (s.sp == 0) finished = true;
+                else s.group = stack[--s.sp];
+            }
+            if (finished) have = false;
+        }
+        __syncwarp();  // before the entries read are pushed over
+    }
+}
+
 // Single-ray forms of the two queries (test hooks).
 RMD_HD bool traceClosest(const WideNode *__restrict__ nodes, const float4 *__restrict__ tris, float3 o, float3 d,
                          float tmin, float tmax, float4 &hit, uint32_t &inst, uint32_t *errors) {

@@ -1,17 +1,21 @@
 // Path state, queues and counters of the persistent wavefront, shared by the
 // static kernels (film / regeneration, traversal) and the NVRTC shading
 // module.  One iteration is
-//     film+regen -> closest-hit trace -> shade (NEE, BSDF sample) -> shadow trace
+//     film+regen -> trace (closest hits, the previous iteration's shadow rays)
+//     -> shade (NEE, BSDF sample)
 // and replaces one depth step of Renderer.execute (Renderer.swift:545-673)
 // for every path in flight; finished paths are replaced by new camera
-// samples, so the pool stays full until the last samples drain.
+// samples, so the pool stays full until the last samples drain.  A render
+// that trains the guide traces its shadow rays right after shading instead,
+// so that the training records are complete when the host looks at them.
 //
 // Path state is kept in queue order, not in fixed slots: iteration i (parity
 // p = i & 1) reads the active paths from S[p] at positions 0..n-1, and the
 // shading pass writes every path it continues to the next free position of
 // S[p ^ 1] (one atomic per warp), so each kernel reads and writes its path
 // records with coalesced 16-byte accesses.  Paths that end go to the finish
-// list with their radiance; the next film pass adds them to the film.
+// list of their parity with their radiance; the film pass adds them to the
+// film once their shadow rays are traced.
 #pragma once
 #include "guide.cuh"
 #include "scene.cuh"
@@ -48,11 +52,12 @@ struct Counters {
     uint32_t padQ[62];
     uint32_t nF[2];       // finished paths written by the shading pass of parity p
     uint32_t padF[62];
-    uint32_t nShadow;     // shadow rays of this iteration
-    uint32_t padS[63];
-    uint32_t traceWork;   // persistent closest-hit work counter
+    uint32_t nShadow;     // shadow rays cast by the shading pass
+    uint32_t nShadowPrev; // by the previous iteration's
+    uint32_t padS[62];
+    uint32_t traceWork;   // work counter of the trace kernel
     uint32_t padT[63];
-    uint32_t shadowWork;  // persistent any-hit work counter
+    uint32_t shadowWork;  // work counter of a trace of shadow rays alone
     uint32_t padW[63];
     uint32_t nHit;        // active paths whose closest-hit ray hit a surface (front of `order`)
     uint32_t padH[63];
@@ -66,24 +71,31 @@ struct Counters {
     uint32_t loopIterations;  // device-driven render loop: wavefront iterations so far
     uint32_t padL;
     unsigned long long numPaths;    // paths of this render
-    unsigned long long nextPath;    // next path id handed out by the film kernel
+    unsigned long long nextPath;    // first path id that the film kernel of this iteration handed out
     unsigned long long endPath;     // one past the last path id of this render
     unsigned long long pathsDone;   // paths whose radiance reached the film
     unsigned long long segments;    // closest-hit rays shaded
     unsigned long long shadowRays;  // shadow rays traced
     unsigned long long rays;        // closest-hit rays traced (hits and misses)
     unsigned long long invalid;     // light and BSDF samples dropped for a non-finite weight
+    unsigned long long handOut[2];  // next path id before the film kernel of parity p
+    // stage times by the device's clocks: starts of the film and trace kernels and end of the trace (ns), their
+    // sums over the iterations, and the trace kernel's clocks spent on closest hits and on shadow rays
+    unsigned long long filmStart, traceStart, traceEnd;
+    unsigned long long nsFilm, nsTrace, nsShade;
+    unsigned long long traceClocks[2];
 };
 
 
 // camera samples the film kernel of this iteration appends to S[p]
-__device__ __forceinline__ uint32_t newPaths(const Counters *c, uint32_t p) {
-    const unsigned long long next = c->nextPath, end = c->endPath;
+__device__ __forceinline__ uint32_t newPaths(const Counters *c, uint32_t p, unsigned long long next) {
+    const unsigned long long end = c->endPath;
     if (next >= end) return 0u;
     const unsigned long long left = end - next;
     const uint32_t room = c->capacity - c->nQ[p];
     return left < (unsigned long long)room ? (uint32_t)left : room;
 }
+__device__ __forceinline__ uint32_t newPaths(const Counters *c, uint32_t p) { return newPaths(c, p, c->nextPath); }
 // number of active paths in S[p] after the film kernel of this iteration
 __device__ __forceinline__ uint32_t activeCount(const Counters *c, uint32_t p) { return c->nQ[p] + newPaths(c, p); }
 
@@ -130,12 +142,14 @@ struct PathPool {
     float4 *hit;        // per active path of this iteration: t (<= 0: miss), b0, b1, primitive (bits)
     uint32_t *hitInst;  // instance index
     uint32_t *order;    // shading order: positions of hits from the front, of misses from the back
-    float4 *fin;        // finished paths: radiance.xyz, pixel (bits)
+    float4 *fin;        // finished paths: radiance.xyz, pixel (bits); the shading pass's list, one of
+    float4 *finLists[2];  // the lists of the paths finished by the shading passes of parity p
     float4 *shO;        // shadow: origin.xyz, tmax
     float4 *shD;        // shadow: direction.xyz, target (bits; SHADOW_TO_FINISHED, SHADOW_TO_RECORD)
     float4 *shW;        // shadow: weight.xyz; w: 1 / mean throughput of its vertex for a light record (else 0)
     // guide training (nullptr when not training)
-    float4 *finRec;       // the pending records of finished paths (4 per entry)
+    float4 *finRec;       // the pending records of finished paths (4 per entry); the shading pass's list, one of
+    float4 *finRecLists[2];
     float4 *shRec;        // per shadow ray: its vertex's features 0-3 | features 4-6, BSDF pdf of the ray
     GuideRecord *records; // ring of the latest records with a nonzero target (Counters::numRecords)
     uint32_t recordCapacity;  // a power of two
@@ -153,7 +167,7 @@ struct PathPool {
 constexpr size_t pathPoolBytes(uint32_t capacity) {
     const size_t P = capacity, pad = 255;
     const size_t per16 = (P * 16 + pad) & ~pad, per4 = (P * 4 + pad) & ~pad;
-    return 2 * 5 * per16 + 5 * per16 + 2 * per4;
+    return 2 * 5 * per16 + 6 * per16 + 2 * per4;
 }
 inline PathPool carvePathPool(void *base, uint32_t capacity) {
     unsigned char *p = static_cast<unsigned char *>(base);
@@ -172,13 +186,15 @@ inline PathPool carvePathPool(void *base, uint32_t capacity) {
         pool.s[k].rec = nullptr;  // guiding buffers are allocated by the renderer when enabled
     }
     pool.hit = static_cast<float4 *>(take(16));
-    pool.fin = static_cast<float4 *>(take(16));
+    pool.finLists[0] = static_cast<float4 *>(take(16));
+    pool.finLists[1] = static_cast<float4 *>(take(16));
+    pool.fin = pool.finLists[0];
     pool.shO = static_cast<float4 *>(take(16));
     pool.shD = static_cast<float4 *>(take(16));
     pool.shW = static_cast<float4 *>(take(16));
     pool.hitInst = static_cast<uint32_t *>(take(4));
     pool.order = static_cast<uint32_t *>(take(4));
-    pool.finRec = nullptr;
+    pool.finRec = pool.finRecLists[0] = pool.finRecLists[1] = nullptr;
     pool.shRec = nullptr;
     pool.records = nullptr;
     pool.recordCapacity = 0;
@@ -211,6 +227,13 @@ struct ShadeParams {
     FrameParams fp;
     Counters *counters;
     uint32_t cur;
+#ifndef __CUDACC_RTC__
+    void setParity(uint32_t p) {
+        cur = p;
+        pool.fin = pool.finLists[p];
+        pool.finRec = pool.finRecLists[p];
+    }
+#endif
 };
 
 // Appends the calling lane to a queue with one atomic per warp
@@ -244,6 +267,13 @@ __device__ __forceinline__ void warpAdd64(unsigned long long *counter, uint32_t 
     const int leader = __ffs(mask) - 1;
     const uint32_t total = __reduce_add_sync(mask, v);
     if ((int)(threadIdx.x & 31) == leader && total) atomicAdd(counter, (unsigned long long)total);
+}
+
+// Nanoseconds of the device's global timer.
+__device__ __forceinline__ unsigned long long deviceNs() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
 }
 
 // generate.metal:88-91 with 8x8 threadgroups: block-linear ray index and its inverse

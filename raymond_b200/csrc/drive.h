@@ -1,0 +1,52 @@
+// The host-driven loop of wavefront iterations.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "device/wavefront.cuh"
+
+namespace rmdhost {
+
+// Enqueues iterations until `check` ends the loop.  iterate(cur, paths)
+// enqueues one iteration of parity cur with at most `paths` active paths (what
+// its grids need to cover); check(counters, iterations) returns whether the
+// render is over (done, or failed).
+//
+// The first counters are read once every path has been handed out and could
+// have ended, and then after every second iteration, two iterations behind the
+// ones being enqueued: the device never waits for the host, for at most four
+// empty iterations at the end.  (Reading them after every fourth iteration and
+// waiting left a gap of 10-20 us each time.)  `slots`: two Counters in pinned
+// memory; `events`: two events.  On return the last iterations may still run.
+template <class Iterate, class Check>
+cudaError_t driveWavefront(const rmd::Counters *cnt, uint64_t numPaths, uint32_t capacity, rmd::Counters *slots,
+                           cudaEvent_t *events, cudaStream_t st, Iterate iterate, Check check) {
+    uint64_t it = 0, paths = std::min<uint64_t>(numPaths, capacity);
+    uint64_t next = ((numPaths + capacity - 1) / capacity + 3) & ~uint64_t(1);
+    for (uint32_t k = 0;; k++, next += 2) {
+        cudaError_t e;
+        for (; it < next; it++)
+            if ((e = iterate((uint32_t)(it & 1u), paths)) != cudaSuccess) return e;
+        if ((e = cudaMemcpyAsync(&slots[k & 1u], cnt, sizeof(rmd::Counters), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+            (e = cudaEventRecord(events[k & 1u], st)) != cudaSuccess)
+            return e;
+        if (k == 0) continue;
+        if ((e = cudaEventSynchronize(events[(k - 1u) & 1u])) != cudaSuccess) return e;
+        const rmd::Counters &h = slots[(k - 1u) & 1u];
+        if (check(h, it)) return cudaSuccess;
+        if (h.handOut[0] >= h.endPath) paths = std::min<uint64_t>(paths, std::max(h.nQ[0], 1u));
+    }
+}
+
+// blocks of `threads` threads that give `paths` paths a thread each, at most `most`
+inline int gridFor(uint64_t paths, int threads, int most) {
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>((paths + threads - 1) / threads, (uint64_t)most));
+}
+
+// Trace grid: the resident one, or as many blocks as give every closest-hit
+// and shadow ray of `paths` paths its 8 lanes.
+inline int traceGridFor(uint64_t paths, int most) { return gridFor(2 * paths + 8, 16, most); }
+
+}  // namespace rmdhost

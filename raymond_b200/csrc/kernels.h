@@ -11,8 +11,15 @@ cudaError_t rmdLaunchLoopCondition(rmd::Counters *cnt, cudaGraphConditionalHandl
                                    uint32_t maxIterations, cudaStream_t s);
 cudaError_t rmdLaunchFrameInit(const rmd::PathPool &pool, rmd::Counters *cnt, uint64_t firstPath, uint64_t endPath,
                                cudaStream_t s);
+// Stages of an iteration of parity `cur`.  The film kernel adds finish list
+// `fin`: with rmdLaunchTrace (closest hits and the previous iteration's shadow
+// rays) the list of the iteration before the previous one, parity cur; with
+// the closest hits and the shadow rays traced apart, the latter after shading,
+// that of the previous one, cur ^ 1.
 cudaError_t rmdLaunchFilmRegen(const rmd::Context &ctx, const rmd::PathPool &pool, const rmd::FrameParams &fp,
-                               rmd::Counters *cnt, uint32_t cur, int blocks, cudaStream_t s);
+                               rmd::Counters *cnt, uint32_t cur, uint32_t fin, int blocks, cudaStream_t s);
+cudaError_t rmdLaunchTrace(const rmd::WideNode *nodes, const float4 *tris, const rmd::PathPool &pool,
+                           rmd::Counters *cnt, uint32_t cur, int blocks, cudaStream_t s);
 cudaError_t rmdLaunchTraceClosest(const rmd::WideNode *nodes, const float4 *tris, const rmd::PathPool &pool,
                                   rmd::Counters *cnt, uint32_t cur, int blocks, cudaStream_t s);
 cudaError_t rmdLaunchTraceShadow(const rmd::WideNode *nodes, const float4 *tris, const rmd::PathPool &pool,

@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "../../include/raymond.h"
+#include "drive.h"
 #include "kernels.h"
 #include "scene_view.h"
 
@@ -43,6 +44,13 @@ static __device__ __align__(256) unsigned char g_noallocScratch[kScratchBytes];
 
 std::mutex g_mutex;
 void *g_scratch[64] = {};  // device address of g_noallocScratch per device, set by noallocSetup
+// Pinned counters and events of the render loop, per device, made with the
+// first context (2 x sizeof(Counters)) and kept: like the array, shared by all calls.
+struct HostSide {
+    Counters *counters = nullptr;
+    cudaEvent_t events[2] = {};
+};
+HostSide g_host[64];
 
 rmd_status cudaFail(cudaError_t e, const char *what) {
     std::string msg = std::string("rmd_render_noalloc: ") + what + ": " + cudaGetErrorString(e);
@@ -57,10 +65,20 @@ namespace rmdhost {
 rmd_status noallocSetup(int device) {
     if (device < 0 || device >= 64) return RMD_OK;  // rmd_render_noalloc rejects such devices
     void *ptr = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&ptr, g_noallocScratch);
+    cudaError_t e = cudaGetSymbolAddress(&ptr, g_noallocScratch);
     if (e != cudaSuccess) return cudaFail(e, "cudaGetSymbolAddress");
     std::lock_guard<std::mutex> lock(g_mutex);
     g_scratch[device] = ptr;
+    HostSide &h = g_host[device];
+    if (h.events[0] && cudaEventQuery(h.events[0]) != cudaSuccess) {  // gone with a device reset
+        cudaGetLastError();
+        h = HostSide();
+    }
+    for (cudaEvent_t &ev : h.events)
+        if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+            return cudaFail(e, "cudaEventCreate");
+    if (!h.counters && (e = cudaMallocHost((void **)&h.counters, 2 * sizeof(Counters))) != cudaSuccess)
+        return cudaFail(e, "cudaMallocHost");
     return RMD_OK;
 }
 
@@ -87,9 +105,11 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
     if (e != cudaSuccess) return cudaFail(e, "cudaSetDevice");
 
     void *base;
+    HostSide *host;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         base = g_scratch[v.device];  // set when the scene's context was created
+        host = &g_host[v.device];
     }
     if (!base) return rmdhost::setLastError(RMD_ERROR_CUDA, "rmd_render_noalloc: scratch array not set up");
     const uint32_t P = pool_size ? pool_size : kMaxPaths;
@@ -132,31 +152,24 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
 
     if ((e = rmdLaunchFrameInit(pool, cnt, firstPath, firstPath + numPaths, st)) != cudaSuccess)
         return cudaFail(e, "frame init");
-    const uint64_t maxIters = ((numPaths + P - 1) / P + 1) * ((uint64_t)s->max_depth + 1) + 8;
-    uint64_t it = 0;
-    uint32_t cur = 0;
-    Counters h;
-    while (true) {
-        for (int k = 0; k < 4; k++, it++) {
-            if ((e = rmdLaunchFilmRegen(ctx, pool, fp, cnt, cur, rb, st)) != cudaSuccess) return cudaFail(e, "film");
-            if ((e = rmdLaunchTraceClosest(v.nodes, v.tris, pool, cnt, cur, tb, st)) != cudaSuccess)
-                return cudaFail(e, "trace");
-            sp.cur = cur;
-            if ((e = cudaLaunchKernel((const void *)v.shade, dim3(v.shadeBlocks), dim3(128), shadeArgs, 0, st)) !=
-                cudaSuccess)
-                return cudaFail(e, "shade");
-            if ((e = rmdLaunchTraceShadow(v.nodes, v.tris, pool, cnt, cur, tb, st)) != cudaSuccess)
-                return cudaFail(e, "shadow");
-            cur ^= 1u;
-        }
-        // pageable stack destination: no pinned staging buffer is allocated
-        if ((e = cudaMemcpyAsync(&h, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-            return cudaFail(e, "counters");
-        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cudaFail(e, "synchronize");
-        if (h.errors) return rmdhost::setLastError(RMD_ERROR_QUEUE_OVERFLOW, "rmd_render_noalloc: device error flags");
-        if (h.pathsDone >= numPaths) break;
-        if (it > maxIters)
-            return rmdhost::setLastError(RMD_ERROR_WATCHDOG, "rmd_render_noalloc: render did not drain");
-    }
+    const uint64_t maxIters = ((numPaths + P - 1) / P + 1) * ((uint64_t)s->max_depth + 1) + 16;
+    const auto iterate = [&](uint32_t cur, uint64_t paths) {
+        cudaError_t e = rmdLaunchFilmRegen(ctx, pool, fp, cnt, cur, cur, rmdhost::gridFor(paths, 256, rb), st);
+        if (e != cudaSuccess) return e;
+        if ((e = rmdLaunchTrace(v.nodes, v.tris, pool, cnt, cur, rmdhost::traceGridFor(paths, tb), st)) != cudaSuccess) return e;
+        sp.setParity(cur);
+        return cudaLaunchKernel((const void *)v.shade, dim3(rmdhost::gridFor(paths, 128, v.shadeBlocks)), dim3(128), shadeArgs, 0, st);
+    };
+    rmd_status status = RMD_OK;
+    const auto check = [&](const Counters &h, uint64_t iterations) {
+        if (h.errors) status = rmdhost::setLastError(RMD_ERROR_QUEUE_OVERFLOW, "rmd_render_noalloc: device error flags");
+        else if (h.pathsDone < numPaths && iterations > maxIters)
+            status = rmdhost::setLastError(RMD_ERROR_WATCHDOG, "rmd_render_noalloc: render did not drain");
+        return status != RMD_OK || h.pathsDone >= numPaths;
+    };
+    e = rmdhost::driveWavefront(cnt, numPaths, P, host->counters, host->events, st, iterate, check);
+    if (e != cudaSuccess) return cudaFail(e, "wavefront");
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cudaFail(e, "synchronize");
+    if (status != RMD_OK) return status;
     return RMD_OK;
 }

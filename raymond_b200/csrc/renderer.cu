@@ -18,6 +18,7 @@
 #include "bvh_build.h"
 #include "bvh_gpu.h"
 #include "codegen.h"
+#include "drive.h"
 #include "exr.h"
 #include "device/wavefront.cuh"
 #include "guide.h"
@@ -193,7 +194,7 @@ struct rmd_renderer {
     int traceBlocksPerSm = 12;
     DevBuf pool;  // path state, finish list and shadow rays (carvePathPool)
     DevBuf counters, film, film64, resolve;
-    Counters *hostCounters = nullptr;  // pinned
+    Counters *hostCounters = nullptr;  // pinned, two (driveWavefront)
     Context dctx{};
     uint64_t samples = 0;     // samples accumulated in the film (what normalisation divides by)
     uint64_t nextSample = 0;  // sample index a render continues at (first_sample < 0)
@@ -246,7 +247,7 @@ struct rmd_batch {
     uint64_t samples = 0;     // samples of every view accumulated in the films
     uint64_t nextSample = 0;  // sample index a render continues at (first_sample < 0)
     rmd_stats stats{};
-    cudaEvent_t ev[2] = {};
+    cudaEvent_t ev[4] = {};
     // the instantiated render graph and the settings it was captured for
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
@@ -899,7 +900,8 @@ static void applyGuide(const GuideState &g, uint32_t capacity, PathPool &pool) {
     if (g.settings.training && g.pathCapacity >= capacity) {
         pool.s[0].rec = g.rec.as<float4>();
         pool.s[1].rec = g.rec.as<float4>() + 4 * (size_t)capacity;
-        pool.finRec = g.finRec.as<float4>();
+        // one list: a training render's film kernel takes it up before the next shading pass fills it
+        pool.finRec = pool.finRecLists[0] = pool.finRecLists[1] = g.finRec.as<float4>();
         pool.shRec = g.settings.skip_light_records ? nullptr : g.shRec.as<float4>();
         pool.records = g.records.as<GuideRecord>();
         pool.recordCapacity = g.recordCapacity;
@@ -1064,7 +1066,7 @@ rmd_status rmd_renderer_create(rmd_scene *scene, uint32_t width, uint32_t height
     r->capacity = pool_size ? pool_size : (1u << 21);
     rmd_status st = allocatePool(r.get());
     if (st != RMD_OK) return st;
-    RMD_CUDA(cudaMallocHost((void **)&r->hostCounters, sizeof(Counters)));
+    RMD_CUDA(cudaMallocHost((void **)&r->hostCounters, 2 * sizeof(Counters)));
     for (auto &e : r->ev) RMD_CUDA(cudaEventCreate(&e));
     st = rmd_renderer_set_size(r.get(), width, height);
     if (st != RMD_OK) return st;
@@ -1203,51 +1205,78 @@ rmd_status rmd_render(rmd_renderer *r, const rmd_render_settings *s) {
     enum { STAGE_FILM, STAGE_TRACE, STAGE_GUIDE, STAGE_SHADE, STAGE_SHADOW, STAGE_TRAIN, STAGES };
     RMD_CUDA(cudaEventRecord(r->ev[0], st));
     RMD_CUDA(rmdLaunchFrameInit(pool, cnt, firstPath, firstPath + numPaths, st));
-    // every path needs at most max_depth iterations after it is generated, and
+    // every path needs at most max_depth iterations after it is generated and two to reach the film, and
     // each iteration generates min(capacity, remaining) paths
-    const uint64_t maxIters = ((numPaths + r->capacity - 1) / r->capacity + 1) * ((uint64_t)s->max_depth + 1) + 8;
-    uint64_t it = 0;
-    uint32_t cur = 0;
-    bool done = false;
+    const uint64_t maxIters = ((numPaths + r->capacity - 1) / r->capacity + 1) * ((uint64_t)s->max_depth + 1) + 16;
+    // Guided renders time their stages with events between the kernels; the
+    // others by the kernels' own clocks (Counters), without events, which cost
+    // small renders about a tenth of their time.
+    const bool useEvents = guideSampling || guideTraining;
     size_t evi = 0;
-    RMD_CUDA(r->stageEvent(evi++, STAGE_FILM, st));
-    while (!done) {
-        for (int k = 0; k < 4; k++, it++) {
-            RMD_CUDA(rmdLaunchFilmRegen(r->dctx, pool, fp, cnt, cur, rb, st));
-            RMD_CUDA(r->stageEvent(evi++, STAGE_FILM, st));
-            RMD_CUDA(rmdLaunchTraceClosest(scene->bvhNodes.as<WideNode>(), scene->bvhTris.as<float4>(), pool, cnt, cur, tb, st));
-            RMD_CUDA(r->stageEvent(evi++, STAGE_TRACE, st));
-            if (guideSampling) {
-                RMD_CUDA(rmdLaunchGuideInfer(r->dctx, pool, cnt, cur, fp.guideDepth, net, pool.guide, guideBlocks, st));
-                RMD_CUDA(r->stageEvent(evi++, STAGE_GUIDE, st));
+    const auto mark = [&](int stage) { return useEvents ? r->stageEvent(evi++, stage, st) : cudaSuccess; };
+    RMD_CUDA(mark(STAGE_FILM));
+    const WideNode *nodes = scene->bvhNodes.as<WideNode>();
+    const float4 *tris = scene->bvhTris.as<float4>();
+    const auto iterate = [&](uint32_t cur, uint64_t paths) -> cudaError_t {
+        cudaError_t e;
+        const int blocks = rmdhost::traceGridFor(paths, tb);
+        if ((e = rmdLaunchFilmRegen(r->dctx, pool, fp, cnt, cur, guideTraining ? cur ^ 1u : cur,
+                                    rmdhost::gridFor(paths, 256, rb), st)) != cudaSuccess)
+            return e;
+        if ((e = mark(STAGE_FILM)) != cudaSuccess) return e;
+        e = guideTraining ? rmdLaunchTraceClosest(nodes, tris, pool, cnt, cur, blocks, st)
+                          : rmdLaunchTrace(nodes, tris, pool, cnt, cur, blocks, st);
+        if (e != cudaSuccess || (e = mark(STAGE_TRACE)) != cudaSuccess) return e;
+        if (guideSampling) {
+            e = rmdLaunchGuideInfer(r->dctx, pool, cnt, cur, fp.guideDepth, net, pool.guide, guideBlocks, st);
+            if (e != cudaSuccess || (e = mark(STAGE_GUIDE)) != cudaSuccess) return e;
+        }
+        sp.setParity(cur);
+        e = cudaLaunchKernel((const void *)r->shade, dim3(rmdhost::gridFor(paths, 128, sb)), dim3(128), shadeArgs, 0, st);
+        if (e != cudaSuccess || (e = mark(STAGE_SHADE)) != cudaSuccess) return e;
+        if (guideTraining) {
+            e = rmdLaunchTraceShadow(nodes, tris, pool, cnt, cur, blocks, st);
+            if (e != cudaSuccess || (e = mark(STAGE_SHADOW)) != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    };
+    uint64_t it = 0;
+    Counters h;  // of the end
+    rmd_status status = RMD_OK;
+    const auto check = [&](const Counters &c, uint64_t iterations) {
+        h = c;
+        it = iterations;
+        if (c.errors) {
+            r->stats.errors = c.errors;
+            status = c.errors & ERR_GUIDE_TIMEOUT
+                         ? fail(RMD_ERROR_WATCHDOG, "guide inference: a tensor-core wait expired (device error flags " +
+                                                        std::to_string(c.errors) + ")")
+                         : fail(RMD_ERROR_QUEUE_OVERFLOW, "device error flags " + std::to_string(c.errors));
+            return true;
+        }
+        if (c.pathsDone >= numPaths) return true;
+        if (iterations > maxIters) status = fail(RMD_ERROR_WATCHDOG, "render did not drain in the iteration bound");
+        return status != RMD_OK;
+    };
+    if (!guideTraining) {
+        RMD_CUDA(rmdhost::driveWavefront(cnt, numPaths, r->capacity, r->hostCounters, &r->ev[2], st, iterate, check));
+    } else {  // training steps run between counter checks
+        const uint64_t all = std::min<uint64_t>(numPaths, r->capacity);
+        for (bool over = false; !over;) {
+            for (int k = 0; k < 4; k++, it++) RMD_CUDA(iterate((uint32_t)(it & 1u), all));
+            RMD_CUDA(cudaMemcpyAsync(r->hostCounters, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+            RMD_CUDA(cudaStreamSynchronize(st));
+            over = check(*r->hostCounters, it);
+            if (status == RMD_OK && h.numSamples >= batch) {
+                rmd_status gs = guideTrainStep(guide, h, cnt, net, trainBlocks, st, trainSteps);
+                if (gs != RMD_OK) return gs;
+                RMD_CUDA(mark(STAGE_TRAIN));
             }
-            sp.cur = cur;
-            RMD_CUDA(cudaLaunchKernel((const void *)r->shade, dim3(sb), dim3(128), shadeArgs, 0, st));
-            RMD_CUDA(r->stageEvent(evi++, STAGE_SHADE, st));
-            RMD_CUDA(rmdLaunchTraceShadow(scene->bvhNodes.as<WideNode>(), scene->bvhTris.as<float4>(), pool, cnt, cur, tb, st));
-            RMD_CUDA(r->stageEvent(evi++, STAGE_SHADOW, st));
-            cur ^= 1u;
         }
-        RMD_CUDA(cudaMemcpyAsync(r->hostCounters, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-        RMD_CUDA(cudaStreamSynchronize(st));
-        const Counters &h = *r->hostCounters;
-        if (h.errors) {
-            r->stats.errors = h.errors;
-            if (h.errors & ERR_GUIDE_TIMEOUT)
-                return fail(RMD_ERROR_WATCHDOG, "guide inference: a tensor-core wait expired (device error flags " +
-                                                    std::to_string(h.errors) + ")");
-            return fail(RMD_ERROR_QUEUE_OVERFLOW, "device error flags " + std::to_string(h.errors));
-        }
-        if (guideTraining && h.numSamples >= batch) {
-            rmd_status gs = guideTrainStep(guide, h, cnt, net, trainBlocks, st, trainSteps);
-            if (gs != RMD_OK) return gs;
-            RMD_CUDA(r->stageEvent(evi++, STAGE_TRAIN, st));
-        }
-        if (h.pathsDone >= numPaths) done = true;
-        else if (it > maxIters) return fail(RMD_ERROR_WATCHDOG, "render did not drain in the iteration bound");
     }
     RMD_CUDA(cudaEventRecord(r->ev[1], st));
     RMD_CUDA(cudaEventSynchronize(r->ev[1]));
+    if (status != RMD_OK) return status;
     float ms = 0;
     cudaEventElapsedTime(&ms, r->ev[0], r->ev[1]);
     double stage[STAGES] = {};
@@ -1256,11 +1285,20 @@ rmd_status rmd_render(rmd_renderer *r, const rmd_render_settings *s) {
         cudaEventElapsedTime(&t, r->stageEvents[i - 1], r->stageEvents[i]);
         stage[r->stageOf[i]] += t;
     }
+    if (!useEvents) {
+        stage[STAGE_FILM] = 1e-6 * (double)h.nsFilm;
+        stage[STAGE_TRACE] = 1e-6 * (double)h.nsTrace;
+        stage[STAGE_SHADE] = 1e-6 * (double)h.nsShade;
+    }
+    if (!guideTraining) {  // one kernel for closest hits and shadow rays: its time by the clocks spent on each
+        const double closest = (double)h.traceClocks[0], both = closest + (double)h.traceClocks[1];
+        stage[STAGE_SHADOW] = both > 0.0 ? stage[STAGE_TRACE] * (1.0 - closest / both) : 0.0;
+        stage[STAGE_TRACE] -= stage[STAGE_SHADOW];
+    }
     if (trainSteps) {
         rmd_status gs = guideReadLoss(guide);
         if (gs != RMD_OK) return gs;
     }
-    const Counters &h = *r->hostCounters;
     r->stats.paths = h.pathsDone;
     r->stats.segments = h.segments;
     r->stats.rays = h.rays;
@@ -1827,7 +1865,7 @@ rmd_status rmd_batch_create(rmd_context *ctx, const rmd_scene_desc *descs, int32
     if (b->capacity > BATCH_MAX_CAPACITY) return fail(RMD_ERROR_INVALID_ARGUMENT, "batch pools hold at most 2^22 paths");
     rmd_status r = batchAllocatePool(b.get());
     if (r != RMD_OK) return r;
-    RMD_CUDA(cudaMallocHost((void **)&b->hostCounters, sizeof(Counters)));
+    RMD_CUDA(cudaMallocHost((void **)&b->hostCounters, 2 * sizeof(Counters)));
     for (auto &e : b->ev) RMD_CUDA(cudaEventCreate(&e));
     batchSelectShade(b.get(), b->defaultMinBlocks, false);
     *out = b.release();
@@ -1847,27 +1885,26 @@ rmd_status rmd_batch_reset(rmd_batch *b) {
     return RMD_OK;
 }
 
-// Records the render's wavefront loop on `st`: host-driven (counter checks
-// every 4 iterations) or, with `handle`, as the body of a graph while loop
-// (2 iterations and the condition kernel).
-static rmd_status batchEnqueueIterations(rmd_batch *b, const PathPool &pool, const FrameParams &fp, ShadeParams &sp,
-                                         const GuideNetView &net, int iterations, cudaStream_t st) {
+// Enqueues one wavefront iteration of parity `cur` with at most `paths` active paths on `st`.
+static cudaError_t batchEnqueueIteration(rmd_batch *b, const PathPool &pool, const FrameParams &fp, ShadeParams &sp,
+                                         const GuideNetView &net, uint32_t cur, uint64_t paths, cudaStream_t st) {
     Counters *cnt = b->counters.as<Counters>();
-    const int tb = b->ctx->smCount * b->traceBlocksPerSm;
-    const int rb = std::min<int>((b->capacity + 255) / 256, b->ctx->smCount * 8);
+    const bool training = b->guide.settings.training != 0;
+    const int tb = rmdhost::traceGridFor(paths, b->ctx->smCount * b->traceBlocksPerSm);
+    const int rb = rmdhost::gridFor(paths, 256, std::min<int>((b->capacity + 255) / 256, b->ctx->smCount * 8));
     void *shadeArgs[] = {&sp};
-    for (int k = 0; k < iterations; k++) {
-        const uint32_t cur = (uint32_t)k & 1u;
-        RMD_CUDA(rmdLaunchFilmRegen(b->scenes[0]->dctx, pool, fp, cnt, cur, rb, st));
-        RMD_CUDA(rmdLaunchTraceClosest(nullptr, nullptr, pool, cnt, cur, tb, st));
-        if (pool.guide)
-            RMD_CUDA(rmdLaunchGuideInfer(b->scenes[0]->dctx, pool, cnt, cur, fp.guideDepth, net, pool.guide,
-                                         b->ctx->smCount, st));
-        sp.cur = cur;
-        RMD_CUDA(cudaLaunchKernel((const void *)b->shade, dim3(b->shadeBlocks), dim3(128), shadeArgs, 0, st));
-        RMD_CUDA(rmdLaunchTraceShadow(nullptr, nullptr, pool, cnt, cur, tb, st));
-    }
-    return RMD_OK;
+    cudaError_t e = rmdLaunchFilmRegen(b->scenes[0]->dctx, pool, fp, cnt, cur, training ? cur ^ 1u : cur, rb, st);
+    if (e != cudaSuccess) return e;
+    e = training ? rmdLaunchTraceClosest(nullptr, nullptr, pool, cnt, cur, tb, st)
+                 : rmdLaunchTrace(nullptr, nullptr, pool, cnt, cur, tb, st);
+    if (e != cudaSuccess) return e;
+    if (pool.guide && (e = rmdLaunchGuideInfer(b->scenes[0]->dctx, pool, cnt, cur, fp.guideDepth, net, pool.guide,
+                                               b->ctx->smCount, st)) != cudaSuccess)
+        return e;
+    sp.setParity(cur);
+    e = cudaLaunchKernel((const void *)b->shade, dim3(rmdhost::gridFor(paths, 128, b->shadeBlocks)), dim3(128), shadeArgs, 0, st);
+    if (e != cudaSuccess) return e;
+    return training ? rmdLaunchTraceShadow(nullptr, nullptr, pool, cnt, cur, tb, st) : cudaSuccess;
 }
 
 rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
@@ -1923,17 +1960,19 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
     sp.fp = fp;
     sp.counters = cnt;
     const uint64_t firstPath = firstSample * b->totalPixels;
-    const uint64_t maxIters = ((numPaths + b->capacity - 1) / b->capacity + 1) * ((uint64_t)s->max_depth + 1) + 8;
+    const uint64_t maxIters = ((numPaths + b->capacity - 1) / b->capacity + 1) * ((uint64_t)s->max_depth + 1) + 16;
+    const uint64_t allPaths = std::min<uint64_t>(numPaths, b->capacity);
     if (maxIters > 0xffffffffull) return fail(RMD_ERROR_INVALID_ARGUMENT, "render too long for one call");
 
     RMD_CUDA(cudaEventRecord(b->ev[0], st));
     RMD_CUDA(rmdLaunchFrameInit(pool, cnt, firstPath, firstPath + numPaths, st));
     uint64_t iterations = 0, trainSteps = 0;
+    Counters last;  // of the end
     // training steps run between counter checks, so a training batch uses the host-driven loop
     if (b->useGraph && !guide.settings.training) {
         // the graph depends on everything but the sample range (frame init sets that)
         const std::vector<uint64_t> key = {s->max_depth, s->sampling_mode, s->rng, s->seed, (uint64_t)fp.filmFp64,
-                                           maxIters, (uint64_t)b->capacity, (uint64_t)b->shadeMinBlocks,
+                                           maxIters, allPaths, (uint64_t)b->capacity, (uint64_t)b->shadeMinBlocks,
                                            (uint64_t)b->traceBlocksPerSm, (uint64_t)fp.guideDepth};
         if (!b->graphExec || b->graphKey != key) {
             if (b->graphExec) cudaGraphExecDestroy(b->graphExec);
@@ -1953,11 +1992,12 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             // the body: two iterations (both parities) and the condition kernel
             RMD_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            rmd_status e = batchEnqueueIterations(b, pool, fp, sp, net, 2, st);
-            cudaError_t ce = e == RMD_OK ? rmdLaunchLoopCondition(cnt, handle, 2, (uint32_t)maxIters, st) : cudaSuccess;
+            cudaError_t ce = cudaSuccess;
+            for (uint32_t cur = 0; cur < 2 && ce == cudaSuccess; cur++)
+                ce = batchEnqueueIteration(b, pool, fp, sp, net, cur, allPaths, st);
+            if (ce == cudaSuccess) ce = rmdLaunchLoopCondition(cnt, handle, 2, (uint32_t)maxIters, st);
             cudaGraph_t captured = nullptr;
             cudaError_t endErr = cudaStreamEndCapture(st, &captured);
-            if (e != RMD_OK) return e;
             RMD_CUDA(ce);
             RMD_CUDA(endErr);
             RMD_CUDA(cudaGraphInstantiate(&b->graphExec, b->graph, 0));
@@ -1966,7 +2006,7 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
         RMD_CUDA(cudaGraphLaunch(b->graphExec, st));
         RMD_CUDA(cudaMemcpyAsync(b->hostCounters, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
         RMD_CUDA(cudaStreamSynchronize(st));
-        const Counters &h = *b->hostCounters;
+        const Counters &h = last = *b->hostCounters;
         iterations = h.loopIterations;
         if (h.errors) {
             b->stats.errors = h.errors;
@@ -1974,28 +2014,44 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
                         "device error flags " + std::to_string(h.errors));
         }
     } else {
-        bool done = false;
-        while (!done) {
-            rmd_status e = batchEnqueueIterations(b, pool, fp, sp, net, 4, st);
-            if (e != RMD_OK) return e;
-            iterations += 4;
-            RMD_CUDA(cudaMemcpyAsync(b->hostCounters, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-            RMD_CUDA(cudaStreamSynchronize(st));
-            const Counters &h = *b->hostCounters;
-            if (h.errors) {
-                b->stats.errors = h.errors;
-                return fail(RMD_ERROR_QUEUE_OVERFLOW, "device error flags " + std::to_string(h.errors));
+        rmd_status status = RMD_OK;
+        const auto iterate = [&](uint32_t cur, uint64_t paths) {
+            return batchEnqueueIteration(b, pool, fp, sp, net, cur, paths, st);
+        };
+        const auto check = [&](const Counters &c, uint64_t done) {
+            last = c;
+            iterations = done;
+            if (c.errors) {
+                b->stats.errors = c.errors;
+                status = fail(RMD_ERROR_QUEUE_OVERFLOW, "device error flags " + std::to_string(c.errors));
+            } else if (c.pathsDone < numPaths && done > maxIters) {
+                status = fail(RMD_ERROR_WATCHDOG, "render did not drain in the iteration bound");
             }
-            if ((e = guideTrainStep(guide, h, cnt, net, b->ctx->smCount, st, trainSteps)) != RMD_OK) return e;
-            if (h.pathsDone >= numPaths) done = true;
-            else if (iterations > maxIters) return fail(RMD_ERROR_WATCHDOG, "render did not drain in the iteration bound");
+            return status != RMD_OK || c.pathsDone >= numPaths;
+        };
+        if (!guide.settings.training) {
+            RMD_CUDA(rmdhost::driveWavefront(cnt, numPaths, b->capacity, b->hostCounters, &b->ev[2], st, iterate, check));
+        } else {
+            for (bool over = false; !over;) {
+                for (uint32_t k = 0; k < 4; k++) RMD_CUDA(iterate(k & 1u, allPaths));
+                RMD_CUDA(cudaMemcpyAsync(b->hostCounters, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+                RMD_CUDA(cudaStreamSynchronize(st));
+                over = check(b->hostCounters[0], iterations + 4);
+                rmd_status e = status == RMD_OK ? guideTrainStep(guide, b->hostCounters[0], cnt, net, b->ctx->smCount, st, trainSteps)
+                                                : status;
+                if (e != RMD_OK) return e;
+            }
+        }
+        if (status != RMD_OK) {
+            cudaStreamSynchronize(st);
+            return status;
         }
     }
     RMD_CUDA(cudaEventRecord(b->ev[1], st));
     RMD_CUDA(cudaEventSynchronize(b->ev[1]));
     float ms = 0;
     cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
-    const Counters &h = *b->hostCounters;
+    const Counters &h = last;
     b->stats.paths = h.pathsDone;
     b->stats.segments = h.segments;
     b->stats.rays = h.rays;
