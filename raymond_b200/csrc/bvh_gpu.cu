@@ -20,11 +20,12 @@
 //     regular geometry (grids of equal triangles) still merges in parallel;
 //     an iteration that merges fewer than 1/16 of the clusters is replaced
 //     by merging Morton neighbours pairwise, which bounds the iteration count.
+//     One cooperative launch runs all iterations.
 //  4. The SAH-optimal collapse into 8-wide nodes, as the host builder makes
-//     it (Ylitie, Karras and Laine 2017, section 3.1): bottom up, one launch
-//     per clustering iteration (a node's children were made in earlier
-//     iterations), every binary node gets the least surface-area cost of its
-//     subtree as at most 1..8 slots of its parent (a leaf of at most 3
+//     it (Ylitie, Karras and Laine 2017, section 3.1): when it is made (its
+//     children were made in earlier iterations), every binary node gets the
+//     least surface-area cost of its subtree as at most 1..8 slots of its
+//     parent (a leaf of at most 3
 //     triangles, an inner node, or a spread over several slots) and the
 //     choices that reach it.  Then level by level from the root, each node
 //     collects its slots from those choices, places the children in octant
@@ -34,9 +35,11 @@
 //     collapsed again greedily (open the inner child of largest area until a
 //     node has 8 children).
 //
-// Every kernel's indexes are bounded by its element count; the host loop
-// reads one 8-byte total per clustering iteration and per tree level.
+// Every kernel's indexes are bounded by its element count; the host reads the
+// clustering's result and one 8-byte total per tree level.
 #include "bvh_gpu.h"
+
+#include <cooperative_groups.h>
 
 #include <cfloat>
 #include <cmath>
@@ -47,6 +50,7 @@
 #include <vector>
 
 #include "bvh_build.h"
+#include "device/traverse.cuh"
 
 namespace rmd {
 namespace {
@@ -327,87 +331,6 @@ __global__ void k_bvh_leaves(const uint32_t *sortedTri, uint32_t n, const float4
     }
 }
 
-// nearest neighbour of each cluster within kRadius positions
-constexpr int kNnThreads = 256;
-__global__ void __launch_bounds__(kNnThreads) k_ploc_nn(const float4 *clLo, const float4 *clHi, uint32_t n,
-                                                         int radius, uint32_t *nn) {
-    __shared__ float4 sLo[kNnThreads + 2 * kMaxRadius], sHi[kNnThreads + 2 * kMaxRadius];
-    const int64_t base = (int64_t)blockIdx.x * kNnThreads;
-    for (int k = threadIdx.x; k < kNnThreads + 2 * radius; k += kNnThreads) {
-        const int64_t j = base - radius + k;
-        if (j >= 0 && j < (int64_t)n) {
-            sLo[k] = clLo[j];
-            sHi[k] = clHi[j];
-        }
-    }
-    __syncthreads();
-    const int64_t i = base + threadIdx.x;
-    if (i >= (int64_t)n) return;
-    const float4 al = sLo[threadIdx.x + radius], ah = sHi[threadIdx.x + radius];
-    uint64_t best = ~0ull;
-    uint32_t bestJ = 0u;
-    for (int d = -radius; d <= radius; d++) {
-        const int64_t j = i + d;
-        if (d == 0 || j < 0 || j >= (int64_t)n) continue;
-        const float c = unionArea(al, ah, sLo[threadIdx.x + radius + d], sHi[threadIdx.x + radius + d]);
-        // cost >= 0, so its bits order like the float; the hash orders ties
-        const uint64_t key = ((uint64_t)__float_as_uint(fmaxf(c, 0.0f)) << 32) | pairHash((uint32_t)i, (uint32_t)j);
-        if (key < best) {
-            best = key;
-            bestJ = (uint32_t)j;
-        }
-    }
-    nn[i] = bestJ;
-}
-
-// per cluster: (survives, leads a merge).  pairwise: merge Morton neighbours
-// (2k, 2k + 1) instead of mutual nearest neighbours.
-__global__ void k_ploc_flags(uint32_t *nn, uint32_t n, int pairwise, uint2 *flags) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        bool leader, follower;
-        if (pairwise) {
-            leader = (i & 1u) == 0u && i + 1u < n;
-            follower = (i & 1u) == 1u;
-            if (leader) nn[i] = i + 1u;
-        } else {
-            const uint32_t j = nn[i];
-            const bool mutual = nn[j] == i;
-            leader = mutual && i < j;
-            follower = mutual && i > j;
-        }
-        flags[i] = make_uint2(follower ? 0u : 1u, leader ? 1u : 0u);
-    }
-}
-
-// survivors to their scanned positions; leaders create the merged node
-__global__ void k_ploc_compact(const uint32_t *cl, const float4 *clLo, const float4 *clHi, const uint32_t *nn,
-                               const uint2 *flags, const uint2 *pos, uint32_t n, uint32_t nodeBase, uint32_t *clOut,
-                               float4 *clLoOut, float4 *clHiOut, float4 *nodeLo, float4 *nodeHi, int2 *nodeChild) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint2 f = flags[i];
-        if (!f.x) continue;
-        const uint32_t p = pos[i].x;
-        if (f.y) {
-            const uint32_t j = nn[i];
-            const float4 al = clLo[i], ah = clHi[i], bl = clLo[j], bh = clHi[j];
-            const uint32_t count = __float_as_uint(al.w) + __float_as_uint(bl.w);
-            const float4 l = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __uint_as_float(count));
-            const float4 h = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.0f);
-            const uint32_t id = nodeBase + pos[i].y;
-            nodeLo[id] = l;
-            nodeHi[id] = h;
-            nodeChild[id] = make_int2((int)cl[i], (int)cl[j]);
-            clOut[p] = id;
-            clLoOut[p] = l;
-            clHiOut[p] = h;
-        } else {
-            clOut[p] = cl[i];
-            clLoOut[p] = clLo[i];
-            clHiOut[p] = clHi[i];
-        }
-    }
-}
-
 // ------------------------------------------------------- optimal collapse
 // cost[8 i + s - 1]: the least cost of node i's subtree given as at most s
 // slots of its parent (leaf slot: area * triangles; inner node: area + its
@@ -431,47 +354,220 @@ __global__ void k_dp_leaves(const float4 *lo, const float4 *hi, uint32_t n, floa
     }
 }
 
-__global__ void k_dp_nodes(const float4 *lo, const float4 *hi, const int2 *child, uint32_t base, uint32_t count,
-                           float *cost, uint8_t *choice, uint8_t *split) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
-        const size_t i = (size_t)base + j;
-        const int2 ch = child[i];
-        const float4 l = lo[i], h = hi[i];
-        const uint32_t tris = __float_as_uint(l.w);
-        const float area = boxArea(l, h);
-        const float leaf = tris <= kLeafTris ? area * (float)tris : FLT_MAX;
-        float cl[8], cr[8];
-        for (int k = 0; k < 8; k++) {
-            cl[k] = cost[8 * (size_t)ch.x + k];
-            cr[k] = cost[8 * (size_t)ch.y + k];
+// node i's costs and choices from its children's
+__device__ void dpNode(size_t i, int2 ch, float4 l, float4 h, float *cost, uint8_t *choice, uint8_t *split) {
+    const uint32_t tris = __float_as_uint(l.w);
+    const float area = boxArea(l, h);
+    const float leaf = tris <= kLeafTris ? area * (float)tris : FLT_MAX;
+    float cl[8], cr[8];
+    for (int k = 0; k < 8; k++) {
+        cl[k] = cost[8 * (size_t)ch.x + k];
+        cr[k] = cost[8 * (size_t)ch.y + k];
+    }
+    float dist[9];
+    uint8_t distK[9];
+    for (int s = 2; s <= 8; s++) {
+        dist[s] = FLT_MAX;
+        distK[s] = 1;
+        for (int k = 1; k < s; k++) {
+            const float v = cl[k - 1] + cr[s - k - 1];
+            if (v < dist[s]) {
+                dist[s] = v;
+                distK[s] = (uint8_t)k;
+            }
         }
-        float dist[9];
-        uint8_t distK[9];
-        for (int s = 2; s <= 8; s++) {
-            dist[s] = FLT_MAX;
-            distK[s] = 1;
-            for (int k = 1; k < s; k++) {
-                const float v = cl[k - 1] + cr[s - k - 1];
-                if (v < dist[s]) {
-                    dist[s] = v;
-                    distK[s] = (uint8_t)k;
+    }
+    const float inner = area + dist[8];
+    split[i] = distK[8];
+    float c = fminf(leaf, inner);
+    cost[8 * i] = c;
+    choice[8 * i] = tris <= kLeafTris && leaf <= inner ? 1 : 0;
+    for (int s = 2; s <= 8; s++) {
+        if (dist[s] <= c) {
+            c = dist[s];
+            choice[8 * i + s - 1] = distK[s];
+        } else {
+            choice[8 * i + s - 1] = 0;
+        }
+        cost[8 * i + s - 1] = c;
+    }
+}
+
+// ------------------------------------------------------------- clustering
+constexpr uint32_t kClusterThreads = 256;
+constexpr uint32_t kClusterWarps = kClusterThreads / 32;
+constexpr uint32_t kAlone = 512;           // clusters from which one block goes on alone
+constexpr uint32_t kMaxClusterIterations = 4096;
+
+struct ClusterArgs {
+    uint32_t *cl[2];            // binary node of each cluster, in Morton order; double buffered
+    float4 *clLo[2], *clHi[2];  // its box
+    uint32_t *nn;               // the position each cluster would merge with
+    float4 *nodeLo, *nodeHi;
+    int2 *nodeChild;
+    float *dpCost;
+    uint8_t *dpChoice, *dpSplit;
+    uint2 *blockTotals;         // per block: surviving clusters, merges
+    uint32_t *result;           // root, iterations, whether it converged
+    uint32_t n;
+    int radius;
+};
+
+struct ClusterFate {
+    bool survives, leads;  // a merge
+};
+__device__ __forceinline__ ClusterFate clusterFate(const uint32_t *nn, uint32_t i, uint32_t n, bool pairwise) {
+    if (pairwise) return {(i & 1u) == 0u, (i & 1u) == 0u && i + 1u < n};
+    const uint32_t j = nn[i];
+    const bool mutual = nn[j] == i;
+    return {!(mutual && i > j), mutual && i < j};
+}
+
+// The whole clustering in one cooperative launch.  Each iteration every block
+// takes a contiguous run of the clusters: finds their nearest neighbours
+// within `radius` positions, counts its survivors and merges, and, with the
+// other blocks' counts, moves the survivors to their places in the next
+// iteration's arrays and makes the merged nodes, costs and choices of the
+// optimal collapse included (the children's are there since an earlier
+// iteration); grid barriers stand between.  The last kAlone clusters, half of
+// the iterations, are one block's work with block barriers.
+//
+// Bound by latency: 852 k triangles take 61 iterations, and as five launches,
+// a three-kernel scan and an 8-byte read by the host each they cost 3.4 ms of
+// which the kernels ran 1.9.
+__global__ void __launch_bounds__(kClusterThreads) k_cluster(ClusterArgs A) {
+    __shared__ float4 sLo[kClusterThreads + 2 * kMaxRadius], sHi[kClusterThreads + 2 * kMaxRadius];
+    __shared__ uint2 sums[kClusterWarps];
+    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const int radius = A.radius;
+    uint32_t clusters = A.n, nodeBase = A.n, iterations = 0;
+    int c = 0;
+    while (clusters > 1u && iterations < kMaxClusterIterations) {
+        iterations++;
+        const bool alone = clusters <= kAlone;
+        if (alone && blockIdx.x != 0u) return;
+        const uint32_t blocks = alone ? 1u : gridDim.x;
+        const uint32_t per = ((clusters + blocks - 1u) / blocks + kClusterThreads - 1u) / kClusterThreads * kClusterThreads;
+        const uint32_t begin = min(blockIdx.x * per, clusters), end = min(begin + per, clusters);
+        uint32_t *cl = A.cl[c];
+        float4 *lo = A.clLo[c], *hi = A.clHi[c];
+        // nearest neighbour of each cluster within `radius` positions
+        for (uint32_t base = begin; base < end; base += kClusterThreads) {
+            for (uint32_t k = tid; k < kClusterThreads + 2u * radius; k += kClusterThreads) {
+                const int64_t j = (int64_t)base - radius + k;
+                if (j >= 0 && j < (int64_t)clusters) {
+                    sLo[k] = lo[j];
+                    sHi[k] = hi[j];
+                }
+            }
+            __syncthreads();
+            const uint32_t i = base + tid;
+            if (i < end) {
+                const float4 al = sLo[tid + radius], ah = sHi[tid + radius];
+                uint64_t best = ~0ull;
+                uint32_t bestJ = 0u;
+                for (int d = -radius; d <= radius; d++) {
+                    const int64_t j = (int64_t)i + d;
+                    if (d == 0 || j < 0 || j >= (int64_t)clusters) continue;
+                    const float a = unionArea(al, ah, sLo[tid + radius + d], sHi[tid + radius + d]);
+                    // cost >= 0, so its bits order like the float; the hash orders ties
+                    const uint64_t key = ((uint64_t)__float_as_uint(fmaxf(a, 0.0f)) << 32) | pairHash(i, (uint32_t)j);
+                    if (key < best) {
+                        best = key;
+                        bestJ = (uint32_t)j;
+                    }
+                }
+                A.nn[i] = bestJ;
+            }
+            __syncthreads();
+        }
+        if (alone) __syncthreads();
+        else grid.sync();
+        // this block's survivors and merges
+        uint32_t survivors = 0, merges = 0;
+        for (uint32_t i = begin + tid; i < end; i += kClusterThreads) {
+            const ClusterFate f = clusterFate(A.nn, i, clusters, false);
+            survivors += f.survives;
+            merges += f.leads;
+        }
+        survivors = __reduce_add_sync(0xffffffffu, survivors);
+        merges = __reduce_add_sync(0xffffffffu, merges);
+        if (lane == 0u) sums[warp] = make_uint2(survivors, merges);
+        __syncthreads();
+        if (tid == 0u) {
+            uint2 t = make_uint2(0u, 0u);
+            for (uint32_t w = 0; w < kClusterWarps; w++) t = t + sums[w];
+            A.blockTotals[blockIdx.x] = t;
+        }
+        if (alone) __syncthreads();
+        else grid.sync();
+        // all blocks' totals, and those before this one
+        uint2 before = make_uint2(0u, 0u), total = make_uint2(0u, 0u);
+        for (uint32_t k = lane; k < blocks; k += 32u) {  // every warp sums all of them
+            const uint2 t = A.blockTotals[k];
+            total = total + t;
+            if (k < blockIdx.x) before = before + t;
+        }
+        total = make_uint2(__reduce_add_sync(0xffffffffu, total.x), __reduce_add_sync(0xffffffffu, total.y));
+        before = make_uint2(__reduce_add_sync(0xffffffffu, before.x), __reduce_add_sync(0xffffffffu, before.y));
+        // too few mutual pairs: merge neighbours pairwise
+        const bool pairwise = total.y < max(1u, clusters / 16u);
+        if (pairwise) {
+            total = make_uint2((clusters + 1u) / 2u, clusters / 2u);
+            before = make_uint2((begin + 1u) / 2u, begin / 2u);
+        }
+        // survivors to their places; leaders make the merged node
+        uint32_t *clOut = A.cl[c ^ 1];
+        float4 *loOut = A.clLo[c ^ 1], *hiOut = A.clHi[c ^ 1];
+        for (uint32_t base = begin; base < end; base += kClusterThreads) {
+            const uint32_t i = base + tid;
+            ClusterFate f = {false, false};
+            if (i < end) f = clusterFate(A.nn, i, clusters, pairwise);
+            const uint32_t keep = __ballot_sync(0xffffffffu, f.survives), lead = __ballot_sync(0xffffffffu, f.leads);
+            __syncthreads();  // the previous use of sums
+            if (lane == 0u) sums[warp] = make_uint2(__popc(keep), __popc(lead));
+            __syncthreads();
+            uint2 at = before;
+            for (uint32_t w = 0; w < kClusterWarps; w++) {
+                if (w < warp) at = at + sums[w];
+                before = before + sums[w];
+            }
+            if (f.survives) {
+                const uint32_t below = (1u << lane) - 1u;
+                const uint32_t p = at.x + __popc(keep & below);
+                if (f.leads) {
+                    const uint32_t j = pairwise ? i + 1u : A.nn[i];
+                    const float4 al = lo[i], ah = hi[i], bl = lo[j], bh = hi[j];
+                    const uint32_t count = __float_as_uint(al.w) + __float_as_uint(bl.w);
+                    const float4 l = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __uint_as_float(count));
+                    const float4 h = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.0f);
+                    const uint32_t id = nodeBase + at.y + __popc(lead & below);
+                    const int2 ch = make_int2((int)cl[i], (int)cl[j]);
+                    A.nodeLo[id] = l;
+                    A.nodeHi[id] = h;
+                    A.nodeChild[id] = ch;
+                    clOut[p] = id;
+                    loOut[p] = l;
+                    hiOut[p] = h;
+                    dpNode(id, ch, l, h, A.dpCost, A.dpChoice, A.dpSplit);
+                } else {
+                    clOut[p] = cl[i];
+                    loOut[p] = lo[i];
+                    hiOut[p] = hi[i];
                 }
             }
         }
-        const float inner = area + dist[8];
-        split[i] = distK[8];
-        float c = fminf(leaf, inner);
-        cost[8 * i] = c;
-        choice[8 * i] = tris <= kLeafTris && leaf <= inner ? 1 : 0;
-        for (int s = 2; s <= 8; s++) {
-            if (dist[s] <= c) {
-                c = dist[s];
-                choice[8 * i + s - 1] = distK[s];
-            } else {
-                choice[8 * i + s - 1] = 0;
-            }
-            cost[8 * i + s - 1] = c;
-        }
+        if (alone) __syncthreads();
+        else grid.sync();
+        nodeBase += total.y;
+        clusters = total.x;
+        c ^= 1;
+    }
+    if (blockIdx.x == 0u && tid == 0u) {
+        A.result[0] = A.cl[c][0];
+        A.result[1] = iterations;
+        A.result[2] = clusters <= 1u ? 1u : 0u;
     }
 }
 
@@ -672,11 +768,19 @@ __global__ void k_collapse_emit(Tree t, const uint2 *entries, uint32_t m, const 
                 const int2 ch = t.child[x];
                 if (ch.x < 0) {
                     const uint32_t tri = (uint32_t)ch.y;
-                    float4 *o = &tris[3 * ((size_t)w.triBase + triAt)];
+                    float4 *o = &tris[TRI_FLOAT4 * ((size_t)w.triBase + triAt)];
                     const float3 a = load3(v0, tri), b = load3(v1, tri), cc = load3(v2, tri);
-                    o[0] = make_float4(a.x, a.y, a.z, __uint_as_float(inst[tri]));
-                    o[1] = make_float4(b.x, b.y, b.z, __uint_as_float(prim[tri]));
-                    o[2] = make_float4(cc.x, cc.y, cc.z, 0.0f);
+                    const float wa = __uint_as_float(inst[tri]), wb = __uint_as_float(prim[tri]);
+                    // the three rotated copies that traversal reads (device/traverse.cuh)
+                    o[0] = make_float4(a.y, a.z, a.x, wa);
+                    o[1] = make_float4(b.y, b.z, b.x, wb);
+                    o[2] = make_float4(cc.y, cc.z, cc.x, 0.0f);
+                    o[3] = make_float4(a.z, a.x, a.y, wa);
+                    o[4] = make_float4(b.z, b.x, b.y, wb);
+                    o[5] = make_float4(cc.z, cc.x, cc.y, 0.0f);
+                    o[6] = make_float4(a.x, a.y, a.z, wa);
+                    o[7] = make_float4(b.x, b.y, b.z, wb);
+                    o[8] = make_float4(cc.x, cc.y, cc.z, 0.0f);
                     triAt++;
                 } else if (sp + 2 <= 8) {
                     stack[sp++] = ch.y;
@@ -689,18 +793,20 @@ __global__ void k_collapse_emit(Tree t, const uint2 *entries, uint32_t m, const 
 }
 
 // --------------------------------------------------------------- host side
-struct Scratch {
-    std::vector<void *> ptrs;
-    ~Scratch() {
-        for (void *p : ptrs) cudaFree(p);
+// The builder's workspace: one allocation, carved into arrays on 256 bytes.
+// (As 45 allocations it cost more than the build: 25 ms, and up to 125 ms in a
+// process that had freed large blocks before.)
+struct Workspace {
+    char *base = nullptr;
+    size_t used = 0;
+    ~Workspace() {
+        if (base) cudaFree(base);
     }
     template <class T>
-    cudaError_t alloc(T *&p, size_t count) {
-        void *q = nullptr;
-        const cudaError_t e = cudaMalloc(&q, std::max<size_t>(1, count) * sizeof(T));
-        if (e == cudaSuccess) ptrs.push_back(q);
-        p = static_cast<T *>(q);
-        return e;
+    T *take(size_t count) {  // null while only sizes are counted
+        T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (std::max<size_t>(1, count) * sizeof(T) + 255) & ~size_t(255);
+        return p;
     }
 };
 
@@ -743,36 +849,62 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
         out.error = "the device BVH builder takes at most 2^24 triangles";
         return cudaErrorInvalidValue;
     }
-    Scratch S;
+    Workspace S;
     float4 *triLo, *triHi, *nodeLo, *nodeHi, *clLo[2], *clHi[2];
     int2 *nodeChild;
     uint64_t *keys[2];
-    uint32_t *vals[2], *centroidBounds, *counts, *offsets, *countPartials, *countTotal, *cl[2], *nn;
-    uint2 *flags, *pos, *pairPartials, *pairTotal;
+    uint32_t *vals[2], *centroidBounds, *counts, *offsets, *countPartials, *countTotal, *cl[2], *nn, *result;
+    uint2 *blockTotals, *entries[2], *plan, *planPos, *pairPartials, *pairTotal;
+    float *dpCost;
+    uint8_t *dpChoice, *dpSplit;
+    int *slots;
+    GpuWideNode *wide;
     const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
     const size_t nodes2 = 2 * (size_t)n;
-    BVH_TRY(S.alloc(triLo, n));
-    BVH_TRY(S.alloc(triHi, n));
-    BVH_TRY(S.alloc(nodeLo, nodes2));
-    BVH_TRY(S.alloc(nodeHi, nodes2));
-    BVH_TRY(S.alloc(nodeChild, nodes2));
-    for (int b = 0; b < 2; b++) {
-        BVH_TRY(S.alloc(keys[b], n));
-        BVH_TRY(S.alloc(vals[b], n));
-        BVH_TRY(S.alloc(cl[b], n));
-        BVH_TRY(S.alloc(clLo[b], n));
-        BVH_TRY(S.alloc(clHi[b], n));
-    }
-    BVH_TRY(S.alloc(centroidBounds, 6));
-    BVH_TRY(S.alloc(counts, 256 * (size_t)tiles));
-    BVH_TRY(S.alloc(offsets, 256 * (size_t)tiles));
-    BVH_TRY(S.alloc(countPartials, kScanTile));
-    BVH_TRY(S.alloc(countTotal, 1));
-    BVH_TRY(S.alloc(nn, n));
-    BVH_TRY(S.alloc(flags, n));
-    BVH_TRY(S.alloc(pos, n));
-    BVH_TRY(S.alloc(pairPartials, kScanTile));
-    BVH_TRY(S.alloc(pairTotal, 1));
+    int device = 0, sms = 0, perSm = 0;
+    BVH_TRY(cudaGetDevice(&device));
+    BVH_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    BVH_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_cluster, kClusterThreads, 0));
+    const uint32_t clusterBlocks = std::min<uint32_t>((uint32_t)std::max(1, perSm * sms), (n + kClusterThreads - 1) / kClusterThreads);
+    const auto carve = [&] {
+        S.used = 0;
+        triLo = S.take<float4>(n);
+        triHi = S.take<float4>(n);
+        nodeLo = S.take<float4>(nodes2);
+        nodeHi = S.take<float4>(nodes2);
+        nodeChild = S.take<int2>(nodes2);
+        dpCost = S.take<float>(8 * nodes2);
+        dpChoice = S.take<uint8_t>(8 * nodes2);
+        dpSplit = S.take<uint8_t>(nodes2);
+        for (int b = 0; b < 2; b++) {
+            keys[b] = S.take<uint64_t>(n);
+            vals[b] = S.take<uint32_t>(n);
+            cl[b] = S.take<uint32_t>(n);
+            clLo[b] = S.take<float4>(n);
+            clHi[b] = S.take<float4>(n);
+        }
+        centroidBounds = S.take<uint32_t>(6);
+        counts = S.take<uint32_t>(256 * (size_t)tiles);
+        offsets = S.take<uint32_t>(256 * (size_t)tiles);
+        countPartials = S.take<uint32_t>(kScanTile);
+        countTotal = S.take<uint32_t>(1);
+        nn = S.take<uint32_t>(n);
+        blockTotals = S.take<uint2>(clusterBlocks);
+        result = S.take<uint32_t>(3);
+        pairPartials = S.take<uint2>(kScanTile);
+        pairTotal = S.take<uint2>(1);
+        wide = S.take<GpuWideNode>(n);
+        entries[0] = S.take<uint2>(n);
+        entries[1] = S.take<uint2>(n);
+        slots = S.take<int>(8 * (size_t)n);
+        plan = S.take<uint2>(n);
+        planPos = S.take<uint2>(n);
+    };
+    carve();
+    BVH_TRY(cudaMalloc(reinterpret_cast<void **>(&S.base), S.used));
+    carve();
+    BVH_TRY(cudaMalloc(&out.tris, (size_t)n * TRI_FLOAT4 * sizeof(float4)));
+    float4 *tris = static_cast<float4 *>(out.tris);
 
     // 1. boxes and centroid bounds
     const uint32_t initBounds[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
@@ -794,68 +926,26 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
     k_bvh_leaves<<<gridFor(n, 256), 256, 0, s>>>(vals[cur], n, triLo, triHi, nodeLo, nodeHi, nodeChild, cl[0],
                                                  clLo[0], clHi[0]);
     BVH_TRY(cudaGetLastError());
+    k_dp_leaves<<<gridFor(n, 256), 256, 0, s>>>(nodeLo, nodeHi, n, dpCost, dpChoice);
+    BVH_TRY(cudaGetLastError());
     // search radius: RMD_BVH_RADIUS overrides the default (1..64)
     int radius = kRadius;
     if (const char *env = std::getenv("RMD_BVH_RADIUS")) radius = std::max(1, std::min(kMaxRadius, std::atoi(env)));
-    uint32_t clusters = n, nodeBase = n;
-    std::vector<std::pair<uint32_t, uint32_t>> made;  // (first node, count) of each clustering iteration
-    int c = 0;
-    while (clusters > 1) {
-        if (++out.clusterIterations > 4096) {
-            out.error = "device BVH clustering did not converge";
-            return cudaErrorInvalidValue;
-        }
-        k_ploc_nn<<<(clusters + kNnThreads - 1) / kNnThreads, kNnThreads, 0, s>>>(clLo[c], clHi[c], clusters, radius,
-                                                                                  nn);
-        k_ploc_flags<<<gridFor(clusters, 256), 256, 0, s>>>(nn, clusters, 0, flags);
-        BVH_TRY(exclusiveScan<uint2>(flags, pos, clusters, pairPartials, pairTotal, s));
-        uint2 total;
-        BVH_TRY(readTotal(pairTotal, total, s));
-        if (total.y < std::max<uint32_t>(1u, clusters / 16u)) {  // too few mutual pairs: merge neighbours pairwise
-            k_ploc_flags<<<gridFor(clusters, 256), 256, 0, s>>>(nn, clusters, 1, flags);
-            BVH_TRY(exclusiveScan<uint2>(flags, pos, clusters, pairPartials, pairTotal, s));
-            BVH_TRY(readTotal(pairTotal, total, s));
-        }
-        k_ploc_compact<<<gridFor(clusters, 256), 256, 0, s>>>(cl[c], clLo[c], clHi[c], nn, flags, pos, clusters,
-                                                               nodeBase, cl[c ^ 1], clLo[c ^ 1], clHi[c ^ 1], nodeLo,
-                                                               nodeHi, nodeChild);
-        BVH_TRY(cudaGetLastError());
-        made.emplace_back(nodeBase, total.y);
-        nodeBase += total.y;
-        clusters = total.x;
-        c ^= 1;
-    }
-    uint32_t root = 0;
-    BVH_TRY(cudaMemcpyAsync(&root, cl[c], sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    ClusterArgs ca = {{cl[0], cl[1]}, {clLo[0], clLo[1]}, {clHi[0], clHi[1]}, nn, nodeLo, nodeHi, nodeChild, dpCost,
+                      dpChoice, dpSplit, blockTotals, result, n, radius};
+    void *args[] = {&ca};
+    BVH_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_cluster), dim3(clusterBlocks), dim3(kClusterThreads), args, 0, s));
+    uint32_t found[3];
+    BVH_TRY(cudaMemcpyAsync(found, result, sizeof(found), cudaMemcpyDeviceToHost, s));
     BVH_TRY(cudaStreamSynchronize(s));
+    if (!found[2]) {
+        out.error = "device BVH clustering did not converge";
+        return cudaErrorInvalidValue;
+    }
+    const uint32_t root = found[0];
+    out.clusterIterations = found[1];
 
     // 4. collapse, level by level; at most n wide nodes (each has >= 2 triangles below it or is the root)
-    GpuWideNode *wide;
-    float4 *tris;
-    uint2 *entries[2];
-    int *slots;
-    uint2 *plan, *planPos;
-    BVH_TRY(cudaMalloc(&out.tris, (size_t)n * 3 * sizeof(float4)));
-    tris = static_cast<float4 *>(out.tris);
-    BVH_TRY(cudaMalloc(&out.nodes, (size_t)n * sizeof(GpuWideNode)));
-    wide = static_cast<GpuWideNode *>(out.nodes);
-    BVH_TRY(S.alloc(entries[0], n));
-    BVH_TRY(S.alloc(entries[1], n));
-    BVH_TRY(S.alloc(slots, 8 * (size_t)n));
-    BVH_TRY(S.alloc(plan, n));
-    BVH_TRY(S.alloc(planPos, n));
-    // the optimal collapse's costs and choices, bottom up
-    float *dpCost;
-    uint8_t *dpChoice, *dpSplit;
-    BVH_TRY(S.alloc(dpCost, 8 * nodes2));
-    BVH_TRY(S.alloc(dpChoice, 8 * nodes2));
-    BVH_TRY(S.alloc(dpSplit, nodes2));
-    k_dp_leaves<<<gridFor(n, 256), 256, 0, s>>>(nodeLo, nodeHi, n, dpCost, dpChoice);
-    for (const auto &r : made)
-        if (r.second > 0)
-            k_dp_nodes<<<gridFor(r.second, 128), 128, 0, s>>>(nodeLo, nodeHi, nodeChild, r.first, r.second, dpCost,
-                                                               dpChoice, dpSplit);
-    BVH_TRY(cudaGetLastError());
     const uint2 first = make_uint2(root, 0u);
     Tree t{nodeLo, nodeHi, nodeChild, dpChoice, dpSplit};
     uint32_t level = 0, width = 0, wideCount = 0, triCount = 0;
@@ -896,6 +986,8 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
                     " triangles";
         return cudaErrorInvalidValue;
     }
+    BVH_TRY(cudaMalloc(&out.nodes, (size_t)wideCount * sizeof(GpuWideNode)));
+    BVH_TRY(cudaMemcpyAsync(out.nodes, wide, (size_t)wideCount * sizeof(GpuWideNode), cudaMemcpyDeviceToDevice, s));
     out.nodeCount = wideCount;
     out.levels = level;
     return cudaStreamSynchronize(s);

@@ -11,7 +11,7 @@ namespace rmdhost {
 struct GpuBvhResult {
     void *nodes = nullptr;   // nodeCount x 80 B (GpuWideNode), cudaMalloc'd, owned by the caller
     uint64_t nodeCount = 0;
-    void *tris = nullptr;    // n x 48 B in leaf order, cudaMalloc'd, owned by the caller
+    void *tris = nullptr;    // n x 144 B in leaf order (three rotated copies), cudaMalloc'd, owned by the caller
     uint32_t levels = 0;     // levels of the 8-wide tree
     uint32_t clusterIterations = 0;
     std::string error;       // set when the build fails for a reason other than a CUDA error

@@ -640,7 +640,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
                                                        dInst.as<uint32_t>(), dPrim.as<uint32_t>(),
                                                        (uint32_t)std::min<size_t>(triInst.size(), 0xffffffffu), st, g);
         s->bvhNodes.adopt(g.nodes, g.nodeCount * sizeof(rmdhost::GpuWideNode));
-        s->bvhTris.adopt(g.tris, triInst.size() * 12 * sizeof(float));
+        s->bvhTris.adopt(g.tris, triInst.size() * TRI_FLOAT4 * sizeof(float4));
         if (e != cudaSuccess) {
             if (!g.error.empty()) return fail(RMD_ERROR_INVALID_ARGUMENT, "device BVH build: " + g.error);
             RMD_CUDA(e);
@@ -766,7 +766,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         RMD_CUDA(s->bvhNodes.upload(bvh.nodes.data(), bvh.nodes.size() * sizeof(rmdhost::GpuWideNode), st));
         RMD_CUDA(s->bvhTris.upload(bvh.tris.data(), bvh.tris.size() * sizeof(float), st));
     }
-    if (s->triangles) {  // the traversal kernels read three rotated copies of each triangle (device/traverse.cuh)
+    if (s->triangles && ctx->bvhBuilder != RMD_BVH_GPU) {  // the traversal kernels read three rotated copies of each triangle (device/traverse.cuh)
         DevBuf rotated;
         RMD_CUDA(rotated.alloc(s->triangles * TRI_FLOAT4 * sizeof(float4)));
         RMD_CUDA(rmdLaunchRotateTriangles(s->bvhTris.as<float4>(), rotated.as<float4>(), (uint32_t)s->triangles, st));
