@@ -797,10 +797,14 @@ __global__ void k_collapse_emit(Tree t, const uint2 *entries, uint32_t m, const 
 // (As 45 allocations it cost more than the build: 25 ms, and up to 125 ms in a
 // process that had freed large blocks before.)
 struct Workspace {
+    cudaStream_t stream;
     char *base = nullptr;
     size_t used = 0;
+    explicit Workspace(cudaStream_t s) : stream(s) {}
     ~Workspace() {
-        if (base) cudaFree(base);
+        if (!base) return;
+        cudaStreamSynchronize(stream);  // after an error its kernels may still run
+        cudaFree(base);
     }
     template <class T>
     T *take(size_t count) {  // null while only sizes are counted
@@ -842,14 +846,14 @@ namespace rmdhost {
 using namespace rmd;
 
 cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, const uint32_t *inst,
-                            const uint32_t *prim, uint32_t n, cudaStream_t s, GpuBvhResult &out) {
+                            const uint32_t *prim, uint32_t n, cudaStream_t s, const DeviceAlloc &alloc, GpuBvhResult &out) {
     out = GpuBvhResult();
     if (n == 0) return cudaSuccess;  // no nodes: everything misses
     if (n > kGpuBvhMaxTriangles) {
         out.error = "the device BVH builder takes at most 2^24 triangles";
         return cudaErrorInvalidValue;
     }
-    Workspace S;
+    Workspace S(s);
     float4 *triLo, *triHi, *nodeLo, *nodeHi, *clLo[2], *clHi[2];
     int2 *nodeChild;
     uint64_t *keys[2];
@@ -901,9 +905,9 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
         planPos = S.take<uint2>(n);
     };
     carve();
-    BVH_TRY(cudaMalloc(reinterpret_cast<void **>(&S.base), S.used));
+    BVH_TRY(alloc(reinterpret_cast<void **>(&S.base), S.used));
     carve();
-    BVH_TRY(cudaMalloc(&out.tris, (size_t)n * TRI_FLOAT4 * sizeof(float4)));
+    BVH_TRY(alloc(&out.tris, (size_t)n * TRI_FLOAT4 * sizeof(float4)));
     float4 *tris = static_cast<float4 *>(out.tris);
 
     // 1. boxes and centroid bounds
@@ -986,7 +990,7 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
                     " triangles";
         return cudaErrorInvalidValue;
     }
-    BVH_TRY(cudaMalloc(&out.nodes, (size_t)wideCount * sizeof(GpuWideNode)));
+    BVH_TRY(alloc(&out.nodes, (size_t)wideCount * sizeof(GpuWideNode)));
     BVH_TRY(cudaMemcpyAsync(out.nodes, wide, (size_t)wideCount * sizeof(GpuWideNode), cudaMemcpyDeviceToDevice, s));
     out.nodeCount = wideCount;
     out.levels = level;

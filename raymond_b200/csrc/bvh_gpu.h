@@ -4,14 +4,18 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <string>
 
 namespace rmdhost {
 
+// allocates device memory that cudaFree frees
+using DeviceAlloc = std::function<cudaError_t(void **, size_t)>;
+
 struct GpuBvhResult {
-    void *nodes = nullptr;   // nodeCount x 80 B (GpuWideNode), cudaMalloc'd, owned by the caller
+    void *nodes = nullptr;   // nodeCount x 80 B (GpuWideNode), allocated, owned by the caller
     uint64_t nodeCount = 0;
-    void *tris = nullptr;    // n x 144 B in leaf order (three rotated copies), cudaMalloc'd, owned by the caller
+    void *tris = nullptr;    // n x 144 B in leaf order (three rotated copies), allocated, owned by the caller
     uint32_t levels = 0;     // levels of the 8-wide tree
     uint32_t clusterIterations = 0;
     std::string error;       // set when the build fails for a reason other than a CUDA error
@@ -26,6 +30,6 @@ constexpr uint32_t kGpuBvhMaxTriangles = 1u << 24;
 // triangle).  Returns cudaErrorInvalidValue with `error` set when the input
 // is out of range or the tree would be deeper than the traversal stack.
 cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, const uint32_t *inst,
-                            const uint32_t *prim, uint32_t n, cudaStream_t s, GpuBvhResult &out);
+                            const uint32_t *prim, uint32_t n, cudaStream_t s, const DeviceAlloc &alloc, GpuBvhResult &out);
 
 }  // namespace rmdhost

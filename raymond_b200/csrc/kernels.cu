@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 
 #include "device/traverse.cuh"
 #include "device/wavefront.cuh"
@@ -507,6 +508,74 @@ __global__ void k_rotate_triangles(const float4 *__restrict__ in, float4 *__rest
     }
 }
 
+// ------------------------------------------------------------- scene building
+// The meshes' packed arrays as the shading kernels read them: positions and
+// normals on 16 bytes, faces with their material.
+__global__ void k_pack_mesh(const float *__restrict__ pos, const float *__restrict__ nrm, uint32_t numVertices,
+                            const uint32_t *__restrict__ idx, const uint16_t *__restrict__ mat, uint32_t numFaces,
+                            float4 *__restrict__ vertices, float4 *__restrict__ normals, uint4 *__restrict__ faces) {
+    const uint32_t n = max(numVertices, numFaces);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const size_t k = 3 * (size_t)i;
+        if (i < numVertices) {
+            vertices[i] = make_float4(pos[k], pos[k + 1], pos[k + 2], 0.0f);
+            normals[i] = make_float4(nrm[k], nrm[k + 1], nrm[k + 2], 0.0f);
+        }
+        if (i < numFaces) faces[i] = make_uint4(idx[k], idx[k + 1], idx[k + 2], mat[i]);
+    }
+}
+
+__device__ __forceinline__ uint32_t orderedBits(float f) {  // unsigned order = float order
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+// The world-space triangles of all instances for the device BVH builder, in
+// the host's order and arithmetic (transformPoint: products and sums rounded
+// one by one), and their bounds (3 minima, 3 maxima, as orderedBits).
+__global__ void k_flatten(const float4 *__restrict__ vertices, const uint4 *__restrict__ faces,
+                          const PerInstanceData *__restrict__ instances, uint32_t numInstances, uint32_t n,
+                          float *__restrict__ v0, float *__restrict__ v1, float *__restrict__ v2,
+                          uint32_t *__restrict__ inst, uint32_t *__restrict__ prim, uint32_t *bounds) {
+    float lo[3] = {inf_f(), inf_f(), inf_f()}, hi[3] = {-inf_f(), -inf_f(), -inf_f()};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t a = 0, b = numInstances;  // the last instance that starts at or before i
+        while (b - a > 1u) {
+            const uint32_t m = (a + b) >> 1;
+            if (instances[m].triOffset <= i) a = m;
+            else b = m;
+        }
+        const PerInstanceData &in = instances[a];
+        const uint4 f = faces[in.faceOffset + (i - in.triOffset)];
+        const uint32_t vi[3] = {f.x, f.y, f.z};
+        float *const out[3] = {v0, v1, v2};
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const float4 p = vertices[in.vertexOffset + vi[j]];
+            const float4 *M = in.pointTransform;
+            float w[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const float x = __fmul_rn(comp(xyz(M[0]), k), p.x), y = __fmul_rn(comp(xyz(M[1]), k), p.y);
+                const float z = __fmul_rn(comp(xyz(M[2]), k), p.z);
+                w[k] = __fadd_rn(__fadd_rn(__fadd_rn(x, y), z), comp(xyz(M[3]), k));
+                lo[k] = fminf(lo[k], w[k]);
+                hi[k] = fmaxf(hi[k], w[k]);
+                out[j][3 * (size_t)i + k] = w[k];
+            }
+        }
+        inst[i] = a;
+        prim[i] = i - in.triOffset;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint32_t l = __reduce_min_sync(0xffffffffu, orderedBits(lo[k])), h = __reduce_max_sync(0xffffffffu, orderedBits(hi[k]));
+        if ((threadIdx.x & 31u) == 0u) {
+            atomicMin(&bounds[k], l);
+            atomicMax(&bounds[3 + k], h);
+        }
+    }
+}
+
 }  // namespace rmd
 
 // ------------------------------------------------------------- launch wrappers
@@ -572,6 +641,33 @@ cudaError_t rmdLaunchFilmResolve(const float4 *film, const double *film64, int f
 cudaError_t rmdLaunchDebugPrng(uint32_t mode, uint64_t a, uint64_t b, int n, float *out, cudaStream_t s) {
     k_debug_prng<<<1, 1, 0, s>>>(mode, a, b, n, out);
     return cudaGetLastError();
+}
+cudaError_t rmdLaunchPackMesh(const float *pos, const float *nrm, uint32_t numVertices, const uint32_t *idx,
+                              const uint16_t *mat, uint32_t numFaces, float4 *vertices, float4 *normals, uint4 *faces,
+                              cudaStream_t s) {
+    const uint32_t n = std::max(numVertices, numFaces);
+    if (n == 0) return cudaSuccess;
+    k_pack_mesh<<<std::min<uint32_t>((n + 255) / 256, 148u * 16u), 256, 0, s>>>(pos, nrm, numVertices, idx, mat, numFaces,
+                                                                             vertices, normals, faces);
+    return cudaGetLastError();
+}
+cudaError_t rmdLaunchFlatten(const float4 *vertices, const uint4 *faces, const PerInstanceData *instances,
+                             uint32_t numInstances, uint32_t n, float *v0, float *v1, float *v2, uint32_t *inst,
+                             uint32_t *prim, uint32_t *boundsScratch, float *bounds, cudaStream_t s) {
+    uint32_t b[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
+    cudaError_t e = cudaMemcpyAsync(boundsScratch, b, sizeof(b), cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    k_flatten<<<std::min<uint32_t>((n + 255) / 256, 148u * 16u), 256, 0, s>>>(vertices, faces, instances, numInstances, n,
+                                                                           v0, v1, v2, inst, prim, boundsScratch);
+    if ((e = cudaGetLastError()) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b, boundsScratch, sizeof(b), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        return e;
+    for (int k = 0; k < 6; k++) {
+        const uint32_t u = (b[k] & 0x80000000u) ? (b[k] & 0x7fffffffu) : ~b[k];
+        memcpy(&bounds[k], &u, sizeof(float));
+    }
+    return cudaSuccess;
 }
 cudaError_t rmdLaunchRotateTriangles(const float4 *in, float4 *out, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;

@@ -33,6 +33,14 @@ cudaError_t rmdLaunchFilmResolve(const float4 *film, const double *film64, int f
                                  float exposure, float divisor, uint32_t tonemapping, uint32_t channels,
                                  cudaStream_t s);
 cudaError_t rmdLaunchDebugPrng(uint32_t mode, uint64_t a, uint64_t b, int n, float *out, cudaStream_t s);
+// the packed mesh arrays as the shading kernels read them
+cudaError_t rmdLaunchPackMesh(const float *pos, const float *nrm, uint32_t numVertices, const uint32_t *idx,
+                              const uint16_t *mat, uint32_t numFaces, float4 *vertices, float4 *normals, uint4 *faces,
+                              cudaStream_t s);
+// world-space triangles of all instances (n in all) and their bounds (host; min xyz, max xyz), waiting for them
+cudaError_t rmdLaunchFlatten(const float4 *vertices, const uint4 *faces, const rmd::PerInstanceData *instances,
+                             uint32_t numInstances, uint32_t n, float *v0, float *v1, float *v2, uint32_t *inst,
+                             uint32_t *prim, uint32_t *boundsScratch, float *bounds, cudaStream_t s);
 // three rotated copies per triangle (the traversal kernels' layout) from n x (v0, v1, v2)
 cudaError_t rmdLaunchRotateTriangles(const float4 *in, float4 *out, uint32_t n, cudaStream_t s);
 cudaError_t rmdLaunchDebugTrace(const rmd::WideNode *nodes, const float4 *tris, const float *rays, int n, int any,

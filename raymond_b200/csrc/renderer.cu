@@ -83,7 +83,6 @@ rmd_status fail(rmd_status s, const std::string &msg) {
                         std::string(#expr) + ": " + cudaGetErrorString(e_));                               \
     } while (0)
 
-// Device buffer owned by a scene or renderer.
 // Register budget of the shading kernel before autotuning: at least this many
 // 128-thread blocks per SM (measured best on the 1080p benchmark scene: 5-6);
 // RMD_SHADE_MIN_BLOCKS overrides it.
@@ -93,9 +92,46 @@ static int defaultShadeMinBlocks() {
     return v >= 1 && v <= 16 ? v : 5;
 }
 
+// A context's device memory: blocks that its scenes, renderers and batches free
+// stay with it for the next ones, up to kMemoryKept bytes; beyond that, and
+// with the context, they go back to the device.  cudaMalloc and cudaFree of
+// the 10-500 MB blocks that a scene and its renderer take cost 1-10 ms each,
+// and now and then hundreds (the 852 k-triangle scene: 20 ms to 4 s of a
+// creation); a block that the pool holds costs microseconds.  Any thread may
+// allocate and free.
+struct DevPool {
+    static constexpr uint64_t kMemoryKept = 2ull << 30;
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;  // orders the allocations alone; waited for by each
+    cudaError_t create(int device) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        uint64_t kept = kMemoryKept;
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        return e;
+    }
+    // The block may be used on any stream at once: its allocation has completed.
+    cudaError_t alloc(void **p, size_t n) const {
+        cudaError_t e = cudaMallocFromPoolAsync(p, n, pool, stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+    }
+    ~DevPool() {  // blocks in use stay valid; the pool goes with the last of them
+        if (stream) cudaStreamDestroy(stream);
+        if (pool) cudaMemPoolDestroy(pool);
+    }
+};
+
+// Device buffer owned by a scene, renderer or batch, from its context's pool
+// where one is set.  Whoever frees it has waited for the work that uses it:
+// cudaFree of a pool's block does not.
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
+    const DevPool *from = nullptr;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
@@ -109,9 +145,9 @@ struct DevBuf {
         release();
         bytes = n;
         if (n == 0) return cudaSuccess;
-        return cudaMalloc(&ptr, n);
+        return from ? from->alloc(&ptr, n) : cudaMalloc(&ptr, n);
     }
-    void adopt(void *p, size_t n) {  // takes ownership of a cudaMalloc'd block
+    void adopt(void *p, size_t n) {  // takes ownership of an allocated block
         release();
         ptr = p;
         bytes = n;
@@ -140,6 +176,7 @@ struct rmd_context {
     int smCount = 148;
     cudaStream_t stream = nullptr;
     uint32_t bvhBuilder = RMD_BVH_HOST;  // builder of the scenes created next
+    DevPool memory;
 };
 
 struct rmd_scene {
@@ -164,7 +201,14 @@ struct rmd_scene {
     int shadeBlocks = 0, traceBlocks = 0, regenBlocks = 0;
     int defaultMinBlocks = 1;
     bool ownsModule = true;  // false for the scenes of a batch (the batch owns the shared module)
+    void takeMemoryFrom(const DevPool &p) {
+        for (DevBuf *b : {&vertices, &normals, &texcoords, &faces, &instances, &lightFaces, &envPdfs, &envMipmap, &areaLights,
+                          &pointLights, &sunLights, &spotLights, &shapeLights, &surfaceTable, &lightTable, &materialParams,
+                          &bvhNodes, &bvhTris, &textureTexels, &textureViews})
+            b->from = &p;
+    }
     ~rmd_scene() {
+        cudaDeviceSynchronize();
         for (auto &kv : variants) rmdhost::unloadModule(*kv.second);
         if (ownsModule) rmdhost::unloadModule(jit);
     }
@@ -181,6 +225,9 @@ struct GuideState {
     uint32_t recordCapacity = 0;  // nonzero-target records the replay ring holds
     bool initialised = false;
     float3 frameMin = {0, 0, 0}, frameInvExtent = {1, 1, 1};  // position encoding frame (scene bounds)
+    void takeMemoryFrom(const DevPool &p) {
+        for (DevBuf *b : {&mixtures, &features, &rec, &finRec, &shRec, &records}) b->from = &p;
+    }
 };
 
 struct rmd_renderer {
@@ -204,6 +251,7 @@ struct rmd_renderer {
     std::vector<int> stageOf;              // stage of the interval that ends at each event
     GuideState guide;  // learned path guiding
     ~rmd_renderer() {
+        cudaDeviceSynchronize();
         if (hostCounters) cudaFreeHost(hostCounters);
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
@@ -253,6 +301,7 @@ struct rmd_batch {
     cudaGraphExec_t graphExec = nullptr;
     std::vector<uint64_t> graphKey;
     ~rmd_batch() {
+        cudaDeviceSynchronize();
         if (graphExec) cudaGraphExecDestroy(graphExec);
         if (graph) cudaGraphDestroy(graph);
         if (hostCounters) cudaFreeHost(hostCounters);
@@ -411,6 +460,7 @@ rmd_status rmd_context_create(int32_t device, rmd_context **out) {
     c->device = device;
     RMD_CUDA(cudaSetDevice(device));
     RMD_CUDA(cudaDeviceGetAttribute(&c->smCount, cudaDevAttrMultiProcessorCount, device));
+    RMD_CUDA(c->memory.create(device));
     RMD_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     const rmd_status ns = rmdhost::noallocSetup(device);
     if (ns != RMD_OK) {
@@ -503,6 +553,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
                                  const rmd_texture *textures, int numTextures) {
     cudaStream_t st = ctx->stream;
     s->ctx = ctx;
+    s->takeMemoryFrom(ctx->memory);
     s->numSurface = d->num_surface_materials;
     s->numLight = d->num_light_materials;
 
@@ -512,56 +563,110 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         float boundsMin[3], boundsMax[3];
         bool hasEmission;
     };
-    std::vector<ShapeInfo> shapes;
-    std::vector<float4> verts, norms;
-    std::vector<float2> uvs;
-    std::vector<uint4> faces;
-    std::vector<float> vertsPacked;  // for the light CDF
-    std::vector<uint32_t> idxPacked;
-    for (int si = 0; si < d->num_shapes; si++) {
-        const rmd_shape &sh = d->shapes[si];
+    std::vector<ShapeInfo> shapes(d->num_shapes);
+    size_t numVertices = 0, numFaces = 0;
+    int checked = 0;  // shapes up to the first without its arrays
+    for (; checked < d->num_shapes; checked++) {
+        const rmd_shape &sh = d->shapes[checked];
         if ((sh.num_vertices && (!sh.vertices || !sh.normals || !sh.texcoords)) ||
             (sh.num_faces && (!sh.indices || !sh.materials)))
-            return fail(RMD_ERROR_INVALID_ARGUMENT, "shape " + std::to_string(si) + " has NULL arrays");
-        ShapeInfo info{};
-        info.vertexOffset = (uint32_t)verts.size();
-        info.faceOffset = (uint32_t)faces.size();
-        info.faceCount = sh.num_faces;
-        for (int k = 0; k < 3; k++) {
-            info.boundsMin[k] = INFINITY;
-            info.boundsMax[k] = -INFINITY;
-        }
-        for (uint32_t v = 0; v < sh.num_vertices; v++) {
-            const float *p = sh.vertices + 3 * v;
-            for (int k = 0; k < 3; k++) {  // PLYReader.m:119-122 (else-if: the first vertex never raises the max)
-                if (p[k] < info.boundsMin[k]) info.boundsMin[k] = p[k];
-                else if (p[k] > info.boundsMax[k]) info.boundsMax[k] = p[k];
-            }
-            verts.push_back(make_float4(p[0], p[1], p[2], 0.0f));
-            vertsPacked.insert(vertsPacked.end(), p, p + 3);
-            const float *n = sh.normals + 3 * v;
-            norms.push_back(make_float4(n[0], n[1], n[2], 0.0f));
-            uvs.push_back(make_float2(sh.texcoords[2 * v], sh.texcoords[2 * v + 1]));
-        }
-        info.hasEmission = false;
-        for (uint32_t f = 0; f < sh.num_faces; f++) {
-            const uint32_t *ix = sh.indices + 3 * f;
-            if (ix[0] >= sh.num_vertices || ix[1] >= sh.num_vertices || ix[2] >= sh.num_vertices)
-                return fail(RMD_ERROR_INVALID_ARGUMENT, "vertex index out of range in shape " + std::to_string(si));
-            const uint16_t m = sh.materials[f];
-            if (m >= d->num_surface_materials)
-                return fail(RMD_ERROR_INVALID_ARGUMENT, "face material out of range in shape " + std::to_string(si));
-            faces.push_back(make_uint4(ix[0], ix[1], ix[2], m));
-            idxPacked.insert(idxPacked.end(), ix, ix + 3);
-            if (mod.surfaceEmissive[surfaceBase + m]) info.hasEmission = true;
-        }
-        shapes.push_back(info);
+            break;
+        shapes[checked].vertexOffset = (uint32_t)numVertices;
+        shapes[checked].faceOffset = (uint32_t)numFaces;
+        shapes[checked].faceCount = sh.num_faces;
+        numVertices += sh.num_vertices;
+        numFaces += sh.num_faces;
     }
+    // Bounds, and the faces' checks: the first bad face of each shape (its
+    // count: none).  All cores go over the shapes' runs of 64 k faces; the
+    // device packs the arrays.  One thread, appending to vectors element by
+    // element, took 20-30 ms for 852 k faces.
+    constexpr uint32_t kRun = 1u << 16;
+    std::vector<std::pair<int, uint32_t>> runs;  // shape, first face
+    for (int si = 0; si < checked; si++)
+        for (uint32_t f = 0; f == 0 || f < d->shapes[si].num_faces; f += kRun) runs.push_back({si, f});
+    std::vector<uint32_t> badFace(runs.size(), 0xffffffffu);
+    std::vector<uint8_t> emits(runs.size(), 0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int64_t k = 0; k < (int64_t)runs.size(); k++) {
+        const rmd_shape &sh = d->shapes[runs[k].first];
+        const uint32_t begin = runs[k].second, end = std::min(sh.num_faces, begin + kRun);
+        if (begin == 0) {
+            ShapeInfo &info = shapes[runs[k].first];
+            for (int c = 0; c < 3; c++) {
+                info.boundsMin[c] = INFINITY;
+                info.boundsMax[c] = -INFINITY;
+            }
+            for (uint32_t v = 0; v < sh.num_vertices; v++) {
+                const float *p = sh.vertices + 3 * (size_t)v;
+                for (int c = 0; c < 3; c++) {  // PLYReader.m:119-122 (else-if: the first vertex never raises the max)
+                    if (p[c] < info.boundsMin[c]) info.boundsMin[c] = p[c];
+                    else if (p[c] > info.boundsMax[c]) info.boundsMax[c] = p[c];
+                }
+            }
+        }
+        for (uint32_t f = begin; f < end; f++) {
+            const uint32_t *ix = sh.indices + 3 * (size_t)f;
+            const uint16_t m = sh.materials[f];
+            if (ix[0] >= sh.num_vertices || ix[1] >= sh.num_vertices || ix[2] >= sh.num_vertices ||
+                m >= d->num_surface_materials) {
+                badFace[k] = f;
+                break;
+            }
+            if (mod.surfaceEmissive[surfaceBase + m]) emits[k] = 1;
+        }
+    }
+    for (size_t k = 0; k < runs.size(); k++) {
+        const int si = runs[k].first;
+        if (badFace[k] != 0xffffffffu) {
+            const uint32_t *ix = d->shapes[si].indices + 3 * (size_t)badFace[k], n = d->shapes[si].num_vertices;
+            const bool vertex = ix[0] >= n || ix[1] >= n || ix[2] >= n;
+            return fail(RMD_ERROR_INVALID_ARGUMENT, std::string(vertex ? "vertex index" : "face material") +
+                                                        " out of range in shape " + std::to_string(si));
+        }
+        if (emits[k]) shapes[si].hasEmission = true;
+    }
+    if (checked < d->num_shapes)
+        return fail(RMD_ERROR_INVALID_ARGUMENT, "shape " + std::to_string(checked) + " has NULL arrays");
+    // the meshes one after the other in one block, uploaded as they are
+    const size_t posBytes = numVertices * 12, uvBytes = numVertices * 8, idxBytes = numFaces * 12;
+    const size_t meshBytes = 2 * posBytes + uvBytes + idxBytes + numFaces * 2;
+    std::unique_ptr<unsigned char[]> mesh(new unsigned char[std::max<size_t>(1, meshBytes)]);
+    unsigned char *hostPos = mesh.get(), *hostNrm = hostPos + posBytes, *hostUv = hostNrm + posBytes;
+    unsigned char *hostIdx = hostUv + uvBytes, *hostMat = hostIdx + idxBytes;
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int64_t k = 0; k < 5 * (int64_t)d->num_shapes; k++) {
+        const rmd_shape &sh = d->shapes[k / 5];
+        const ShapeInfo &info = shapes[k / 5];
+        const size_t v = info.vertexOffset, f = info.faceOffset;
+        if (k % 5 == 0 && sh.num_vertices) std::memcpy(hostPos + 12 * v, sh.vertices, 12 * (size_t)sh.num_vertices);
+        if (k % 5 == 1 && sh.num_vertices) std::memcpy(hostNrm + 12 * v, sh.normals, 12 * (size_t)sh.num_vertices);
+        if (k % 5 == 2 && sh.num_vertices) std::memcpy(hostUv + 8 * v, sh.texcoords, 8 * (size_t)sh.num_vertices);
+        if (k % 5 == 3 && sh.num_faces) std::memcpy(hostIdx + 12 * f, sh.indices, 12 * (size_t)sh.num_faces);
+        if (k % 5 == 4 && sh.num_faces) std::memcpy(hostMat + 2 * f, sh.materials, 2 * (size_t)sh.num_faces);
+    }
+    DevBuf staged;
+    staged.from = &ctx->memory;
+    RMD_CUDA(staged.upload(mesh.get(), meshBytes, st));
+    RMD_CUDA(s->vertices.alloc(numVertices * sizeof(float4)));
+    RMD_CUDA(s->normals.alloc(numVertices * sizeof(float4)));
+    RMD_CUDA(s->texcoords.alloc(uvBytes));
+    RMD_CUDA(s->faces.alloc(numFaces * sizeof(uint4)));
+    const unsigned char *devPos = staged.as<unsigned char>();
+    RMD_CUDA(rmdLaunchPackMesh(reinterpret_cast<const float *>(devPos), reinterpret_cast<const float *>(devPos + posBytes),
+                               (uint32_t)numVertices, reinterpret_cast<const uint32_t *>(devPos + 2 * posBytes + uvBytes),
+                               reinterpret_cast<const uint16_t *>(devPos + 2 * posBytes + uvBytes + idxBytes),
+                               (uint32_t)numFaces, s->vertices.as<float4>(), s->normals.as<float4>(),
+                               s->faces.as<uint4>(), st));
+    if (uvBytes)
+        RMD_CUDA(cudaMemcpyAsync(s->texcoords.ptr, devPos + 2 * posBytes, uvBytes, cudaMemcpyDeviceToDevice, st));
+    RMD_CUDA(cudaStreamSynchronize(st));  // `staged` goes back to the pool
+    staged.release();
+    mesh.reset();
 
     // EntityBuilder.build (EntityBuilder.swift:79-141), flattened into one BVH
     std::vector<PerInstanceData> insts;
-    std::vector<float> t0, t1, t2;
-    std::vector<uint32_t> triInst, triPrim;
+    size_t numTriangles = 0;
     struct PendingLight {
         uint32_t instance, shape;
         HostMat4 M;
@@ -579,7 +684,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         inst.faceOffset = si.faceOffset;
         inst.visibility = e.visibility;
         inst.lightIndex = 0xffffffffu;
-        inst.triOffset = (uint32_t)triInst.size();
+        inst.triOffset = (uint32_t)numTriangles;
         inst.boundsMin = make_float4(si.boundsMin[0], si.boundsMin[1], si.boundsMin[2], 0.0f);
         inst.boundsSize = make_float4(si.boundsMax[0] - si.boundsMin[0], si.boundsMax[1] - si.boundsMin[1],
                                       si.boundsMax[2] - si.boundsMin[2], 0.0f);
@@ -595,33 +700,41 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
             lightFaceOffset += si.faceCount;
         }
         insts.push_back(inst);
-        for (uint32_t f = 0; f < si.faceCount; f++) {
-            const uint4 fc = faces[si.faceOffset + f];
-            const uint32_t vi[3] = {fc.x, fc.y, fc.z};
-            float w[3][3];
-            for (int j = 0; j < 3; j++) {
-                const float4 p = verts[si.vertexOffset + vi[j]];
-                const float pp[3] = {p.x, p.y, p.z};
-                transformPoint(M, pp, w[j]);
-            }
-            t0.insert(t0.end(), w[0], w[0] + 3);
-            t1.insert(t1.end(), w[1], w[1] + 3);
-            t2.insert(t2.end(), w[2], w[2] + 3);
-            triInst.push_back((uint32_t)ei);
-            triPrim.push_back(f);
-        }
+        numTriangles += si.faceCount;
     }
-    s->triangles = triInst.size();
-    if (!t0.empty()) {
-        for (int k = 0; k < 3; k++) {
-            s->boundsMin[k] = INFINITY;
-            s->boundsMax[k] = -INFINITY;
-        }
-        for (const std::vector<float> *t : {&t0, &t1, &t2})
-            for (size_t i = 0; i < t->size(); i++) {
-                s->boundsMin[i % 3] = std::min(s->boundsMin[i % 3], (*t)[i]);
-                s->boundsMax[i % 3] = std::max(s->boundsMax[i % 3], (*t)[i]);
+    s->triangles = numTriangles;
+    RMD_CUDA(s->instances.upload(insts.data(), insts.size() * sizeof(PerInstanceData), st));
+    // the world-space triangles: on the device for its builder, else on the host
+    std::vector<float> t0, t1, t2;
+    std::vector<uint32_t> triInst, triPrim;
+    if (numTriangles && ctx->bvhBuilder != RMD_BVH_GPU) {
+        for (std::vector<float> *t : {&t0, &t1, &t2}) t->resize(3 * numTriangles);
+        triInst.resize(numTriangles);
+        triPrim.resize(numTriangles);
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+#pragma omp parallel for schedule(dynamic, 1) reduction(min : lo[:3]) reduction(max : hi[:3])
+        for (int ei = 0; ei < d->num_entities; ei++) {
+            const rmd_entity &e = d->entities[ei];
+            const rmd_shape &sh = d->shapes[e.shape];
+            const HostMat4 M = toMat(e.matrix);
+            const size_t base = insts[ei].triOffset;
+            for (uint32_t f = 0; f < sh.num_faces; f++) {
+                float *const w[3] = {&t0[3 * (base + f)], &t1[3 * (base + f)], &t2[3 * (base + f)]};
+                for (int j = 0; j < 3; j++) {
+                    transformPoint(M, sh.vertices + 3 * (size_t)sh.indices[3 * (size_t)f + j], w[j]);
+                    for (int k = 0; k < 3; k++) {
+                        lo[k] = std::min(lo[k], w[j][k]);
+                        hi[k] = std::max(hi[k], w[j][k]);
+                    }
+                }
+                triInst[base + f] = (uint32_t)ei;
+                triPrim[base + f] = f;
             }
+        }
+        for (int k = 0; k < 3; k++) {
+            s->boundsMin[k] = lo[k];
+            s->boundsMax[k] = hi[k];
+        }
     }
     // ShapeBuilder / EntityBuilder acceleration structures: one BVH over the
     // flattened world-space triangles, built on the host or on the device
@@ -629,18 +742,24 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     const auto buildStart = std::chrono::steady_clock::now();
     s->bvhStats.builder = ctx->bvhBuilder;
     if (ctx->bvhBuilder == RMD_BVH_GPU) {
-        DevBuf d0, d1, d2, dInst, dPrim;
-        RMD_CUDA(d0.upload(t0.data(), t0.size() * sizeof(float), st));
-        RMD_CUDA(d1.upload(t1.data(), t1.size() * sizeof(float), st));
-        RMD_CUDA(d2.upload(t2.data(), t2.size() * sizeof(float), st));
-        RMD_CUDA(dInst.upload(triInst.data(), triInst.size() * sizeof(uint32_t), st));
-        RMD_CUDA(dPrim.upload(triPrim.data(), triPrim.size() * sizeof(uint32_t), st));
+        DevBuf world;  // three vertices, instance and primitive per triangle, then the bounds
+        world.from = &ctx->memory;
+        RMD_CUDA(world.alloc(numTriangles * 44 + 6 * sizeof(uint32_t)));
+        float *w0 = world.as<float>(), *w1 = w0 + 3 * numTriangles, *w2 = w1 + 3 * numTriangles;
+        uint32_t *wInst = reinterpret_cast<uint32_t *>(w2 + 3 * numTriangles), *wPrim = wInst + numTriangles;
+        const uint32_t n = (uint32_t)std::min<size_t>(numTriangles, 0xffffffffu);
+        if (n) {
+            float bounds[6];
+            RMD_CUDA(rmdLaunchFlatten(s->vertices.as<float4>(), s->faces.as<uint4>(), s->instances.as<PerInstanceData>(),
+                                      (uint32_t)insts.size(), n, w0, w1, w2, wInst, wPrim, wPrim + numTriangles, bounds, st));
+            std::memcpy(s->boundsMin, bounds, sizeof(s->boundsMin));
+            std::memcpy(s->boundsMax, bounds + 3, sizeof(s->boundsMax));
+        }
         rmdhost::GpuBvhResult g;
-        const cudaError_t e = rmdhost::buildWideBvhGpu(d0.as<float>(), d1.as<float>(), d2.as<float>(),
-                                                       dInst.as<uint32_t>(), dPrim.as<uint32_t>(),
-                                                       (uint32_t)std::min<size_t>(triInst.size(), 0xffffffffu), st, g);
+        const cudaError_t e = rmdhost::buildWideBvhGpu(
+            w0, w1, w2, wInst, wPrim, n, st, [&](void **p, size_t bytes) { return ctx->memory.alloc(p, bytes); }, g);
         s->bvhNodes.adopt(g.nodes, g.nodeCount * sizeof(rmdhost::GpuWideNode));
-        s->bvhTris.adopt(g.tris, triInst.size() * TRI_FLOAT4 * sizeof(float4));
+        s->bvhTris.adopt(g.tris, numTriangles * TRI_FLOAT4 * sizeof(float4));
         if (e != cudaSuccess) {
             if (!g.error.empty()) return fail(RMD_ERROR_INVALID_ARGUMENT, "device BVH build: " + g.error);
             RMD_CUDA(e);
@@ -662,8 +781,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         const ShapeInfo &si = shapes[p.shape];
         ShapeLight sl;
         sl.instanceIndex = p.instance;
-        sl.emissiveArea = buildLightDistribution(p.M, idxPacked.data() + 3 * (size_t)si.faceOffset,
-                                                 vertsPacked.data() + 3 * (size_t)si.vertexOffset, si.faceCount,
+        sl.emissiveArea = buildLightDistribution(p.M, d->shapes[p.shape].indices, d->shapes[p.shape].vertices, si.faceCount,
                                                  lightFaces.data() + p.lightFaceOffset);
         shapeLights.push_back(sl);
     }
@@ -733,11 +851,6 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     if (stab.empty()) stab.push_back(make_uint2(0, 0));
 
     // uploads
-    RMD_CUDA(s->vertices.upload(verts.data(), verts.size() * sizeof(float4), st));
-    RMD_CUDA(s->normals.upload(norms.data(), norms.size() * sizeof(float4), st));
-    RMD_CUDA(s->texcoords.upload(uvs.data(), uvs.size() * sizeof(float2), st));
-    RMD_CUDA(s->faces.upload(faces.data(), faces.size() * sizeof(uint4), st));
-    RMD_CUDA(s->instances.upload(insts.data(), insts.size() * sizeof(PerInstanceData), st));
     s->instanceRecords.assign(insts.size(), rmd_per_instance_data{});
     for (size_t i = 0; i < insts.size(); i++) {
         const PerInstanceData &p = insts[i];
@@ -768,6 +881,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     }
     if (s->triangles && ctx->bvhBuilder != RMD_BVH_GPU) {  // the traversal kernels read three rotated copies of each triangle (device/traverse.cuh)
         DevBuf rotated;
+        rotated.from = &ctx->memory;
         RMD_CUDA(rotated.alloc(s->triangles * TRI_FLOAT4 * sizeof(float4)));
         RMD_CUDA(rmdLaunchRotateTriangles(s->bvhTris.as<float4>(), rotated.as<float4>(), (uint32_t)s->triangles, st));
         RMD_CUDA(cudaStreamSynchronize(st));
@@ -1059,6 +1173,8 @@ rmd_status rmd_renderer_create(rmd_scene *scene, uint32_t width, uint32_t height
     RMD_CUDA(cudaSetDevice(scene->ctx->device));
     auto r = std::make_unique<rmd_renderer>();
     r->scene = scene;
+    for (DevBuf *b : {&r->pool, &r->counters, &r->resolve}) b->from = &scene->ctx->memory;  // not the films: callers share them
+    r->guide.takeMemoryFrom(scene->ctx->memory);
     r->dctx = scene->dctx;
     r->shade = scene->jit.shade;
     r->shadeBlocks = scene->shadeBlocks;
@@ -1769,6 +1885,8 @@ rmd_status rmd_batch_create(rmd_context *ctx, const rmd_scene_desc *descs, int32
     RMD_CUDA(cudaSetDevice(ctx->device));
     auto b = std::make_unique<rmd_batch>();
     b->ctx = ctx;
+    for (DevBuf *m : {&b->viewTable, &b->pool, &b->counters, &b->resolve}) m->from = &ctx->memory;
+    b->guide.takeMemoryFrom(ctx->memory);
     b->useGraph = !(flags & RMD_BATCH_NO_GRAPH);
     // one material module for all scenes: their materials concatenated
     std::vector<rmd_material> surf, light;
