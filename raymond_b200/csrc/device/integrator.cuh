@@ -290,6 +290,7 @@ __device__ __forceinline__ bool shadePath(const ShadeParams &p, uint32_t i, uint
 #define RMD_SHADE_MIN_BLOCKS 1
 #endif
 extern "C" __global__ void __launch_bounds__(128, RMD_SHADE_MIN_BLOCKS) rmd_shade(const __grid_constant__ rmd::ShadeParams p) {
+    rmd::waitForPreviousKernel();
     const unsigned n = rmd::activeCount(p.counters, p.cur);
     unsigned segments = 0, rays = 0;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {

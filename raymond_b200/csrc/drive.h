@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <tuple>
 
 #include "device/wavefront.cuh"
 
@@ -38,6 +39,31 @@ cudaError_t driveWavefront(const rmd::Counters *cnt, uint64_t numPaths, uint32_t
         if (check(h, it)) return cudaSuccess;
         if (h.handOut[0] >= h.endPath) paths = std::min<uint64_t>(paths, std::max(h.nQ[0], 1u));
     }
+}
+
+// Launches a kernel that begins with waitForPreviousKernel so that its set-up
+// overlaps the end of the kernel before it on the stream.
+inline cudaError_t launchOverlapped(const void *kernel, int blocks, int threads, void **args, cudaStream_t st) {
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+template <class... Params, class... Args>
+cudaError_t launchOverlapped(void (*kernel)(Params...), int blocks, int threads, cudaStream_t st, Args... values) {
+    std::tuple<Params...> params(values...);
+    return std::apply(
+        [&](Params &...p) {
+            void *args[] = {(void *)&p...};
+            return launchOverlapped((const void *)kernel, blocks, threads, args, st);
+        },
+        params);
 }
 
 // blocks of `threads` threads that give `paths` paths a thread each, at most `most`

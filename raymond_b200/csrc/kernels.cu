@@ -10,6 +10,7 @@
 
 #include "device/traverse.cuh"
 #include "device/wavefront.cuh"
+#include "drive.h"
 #include "kernels.h"
 #include "sky.h"
 
@@ -49,6 +50,7 @@ __global__ void k_frame_init(Counters *cnt, uint32_t capacity, uint64_t firstPat
 template <bool BATCH>
 __global__ void __launch_bounds__(256) k_film_regen(Context ctx, PathPool pool, FrameParams fp, Counters *cnt,
                                                     uint32_t p, uint32_t f) {
+    waitForPreviousKernel();
     const uint32_t nFin = cnt->nF[f];
     const uint32_t base = cnt->nQ[p];
     const unsigned long long first = cnt->handOut[p];
@@ -301,6 +303,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, 8) k_trace(const WideNode *__re
                                                             const __grid_constant__ PathPool pool, Counters *cnt,
                                                             uint32_t p, uint32_t q) {
     __shared__ uint32_t clocks[2];  // of the block's warps on closest hits and on shadow rays
+    waitForPreviousKernel();
     const uint32_t nClosest = CLOSEST ? activeCount(cnt, p) : 0u;
     const uint32_t nShadow = SHADOW ? (CLOSEST ? cnt->nShadowPrev : cnt->nShadow) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -594,27 +597,23 @@ cudaError_t rmdLaunchFrameInit(const PathPool &pool, Counters *cnt, uint64_t fir
 }
 cudaError_t rmdLaunchFilmRegen(const Context &ctx, const PathPool &pool, const FrameParams &fp, Counters *cnt,
                                uint32_t cur, uint32_t fin, int blocks, cudaStream_t s) {
-    if (pool.views) k_film_regen<true><<<blocks, 256, 0, s>>>(ctx, pool, fp, cnt, cur, fin);
-    else k_film_regen<false><<<blocks, 256, 0, s>>>(ctx, pool, fp, cnt, cur, fin);
-    return cudaGetLastError();
+    if (pool.views) return rmdhost::launchOverlapped(k_film_regen<true>, blocks, 256, s, ctx, pool, fp, cnt, cur, fin);
+    return rmdhost::launchOverlapped(k_film_regen<false>, blocks, 256, s, ctx, pool, fp, cnt, cur, fin);
 }
 cudaError_t rmdLaunchTrace(const WideNode *nodes, const float4 *tris, const PathPool &pool, Counters *cnt, uint32_t cur,
                            int blocks, cudaStream_t s) {
-    if (pool.views) k_trace<true, true, true><<<blocks, TRACE_THREADS, 0, s>>>(nodes, tris, pool, cnt, cur, cur ^ 1u);
-    else k_trace<false, true, true><<<blocks, TRACE_THREADS, 0, s>>>(nodes, tris, pool, cnt, cur, cur ^ 1u);
-    return cudaGetLastError();
+    if (pool.views) return rmdhost::launchOverlapped(k_trace<true, true, true>, blocks, TRACE_THREADS, s, nodes, tris, pool, cnt, cur, cur ^ 1u);
+    return rmdhost::launchOverlapped(k_trace<false, true, true>, blocks, TRACE_THREADS, s, nodes, tris, pool, cnt, cur, cur ^ 1u);
 }
 cudaError_t rmdLaunchTraceClosest(const WideNode *nodes, const float4 *tris, const PathPool &pool, Counters *cnt,
                                   uint32_t cur, int blocks, cudaStream_t s) {
-    if (pool.views) k_trace<true, true, false><<<blocks, TRACE_THREADS, 0, s>>>(nodes, tris, pool, cnt, cur, 0u);
-    else k_trace<false, true, false><<<blocks, TRACE_THREADS, 0, s>>>(nodes, tris, pool, cnt, cur, 0u);
-    return cudaGetLastError();
+    if (pool.views) return rmdhost::launchOverlapped(k_trace<true, true, false>, blocks, TRACE_THREADS, s, nodes, tris, pool, cnt, cur, 0u);
+    return rmdhost::launchOverlapped(k_trace<false, true, false>, blocks, TRACE_THREADS, s, nodes, tris, pool, cnt, cur, 0u);
 }
 cudaError_t rmdLaunchTraceShadow(const WideNode *nodes, const float4 *tris, const PathPool &pool, Counters *cnt,
                                  uint32_t cur, int blocks, cudaStream_t s) {
-    if (pool.views) k_trace<true, false, true><<<blocks, TRACE_THREADS, 0, s>>>(nodes, tris, pool, cnt, cur, cur);
-    else k_trace<false, false, true><<<blocks, TRACE_THREADS, 0, s>>>(nodes, tris, pool, cnt, cur, cur);
-    return cudaGetLastError();
+    if (pool.views) return rmdhost::launchOverlapped(k_trace<true, false, true>, blocks, TRACE_THREADS, s, nodes, tris, pool, cnt, cur, cur);
+    return rmdhost::launchOverlapped(k_trace<false, false, true>, blocks, TRACE_THREADS, s, nodes, tris, pool, cnt, cur, cur);
 }
 cudaError_t rmdLaunchEnvmapReduce(float *mip, int cur, cudaStream_t s) {
     dim3 b(8, 8), g((cur + 7) / 8, (cur + 7) / 8);

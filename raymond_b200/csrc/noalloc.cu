@@ -158,7 +158,7 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
         if (e != cudaSuccess) return e;
         if ((e = rmdLaunchTrace(v.nodes, v.tris, pool, cnt, cur, rmdhost::traceGridFor(paths, tb), st)) != cudaSuccess) return e;
         sp.setParity(cur);
-        return cudaLaunchKernel((const void *)v.shade, dim3(rmdhost::gridFor(paths, 128, v.shadeBlocks)), dim3(128), shadeArgs, 0, st);
+        return rmdhost::launchOverlapped((const void *)v.shade, rmdhost::gridFor(paths, 128, v.shadeBlocks), 128, shadeArgs, st);
     };
     rmd_status status = RMD_OK;
     const auto check = [&](const Counters &h, uint64_t iterations) {

@@ -1173,7 +1173,8 @@ rmd_status rmd_renderer_create(rmd_scene *scene, uint32_t width, uint32_t height
     RMD_CUDA(cudaSetDevice(scene->ctx->device));
     auto r = std::make_unique<rmd_renderer>();
     r->scene = scene;
-    for (DevBuf *b : {&r->pool, &r->counters, &r->resolve}) b->from = &scene->ctx->memory;  // not the films: callers share them
+    // not the film, whose address callers get (rmd_film_device)
+    for (DevBuf *b : {&r->pool, &r->counters, &r->resolve, &r->film64}) b->from = &scene->ctx->memory;
     r->guide.takeMemoryFrom(scene->ctx->memory);
     r->dctx = scene->dctx;
     r->shade = scene->jit.shade;
@@ -1348,7 +1349,7 @@ rmd_status rmd_render(rmd_renderer *r, const rmd_render_settings *s) {
             if (e != cudaSuccess || (e = mark(STAGE_GUIDE)) != cudaSuccess) return e;
         }
         sp.setParity(cur);
-        e = cudaLaunchKernel((const void *)r->shade, dim3(rmdhost::gridFor(paths, 128, sb)), dim3(128), shadeArgs, 0, st);
+        e = rmdhost::launchOverlapped((const void *)r->shade, rmdhost::gridFor(paths, 128, sb), 128, shadeArgs, st);
         if (e != cudaSuccess || (e = mark(STAGE_SHADE)) != cudaSuccess) return e;
         if (guideTraining) {
             e = rmdLaunchTraceShadow(nodes, tris, pool, cnt, cur, blocks, st);
@@ -1885,7 +1886,7 @@ rmd_status rmd_batch_create(rmd_context *ctx, const rmd_scene_desc *descs, int32
     RMD_CUDA(cudaSetDevice(ctx->device));
     auto b = std::make_unique<rmd_batch>();
     b->ctx = ctx;
-    for (DevBuf *m : {&b->viewTable, &b->pool, &b->counters, &b->resolve}) m->from = &ctx->memory;
+    for (DevBuf *m : {&b->viewTable, &b->pool, &b->counters, &b->resolve, &b->film, &b->film64}) m->from = &ctx->memory;
     b->guide.takeMemoryFrom(ctx->memory);
     b->useGraph = !(flags & RMD_BATCH_NO_GRAPH);
     // one material module for all scenes: their materials concatenated
@@ -2020,7 +2021,7 @@ static cudaError_t batchEnqueueIteration(rmd_batch *b, const PathPool &pool, con
                                                b->ctx->smCount, st)) != cudaSuccess)
         return e;
     sp.setParity(cur);
-    e = cudaLaunchKernel((const void *)b->shade, dim3(rmdhost::gridFor(paths, 128, b->shadeBlocks)), dim3(128), shadeArgs, 0, st);
+    e = rmdhost::launchOverlapped((const void *)b->shade, rmdhost::gridFor(paths, 128, b->shadeBlocks), 128, shadeArgs, st);
     if (e != cudaSuccess) return e;
     return training ? rmdLaunchTraceShadow(nullptr, nullptr, pool, cnt, cur, tb, st) : cudaSuccess;
 }
