@@ -32,7 +32,7 @@ constexpr float GUIDE_ALPHA_MIN = 0.02f, GUIDE_ALPHA_MAX = 0.5f;
 // weight_j / sum(weights) * C(kappa_j) in FP32; the 8 selection weights as
 // bf16; the selection probability of the guide.  Sampling and pdf read the
 // same rounded values, so they describe the same distribution.
-struct GuideMixture {
+struct alignas(16) GuideMixture {
     uint2 lobe[GUIDE_LOBES];
     float coef[GUIDE_LOBES];
     uint4 weights;
@@ -53,13 +53,36 @@ RMD_HD float vmfNorm(float kappa) { return kappa / (2.0f * M_PI_F * -expm1f(-2.0
 
 RMD_HD float3 lobeMu(uint2 l) { return normalize(make_float3(bf16Lo(l.x), bf16Hi(l.x), bf16Lo(l.y))); }
 
-// pdf of the mixture (solid angle)
+// kappa (cos(mu, w) - 1) of one packed lobe.  The bf16 mean is renormalised by
+// its reciprocal length: rsqrtf and one Newton step with the residual
+// 1 - n r^2 (n r in two parts), then one rounding for product and subtraction.  cos - 1 comes out
+// nearer its 64-bit value than with the root and three divisions it replaces
+// (rms 3.7e-8 against 4.0e-8, at most 1.8e-7 against 2.1e-7).
+RMD_HD float lobeExponent(uint32_t xy, uint32_t zk, float3 w) {
+    const float3 mu = make_float3(bf16Lo(xy), bf16Hi(xy), bf16Lo(zk));
+    const float n = dot(mu, mu);
+    float r = rsqrtf(n);
+    const float nr = n * r, lo = fmaf(n, r, -nr);
+    r = fmaf(0.5f * r, fmaf(-lo, r, fmaf(-nr, r, 1.0f)), r);
+    return bf16Hi(zk) * fmaf(dot(mu, w), r, -1.0f);
+}
+
+// pdf of the mixture (solid angle), read in six 16-byte loads.  The shading
+// kernel evaluates it at the light's and at the sampled direction of each
+// vertex; with a root, three divisions and three narrow loads per lobe the
+// pass took 10.7 instead of 9.9 ms for 31 M vertices (Cornell box).
 RMD_HD float guidePdf(const GuideMixture *m, float3 w) {
+    const uint4 *lobes = reinterpret_cast<const uint4 *>(m->lobe);
+    const float4 *coefs = reinterpret_cast<const float4 *>(m->coef);
     float p = 0.0f;
 #pragma unroll
-    for (int j = 0; j < GUIDE_LOBES; j++) {
-        const uint2 l = m->lobe[j];
-        p += m->coef[j] * __expf(bf16Hi(l.y) * (dot(lobeMu(l), w) - 1.0f));
+    for (int h = 0; h < GUIDE_LOBES / 4; h++) {
+        const uint4 a = lobes[2 * h], b = lobes[2 * h + 1];
+        const float4 c = coefs[h];
+        p += c.x * __expf(lobeExponent(a.x, a.y, w));
+        p += c.y * __expf(lobeExponent(a.z, a.w, w));
+        p += c.z * __expf(lobeExponent(b.x, b.y, w));
+        p += c.w * __expf(lobeExponent(b.z, b.w, w));
     }
     return p;
 }
