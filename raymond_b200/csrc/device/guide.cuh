@@ -32,6 +32,11 @@ constexpr float GUIDE_ALPHA_MIN = 0.02f, GUIDE_ALPHA_MAX = 0.5f;
 // weight_j / sum(weights) * C(kappa_j) in FP32; the 8 selection weights as
 // bf16; the selection probability of the guide.  Sampling and pdf read the
 // same rounded values, so they describe the same distribution.
+// In memory the mixtures of 32 consecutive hits lie interleaved by 16-byte
+// chunk, so that a warp writes and reads each chunk as 512 contiguous bytes
+// (chunks 0-3: lobes, 4-5: coefficients, 6: weights, 7: alpha and invTotal);
+// as 128 consecutive bytes per hit every 16-byte access of a warp touched 32
+// lines.
 struct alignas(16) GuideMixture {
     uint2 lobe[GUIDE_LOBES];
     float coef[GUIDE_LOBES];
@@ -40,6 +45,22 @@ struct alignas(16) GuideMixture {
     float invTotal;  // 1 / sum of the bf16 weights
     float pad[2];
 };
+constexpr uint32_t GUIDE_MIX_STRIDE = 32;  // 16-byte chunks between two chunks of one mixture
+// a mixture's first chunk: hit `q` in shading order
+RMD_HD size_t guideMixtureAt(uint32_t q) { return (size_t)(q >> 5) * (8u * GUIDE_MIX_STRIDE) + (q & 31u); }
+RMD_HD void storeMixture(uint4 *dst, const GuideMixture &m) {
+#pragma unroll
+    for (int j = 0; j < GUIDE_LOBES / 2; j++)
+        dst[j * GUIDE_MIX_STRIDE] = make_uint4(m.lobe[2 * j].x, m.lobe[2 * j].y, m.lobe[2 * j + 1].x, m.lobe[2 * j + 1].y);
+#pragma unroll
+    for (int j = 0; j < GUIDE_LOBES / 4; j++)
+        dst[(4 + j) * GUIDE_MIX_STRIDE] = make_uint4(__float_as_uint(m.coef[4 * j]), __float_as_uint(m.coef[4 * j + 1]),
+                                                     __float_as_uint(m.coef[4 * j + 2]), __float_as_uint(m.coef[4 * j + 3]));
+    dst[6 * GUIDE_MIX_STRIDE] = m.weights;
+    dst[7 * GUIDE_MIX_STRIDE] = make_uint4(__float_as_uint(m.alpha), __float_as_uint(m.invTotal), 0u, 0u);
+}
+// the guide's selection probability
+RMD_HD float guideAlpha(const uint4 *m) { return __uint_as_float(m[7 * GUIDE_MIX_STRIDE].x); }
 
 RMD_HD uint32_t bf16Bits(float x) {  // round to nearest even
     const uint32_t u = __float_as_uint(x);
@@ -71,18 +92,16 @@ RMD_HD float lobeExponent(uint32_t xy, uint32_t zk, float3 w) {
 // kernel evaluates it at the light's and at the sampled direction of each
 // vertex; with a root, three divisions and three narrow loads per lobe the
 // pass took 10.7 instead of 9.9 ms for 31 M vertices (Cornell box).
-RMD_HD float guidePdf(const GuideMixture *m, float3 w) {
-    const uint4 *lobes = reinterpret_cast<const uint4 *>(m->lobe);
-    const float4 *coefs = reinterpret_cast<const float4 *>(m->coef);
+RMD_HD float guidePdf(const uint4 *m, float3 w) {
     float p = 0.0f;
 #pragma unroll
     for (int h = 0; h < GUIDE_LOBES / 4; h++) {
-        const uint4 a = lobes[2 * h], b = lobes[2 * h + 1];
-        const float4 c = coefs[h];
-        p += c.x * __expf(lobeExponent(a.x, a.y, w));
-        p += c.y * __expf(lobeExponent(a.z, a.w, w));
-        p += c.z * __expf(lobeExponent(b.x, b.y, w));
-        p += c.w * __expf(lobeExponent(b.z, b.w, w));
+        const uint4 a = m[2 * h * GUIDE_MIX_STRIDE], b = m[(2 * h + 1) * GUIDE_MIX_STRIDE];
+        const uint4 c = m[(4 + h) * GUIDE_MIX_STRIDE];
+        p += __uint_as_float(c.x) * __expf(lobeExponent(a.x, a.y, w));
+        p += __uint_as_float(c.y) * __expf(lobeExponent(a.z, a.w, w));
+        p += __uint_as_float(c.z) * __expf(lobeExponent(b.x, b.y, w));
+        p += __uint_as_float(c.w) * __expf(lobeExponent(b.z, b.w, w));
     }
     return p;
 }
@@ -90,9 +109,9 @@ RMD_HD float guidePdf(const GuideMixture *m, float3 w) {
 // direction from the mixture: lobe by u.x, then the vMF sample (Wenzel
 // Jakob, "Numerically stable sampling of the von Mises Fisher distribution on
 // S2", 2012) by u.y, u.z
-RMD_HD float3 guideSample(const GuideMixture *m, float3 u) {
-    const float target = u.x / m->invTotal;  // the stored weights sum to 1 / invTotal
-    const uint4 wq = m->weights;
+RMD_HD float3 guideSample(const uint4 *m, float3 u) {
+    const float target = u.x / __uint_as_float(m[7 * GUIDE_MIX_STRIDE].y);  // the stored weights sum to 1 / invTotal
+    const uint4 wq = m[6 * GUIDE_MIX_STRIDE];
     float acc = 0.0f;
     int k = GUIDE_LOBES - 1;
     bool found = false;
@@ -105,7 +124,7 @@ RMD_HD float3 guideSample(const GuideMixture *m, float3 u) {
             found = true;
         }
     }
-    const uint2 l = m->lobe[k];
+    const uint2 l = reinterpret_cast<const uint2 *>(m + (k >> 1) * GUIDE_MIX_STRIDE)[k & 1];
     const float kappa = bf16Hi(l.y);
     const float uy = fmaxf(u.y, 1e-7f);
     const float wz = 1.0f + logf(uy + (1.0f - uy) * __expf(-2.0f * kappa)) / kappa;

@@ -112,8 +112,8 @@ __device__ __forceinline__ bool shadePath(const ShadeParams &p, uint32_t i, uint
         // the guide mixture of this point (one-sample MIS); the technique's pdf is
         // then alpha q + (1 - alpha) p_bsdf in every MIS weight that uses it.
         const bool guided = kGuideCode && depth < fp.guideDepth;
-        const GuideMixture *gm = &pool.guide[orderPos];  // hits are shaded in order: mixture by that position
-        float alpha = guided ? gm->alpha : 0.0f;
+        const uint4 *gm = pool.guide + guideMixtureAt(orderPos);  // hits are shaded in order: mixture by that position
+        float alpha = guided ? guideAlpha(gm) : 0.0f;
         if (guided) {
             // A warp whose lanes are all guided uses one selection probability,
             // the mean of their alphas: the technique choice below is then the

@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(256) k_guide_features(Context ctx, PathPool po
 // stored; tcgen05 tiles of 128 samples.  On an expired wait the CTA sets
 // ERR_GUIDE_TIMEOUT in the counters and stops.
 __global__ void __launch_bounds__(kTcThreads) k_guide_infer(Counters *cnt, const uint4 *features, uint32_t guideDepth,
-                                                         GuideNetView net, GuideMixture *out) {
+                                                         GuideNetView net, uint4 *out) {
     extern __shared__ __align__(16) unsigned char smem[];
     TcSmem &sm = *reinterpret_cast<TcSmem *>(smem);
     tcSetup(sm, net);
@@ -1013,27 +1013,9 @@ __global__ void __launch_bounds__(kTcThreads) k_guide_infer(Counters *cnt, const
             if (row == 0) atomicOr(&cnt->errors, ERR_GUIDE_TIMEOUT);
             break;
         }
-        // The tile's 128 mixtures are one contiguous block of `out`: staged in
-        // the pipeline's A buffer (free once the last layer's MMA has read it),
-        // each row's eight 16-byte chunks rotated by the row so that 8
-        // consecutive rows store to different banks, then copied out by the
-        // pipeline with coalesced stores.  Rows past the guided depth are
-        // written too; shading reads a mixture only at guided depths.
-        union {
-            GuideMixture m;
-            uint4 c[8];
-        } mix;
-        static_assert(sizeof(GuideMixture) == 8 * sizeof(uint4), "a mixture is eight 16-byte chunks");
-        mix.m = pack(decode(o));
-        uint4 *stage = reinterpret_cast<uint4 *>(sm.a[pipe]);
-#pragma unroll
-        for (int j = 0; j < 8; j++) stage[row * 8 + (j ^ (row & 7))] = mix.c[j];
-        pipeSync(pipe);
-        const uint32_t first = tile * kTcPipeThreads;
-        const uint32_t chunks = min((uint32_t)kTcPipeThreads, nHit - first) * 8u;
-        uint4 *dst = reinterpret_cast<uint4 *>(out + first);
-        for (uint32_t k = row; k < chunks; k += kTcPipeThreads) dst[k] = stage[(k & ~7u) + ((k & 7u) ^ ((k >> 3) & 7u))];
-        pipeSync(pipe);  // the next tile's input rows overwrite the stage
+        // Rows past the guided depth are written too; shading reads a mixture
+        // only at guided depths.
+        if (q < nHit) storeMixture(out + guideMixtureAt(q), pack(decode(o)));
     }
     tcTeardown(sm, pipe, phase);
 }
@@ -1136,16 +1118,17 @@ __global__ void k_guide_refresh(GuideNetView net) {
 __global__ void k_guide_mixture_test(const float *outputs, const float *u, int n, float *dirsPdf, const float *queries,
                                      int m, float *pdfs) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n && i >= m) return;
-    const GuideMixture mix = pack(decode(outputs));
+    __shared__ uint4 mix[8 * GUIDE_MIX_STRIDE];
+    if (threadIdx.x == 0) storeMixture(mix, pack(decode(outputs)));
+    __syncthreads();
     if (i < n) {
-        const float3 d = guideSample(&mix, make_float3(u[3 * i], u[3 * i + 1], u[3 * i + 2]));
+        const float3 d = guideSample(mix, make_float3(u[3 * i], u[3 * i + 1], u[3 * i + 2]));
         dirsPdf[4 * i + 0] = d.x;
         dirsPdf[4 * i + 1] = d.y;
         dirsPdf[4 * i + 2] = d.z;
-        dirsPdf[4 * i + 3] = guidePdf(&mix, d);
+        dirsPdf[4 * i + 3] = guidePdf(mix, d);
     }
-    if (i < m) pdfs[i] = guidePdf(&mix, make_float3(queries[3 * i], queries[3 * i + 1], queries[3 * i + 2]));
+    if (i < m) pdfs[i] = guidePdf(mix, make_float3(queries[3 * i], queries[3 * i + 1], queries[3 * i + 2]));
 }
 
 }  // namespace
@@ -1167,7 +1150,7 @@ cudaError_t rmdGuideConfigure() {
 }
 
 cudaError_t rmdLaunchGuideInfer(const Context &ctx, const PathPool &pool, Counters *cnt, uint32_t cur,
-                                uint32_t guideDepth, const GuideNetView &net, GuideMixture *out, int blocks,
+                                uint32_t guideDepth, const GuideNetView &net, uint4 *out, int blocks,
                                 cudaStream_t s) {
     k_guide_features<<<pool.capacity / 256 < 1184u ? pool.capacity / 256 + 1 : 1184, 256, 0, s>>>(ctx, pool, cnt, cur,
                                                                                               guideDepth);

@@ -42,7 +42,7 @@ size_t rmdGuideSharedBytes(bool training);
 cudaError_t rmdGuideConfigure();
 // mixtures of this iteration's hits whose path depth is below guideDepth
 cudaError_t rmdLaunchGuideInfer(const rmd::Context &ctx, const rmd::PathPool &pool, rmd::Counters *cnt, uint32_t cur,
-                                uint32_t guideDepth, const rmd::GuideNetView &net, rmd::GuideMixture *out, int blocks,
+                                uint32_t guideDepth, const rmd::GuideNetView &net, uint4 *out, int blocks,
                                 cudaStream_t s);
 // `steps` Adam steps (the first is `step`, counting from 1), each on the mean
 // loss over a batch of n records drawn from the `total` stored ones (all of

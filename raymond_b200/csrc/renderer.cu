@@ -1021,7 +1021,7 @@ static void applyGuide(const GuideState &g, uint32_t capacity, PathPool &pool) {
         pool.recordCapacity = g.recordCapacity;
     }
     if (g.settings.sampling && g.pathCapacity >= capacity) {
-        pool.guide = g.mixtures.as<GuideMixture>();
+        pool.guide = g.mixtures.as<uint4>();
         pool.guideFeat = g.features.as<uint4>();
         pool.guideMin = g.frameMin;
         pool.guideInvExtent = g.frameInvExtent;
@@ -1058,7 +1058,7 @@ static rmd_status guideBuffers(GuideState &g, uint32_t capacity, Counters *count
         g.shRec.release();
     }
     if (g.settings.sampling && !g.mixtures.ptr) {
-        RMD_CUDA(g.mixtures.alloc((size_t)capacity * sizeof(GuideMixture)));
+        RMD_CUDA(g.mixtures.alloc(((size_t)capacity + 31u) / 32u * 32u * sizeof(GuideMixture)));
         RMD_CUDA(g.features.alloc((size_t)capacity * sizeof(uint4)));
     }
     if (g.settings.training && !g.rec.ptr) {
