@@ -29,6 +29,13 @@ __device__ __forceinline__ uint16_t toBf16(float x) { return (uint16_t)bf16Bits(
 __device__ __forceinline__ float fromBf16(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 __device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) { return (uint32_t)lo | ((uint32_t)hi << 16); }
 
+// two BF16 values, lo in the lower half, round to nearest even
+__device__ __forceinline__ uint32_t cvtBf16x2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
 __device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 
 // decoded network output of one sample
@@ -81,19 +88,19 @@ __device__ float3 lobeMeanPacked(const Decoded &d, int j) {
 
 __device__ GuideMixture pack(const Decoded &d) {
     GuideMixture m;
-    uint32_t w[4];
-    float total = 0.0f, kappa[GUIDE_LOBES];
+    uint32_t w[GUIDE_LOBES / 2];
+    float total = 0.0f;
+#pragma unroll
     for (int j = 0; j < GUIDE_LOBES; j++) {
         const float3 mu = lobeMeanPacked(d, j);
-        const uint32_t kb = bf16Bits(__expf(d.logKappa[j]));
-        kappa[j] = bf16Lo(kb);
-        total += bf16Lo(bf16Bits(d.lambda[j]));
-        m.lobe[j] = make_uint2(bf16Bits(mu.x) | (bf16Bits(mu.y) << 16), bf16Bits(mu.z) | (kb << 16));
-        if (j & 1) w[j >> 1] |= bf16Bits(d.lambda[j]) << 16;
-        else w[j >> 1] = bf16Bits(d.lambda[j]);
+        m.lobe[j] = make_uint2(cvtBf16x2(mu.x, mu.y), cvtBf16x2(mu.z, __expf(d.logKappa[j])));
+        if (!(j & 1)) w[j >> 1] = cvtBf16x2(d.lambda[j], d.lambda[j + 1]);
+        total += (j & 1) ? bf16Hi(w[j >> 1]) : bf16Lo(w[j >> 1]);
     }
     const float inv = 1.0f / total;
-    for (int j = 0; j < GUIDE_LOBES; j++) m.coef[j] = bf16Lo(bf16Bits(d.lambda[j])) * inv * vmfNormPacked(kappa[j]);
+#pragma unroll
+    for (int j = 0; j < GUIDE_LOBES; j++)
+        m.coef[j] = ((j & 1) ? bf16Hi(w[j >> 1]) : bf16Lo(w[j >> 1])) * inv * vmfNormPacked(bf16Hi(m.lobe[j].y));
     m.weights = make_uint4(w[0], w[1], w[2], w[3]);
     m.alpha = d.alpha;
     m.invTotal = inv;
@@ -188,14 +195,28 @@ __device__ __forceinline__ float oneBlob(float v, int bins, int bin) {
 // independent pipelines of 128 threads; each pipeline takes 128 samples at a
 // time (M = 128), one thread per sample, and the pipelines share one copy of
 // the weights in shared memory.  Each layer is tcgen05.mma (kind::f16, BF16
-// operands from shared memory, FP32 accumulator in the pipeline's 64 columns
-// of tensor memory) issued by the pipeline's first thread; its completion is
-// committed to the pipeline's mbarrier; every thread then reads its own
-// sample's row of the accumulator (tcgen05.ld, TMEM lane = sample), applies
-// bias and ReLU and writes the BF16 row back to shared memory as the next
-// layer's A operand.  The output layer's row stays in the thread's
+// operands, FP32 accumulator in the pipeline's 64 columns of tensor memory)
+// issued by the pipeline's first thread; its completion is committed to the
+// pipeline's mbarrier; every thread then reads its own sample's row of the
+// accumulator (tcgen05.ld, TMEM lane = sample), applies bias and ReLU and
+// writes the BF16 row to tensor memory as the next layer's A operand (the
+// first layer's A, the one-blob inputs, is in shared memory: its columns are
+// addressed by the data).  The output layer's row stays in the thread's
 // registers, so each thread decodes and packs its own sample's mixture.
 // While one pipeline runs its epilogue, the tensor core serves the others.
+//
+// What bounds it, 1.6 M hits of the Cornell box in one launch: with the hidden
+// rows in shared memory, the input row cleared and its bins then stored one by
+// one, and the mixtures staged, 212 us, the shared-memory and store path 56 %
+// busy with threads' accesses and 22 % with the tensor core's operand reads.
+// With the hidden rows in tensor memory, every 16-byte chunk of the input row
+// stored once, biases read four at a time, one barrier per layer, BF16
+// conversions in pairs and the next tile's features loaded ahead: 174 us, that
+// path 31 % busy and issue slots 53 %, the latency of the chain of layers at
+// 16 warps per SM what is left (the input rows' 160 KB allow no more).  A
+// launch of a few tiles took 17 us, most of it set-up (the weights rearranged
+// by the threads); the weights now arrive by one bulk copy before the wait for
+// the kernel before, and few tiles go to different SMs: 8 us.
 //
 // Operand layout (the canonical K-major, no-swizzle layout of the UMMA
 // shared-memory descriptor): 8 x 16-byte "core matrices" (8 rows, 8 BF16
@@ -204,20 +225,26 @@ __device__ __forceinline__ float oneBlob(float v, int bins, int bin) {
 constexpr int kTcPipes = 4;
 constexpr int kTcPipeThreads = 128;
 constexpr int kTcThreads = kTcPipes * kTcPipeThreads;
-constexpr uint32_t kTmemCols = 64 * kTcPipes;
+constexpr uint32_t kTmemPipe = 128;    // a pipeline's columns: 64 accumulator, 32 BF16 hidden rows, 32 unused
+constexpr uint32_t kTmemHidden = 64;   // its hidden rows' first column
+constexpr uint32_t kTmemCols = kTmemPipe * kTcPipes;
 constexpr int kTcSpinLimit = 1 << 22;  // bounded waits: on expiry the pipeline flags an error and stops
+constexpr uint32_t kTcFailed = 2u;     // in a thread's `phase` (bit 0: the mbarrier's parity): a wait expired
 
 struct TcSmem {
     uint16_t w1[GUIDE_HIDDEN * GUIDE_INPUTS];
     uint16_t w2[GUIDE_HIDDEN * GUIDE_HIDDEN];
     uint16_t w3[GUIDE_HIDDEN * GUIDE_HIDDEN];
     uint16_t w4[GUIDE_OUTPUTS * GUIDE_HIDDEN];
-    uint16_t a[kTcPipes][kTcPipeThreads * GUIDE_INPUTS];  // each pipeline's A operand (inputs, then hidden)
+    uint16_t a[kTcPipes][kTcPipeThreads * GUIDE_INPUTS];  // each pipeline's input rows
     float b[3 * GUIDE_HIDDEN + GUIDE_OUTPUTS];
-    unsigned long long mbar[kTcPipes];
+    unsigned long long mbar[kTcPipes + 1];  // the pipelines' MMAs; the weight image
     uint32_t tmemBase;
-    int failed[kTcPipes];
 };
+// the weight image (GuideNetView::image) is also TcSmem's leading weight region
+constexpr uint32_t kTcImageBytes = (uint32_t)offsetof(TcSmem, a);
+static_assert(offsetof(TcSmem, w1) == 0 && kTcImageBytes % 16 == 0 && kTcImageBytes == sizeof(uint16_t) * GUIDE_WEIGHTS,
+              "the weight image must be the contiguous weight region of the inference CTA's shared memory");
 
 __device__ __forceinline__ uint32_t smemU32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -291,6 +318,14 @@ __device__ __forceinline__ void umma(uint32_t tmem, uint64_t a, uint64_t b, uint
         "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
+// the same with A's rows in tensor memory (lane = row, two BF16 along K per column)
+__device__ __forceinline__ void ummaTmem(uint32_t tmem, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem),
+        "r"(a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+
 __device__ __forceinline__ void ummaCommit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
                  : "memory");
@@ -310,11 +345,8 @@ __device__ __forceinline__ bool mbarWait(uint32_t mbar, uint32_t phase) {
     return false;
 }
 
-// barrier of one pipeline's 128 threads (named barrier 1 + pipe)
-__device__ __forceinline__ void pipeSync(int pipe) {
-    asm volatile("bar.sync %0, %1;\n" ::"r"(1 + pipe), "r"(kTcPipeThreads) : "memory");
-}
-// pipeline barrier that also tells whether any of its threads passed true
+// barrier of one pipeline's 128 threads (named barrier 1 + pipe) that also
+// tells whether any of them passed true
 __device__ __forceinline__ bool pipeAny(int pipe, bool v) {
     uint32_t r;
     asm volatile(
@@ -348,6 +380,18 @@ __device__ __forceinline__ void tmemLd16(uint32_t taddr, float *v) {
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
+// 32 columns of the warp's lanes written from registers, and the wait for them
+__device__ __forceinline__ void tmemSt32(uint32_t taddr, const uint32_t *r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};\n"
+        "tcgen05.wait::st.sync.aligned;\n" ::"r"(r[0]),
+        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+        "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+        "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmemLdWait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 // the wait, with v[0..32) tied to it, so no use of them moves above it
 __device__ __forceinline__ void tmemLdWaitFor(float *v) {
@@ -360,33 +404,27 @@ __device__ __forceinline__ void tcFenceBefore() { asm volatile("tcgen05.fence::b
 __device__ __forceinline__ void tcFenceAfter() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void asyncProxyFence() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-// copies a row-major [rows][K] bf16 weight matrix into the canonical layout
-__device__ void loadCanonical(uint16_t *dst, const uint16_t *src, int rows, int K) {
-    const int chunks = K / 8;
-    for (int i = threadIdx.x; i < rows * chunks; i += blockDim.x) {
-        const int r = i / chunks, c = i - r * chunks;
-        *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(dst) + canonOffset(r, 8 * c, K)) =
-            __ldg(reinterpret_cast<const uint4 *>(&src[r * K + 8 * c]));
-    }
-}
-
-// The CTA's set-up: weights and biases into shared memory, the pipelines'
-// mbarriers, and kTmemCols columns of tensor memory (warp 0 allocates).
+// The CTA's set-up: the weight image on its way into shared memory (it already
+// has that layout; mbarrier kTcPipes completes with it), the biases, the
+// pipelines' mbarriers, and kTmemCols columns of tensor memory (warp 0
+// allocates).  Reads only the network, which no kernel of an iteration writes,
+// so it runs before the wait for the kernel before.
 __device__ void tcSetup(TcSmem &sm, const GuideNetView &net) {
-    loadCanonical(sm.w1, net.w[0], GUIDE_HIDDEN, GUIDE_INPUTS);
-    loadCanonical(sm.w2, net.w[1], GUIDE_HIDDEN, GUIDE_HIDDEN);
-    loadCanonical(sm.w3, net.w[2], GUIDE_HIDDEN, GUIDE_HIDDEN);
-    loadCanonical(sm.w4, net.w[3], GUIDE_OUTPUTS, GUIDE_HIDDEN);
+    if (threadIdx.x == 0) {
+        for (int p = 0; p <= kTcPipes; p++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smemU32(&sm.mbar[p])), "r"(1) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        const uint32_t mbar = smemU32(&sm.mbar[kTcPipes]);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(kTcImageBytes)
+                     : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                         smemU32(sm.w1)),
+                     "l"(net.image), "r"(kTcImageBytes), "r"(mbar)
+                     : "memory");
+    }
     for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) {
         const int l = min(i / GUIDE_HIDDEN, 3);
         sm.b[i] = __ldg(&net.b[l][i - l * GUIDE_HIDDEN]);
-    }
-    if (threadIdx.x == 0) {
-        for (int p = 0; p < kTcPipes; p++) {
-            sm.failed[p] = 0;
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smemU32(&sm.mbar[p])), "r"(1) : "memory");
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if ((threadIdx.x >> 5) == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemU32(&sm.tmemBase)),
@@ -394,14 +432,21 @@ __device__ void tcSetup(TcSmem &sm, const GuideNetView &net) {
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    asyncProxyFence();
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
 }
 
+// A pipeline's starting `phase`, once the weights have arrived.
+__device__ __forceinline__ uint32_t tcStart(TcSmem &sm) {
+    return mbarWait(smemU32(&sm.mbar[kTcPipes]), 0u) ? 0u : kTcFailed;
+}
+
 __device__ void tcTeardown(TcSmem &sm, int pipe, uint32_t phase) {
-    if (sm.failed[pipe]) mbarWait(smemU32(&sm.mbar[pipe]), phase);  // a last bounded wait for work in flight
+    if (phase & kTcFailed) {  // a last bounded wait for work in flight
+        mbarWait(smemU32(&sm.mbar[kTcPipes]), 0u);
+        mbarWait(smemU32(&sm.mbar[pipe]), phase & 1u);
+    }
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
@@ -410,95 +455,108 @@ __device__ void tcTeardown(TcSmem &sm, int pipe, uint32_t phase) {
                      : "memory");
 }
 
-// One layer of a pipeline: D (its TMEM columns) = A (its sm.a, [128][K]) x
-// W^T (W [N][K]); the pipeline's first thread issues, all its threads wait.
-// False if the wait expired (the pipeline then stops).
-__device__ bool tcLayer(TcSmem &sm, int pipe, const uint16_t *w, int K, int N, uint32_t &phase) {
-    asyncProxyFence();  // the A rows written by the pipeline's threads, visible to the tensor core
+// One layer of a pipeline: D (its TMEM columns) = A x W^T (W [N][K]); A is
+// its input rows in shared memory (FIRST) or its hidden rows in tensor memory.
+// The pipeline's first thread issues, all its threads wait.  A thread whose
+// wait expires notes that in its `phase`; the barrier before the pipeline's
+// next layer tells all its threads, which stop there together, so a layer
+// needs no second barrier after its wait.  False if a wait of an earlier layer
+// has expired.
+template <bool FIRST>
+__device__ __forceinline__ bool tcLayer(TcSmem &sm, int pipe, const uint16_t *w, int K, int N, uint32_t &phase) {
+    if (FIRST) asyncProxyFence();  // the input rows written by the pipeline's threads, visible to the tensor core
     tcFenceBefore();
-    pipeSync(pipe);
+    const bool failed = pipeAny(pipe, phase & kTcFailed);
     tcFenceAfter();
+    if (failed) return false;
     const uint32_t mbar = smemU32(&sm.mbar[pipe]);
     if ((threadIdx.x & (kTcPipeThreads - 1)) == 0) {
         const uint32_t idesc = ummaInstr(kTcPipeThreads, N);
         const uint32_t aBase = smemU32(sm.a[pipe]), bBase = smemU32(w);
         const uint32_t sbo = (uint32_t)(K / 8) * 128u;
-        const uint32_t tmem = sm.tmemBase + 64u * pipe;
-        for (int kb = 0; kb < K / 16; kb++)
-            umma(tmem, ummaDesc(aBase + kb * 256u, sbo), ummaDesc(bBase + kb * 256u, sbo), idesc, kb > 0);
+        const uint32_t tmem = sm.tmemBase + kTmemPipe * pipe;
+#pragma unroll
+        for (int kb = 0; kb < K / 16; kb++) {
+            const uint64_t b = ummaDesc(bBase + kb * 256u, sbo);
+            if (FIRST) umma(tmem, ummaDesc(aBase + kb * 256u, sbo), b, idesc, kb > 0);
+            else ummaTmem(tmem, tmem + kTmemHidden + 8u * kb, b, idesc, kb > 0);
+        }
         ummaCommit(mbar);
     }
-    // on expiry `phase` stays that of the commit in flight, which the
+    // on expiry `phase` keeps the parity of the commit in flight, which the
     // teardown's last bounded wait then waits for
-    const bool ok = mbarWait(mbar, phase);
-    if (ok) phase ^= 1u;
+    if (mbarWait(mbar, phase & 1u)) phase ^= 1u;
+    else phase |= kTcFailed;
+    __syncwarp();
     tcFenceAfter();
-    if (!ok) atomicExch(&sm.failed[pipe], 1);
-    pipeSync(pipe);
-    return sm.failed[pipe] == 0;
+    return true;
 }
 
-// bias + ReLU of a 64-wide hidden row from TMEM, written as the next A row
-__device__ void tcHiddenEpilogue(uint16_t *a, uint32_t taddr, const float *bias, int row) {
-    float v[32];
+// bias + ReLU of a 64-wide hidden row, from the accumulator's columns to the
+// hidden rows' (the next layer's A operand)
+__device__ __forceinline__ void tcHiddenEpilogue(uint32_t taddr, const float *bias) {
+    uint32_t q[32];
 #pragma unroll
     for (int half = 0; half < 2; half++) {
+        float v[32];
         tmemLd32(taddr + 32u * half, v);
         tmemLdWait();
 #pragma unroll
-        for (int c = 0; c < 32; c += 8) {
-            uint32_t q[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                q[k] = biasReluBf16x2(v[c + 2 * k], v[c + 2 * k + 1],
-                                      *reinterpret_cast<const float2 *>(&bias[32 * half + c + 2 * k]));
-            *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(a) +
-                                       canonOffset(row, 32 * half + c, GUIDE_HIDDEN)) = make_uint4(q[0], q[1], q[2], q[3]);
+        for (int k = 0; k < 16; k += 2) {
+            const float4 b = *reinterpret_cast<const float4 *>(&bias[32 * half + 2 * k]);
+            q[16 * half + k] = biasReluBf16x2(v[2 * k], v[2 * k + 1], make_float2(b.x, b.y));
+            q[16 * half + k + 1] = biasReluBf16x2(v[2 * k + 2], v[2 * k + 3], make_float2(b.z, b.w));
         }
+    }
+    tmemSt32(taddr + kTmemHidden, q);
+}
+
+// The one-blob columns [first, first + BINS) of a row for a feature's value v,
+// every 16-byte chunk written once.  v is non-zero only in bins
+// b = floor(v BINS - 1/2) and b + 1 (|v BINS - (bin + 1/2)| < 1); `even` and
+// `odd` are the two columns' values as the 32-bit words b / 2 and b / 2 + 1.
+template <int BINS>
+__device__ __forceinline__ void oneBlobColumns(unsigned char *a, int row, int first, float v) {
+    const int b = (int)floorf(v * (float)BINS - 0.5f);
+    const uint32_t pair = cvtBf16x2(oneBlob(v, BINS, b), oneBlob(v, BINS, b + 1));
+    const int word = b >> 1;
+    const uint32_t even = (b & 1) ? pair << 16 : pair, odd = (b & 1) ? pair >> 16 : 0u;
+#pragma unroll
+    for (int c = 0; c < BINS / 8; c++) {
+        uint32_t q[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) q[k] = word == 4 * c + k ? even : word == 4 * c + k - 1 ? odd : 0u;
+        *reinterpret_cast<uint4 *>(a + canonOffset(row, first + 8 * c, GUIDE_INPUTS)) = make_uint4(q[0], q[1], q[2], q[3]);
     }
 }
 
 // Forward pass of a pipeline's 128 samples (its thread r: sample r, features
 // f); writes the 48 raw outputs to `o`.  False if a wait expired.
-__device__ bool tcForward(TcSmem &sm, int pipe, const GuideFeatures &f, float *o, uint32_t &phase) {
+__device__ __forceinline__ bool tcForward(TcSmem &sm, int pipe, const GuideFeatures &f, float *o, uint32_t &phase) {
     const int row = threadIdx.x & (kTcPipeThreads - 1);
-    uint16_t *a = sm.a[pipe];
-    // one-blob input row.  A feature v with b bins is non-zero only in bins
-    // floor(v b - 1/2) and the one after (|v b - (bin + 1/2)| < 1), so the
-    // row is cleared and those two bins of each of the 7 features written.
-    unsigned char *aRow = reinterpret_cast<unsigned char *>(a);
+    unsigned char *a = reinterpret_cast<unsigned char *>(sm.a[pipe]);
 #pragma unroll
-    for (int c = 0; c < GUIDE_INPUTS / 8; c++)
-        *reinterpret_cast<uint4 *>(aRow + canonOffset(row, 8 * c, GUIDE_INPUTS)) = make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < 3; k++) oneBlobColumns<32>(a, row, 32 * k, f.v[k]);
 #pragma unroll
-    for (int feature = 0; feature < 7; feature++) {
-        const int bins = feature < 3 ? 32 : 16;
-        const int first = feature < 3 ? 32 * feature : 96 + 16 * (feature - 3);
-        const float v = f.v[feature];
-        const int b = (int)floorf(v * (float)bins - 0.5f);
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int bin = b + k;
-            if (bin >= 0 && bin < bins)
-                *reinterpret_cast<uint16_t *>(aRow + canonOffset(row, first + bin, GUIDE_INPUTS)) =
-                    cvtBf16(oneBlob(v, bins, bin));
-        }
-    }
-    // this warp's 32 lanes (its quarter of the pipeline's rows) in the pipeline's 64 columns
-    const uint32_t taddr = sm.tmemBase + 64u * pipe + ((uint32_t)(row & ~31) << 16);
-    if (!tcLayer(sm, pipe, sm.w1, GUIDE_INPUTS, GUIDE_HIDDEN, phase)) return false;
-    tcHiddenEpilogue(a, taddr, sm.b, row);
-    if (!tcLayer(sm, pipe, sm.w2, GUIDE_HIDDEN, GUIDE_HIDDEN, phase)) return false;
-    tcHiddenEpilogue(a, taddr, sm.b + GUIDE_HIDDEN, row);
-    if (!tcLayer(sm, pipe, sm.w3, GUIDE_HIDDEN, GUIDE_HIDDEN, phase)) return false;
-    tcHiddenEpilogue(a, taddr, sm.b + 2 * GUIDE_HIDDEN, row);
-    if (!tcLayer(sm, pipe, sm.w4, GUIDE_HIDDEN, GUIDE_OUTPUTS, phase)) return false;
+    for (int k = 0; k < 4; k++) oneBlobColumns<16>(a, row, 96 + 16 * k, f.v[3 + k]);
+    // this warp's 32 lanes (its quarter of the pipeline's rows) in the pipeline's columns
+    const uint32_t taddr = sm.tmemBase + kTmemPipe * pipe + ((uint32_t)(row & ~31) << 16);
+    if (!tcLayer<true>(sm, pipe, sm.w1, GUIDE_INPUTS, GUIDE_HIDDEN, phase)) return false;
+    tcHiddenEpilogue(taddr, sm.b);
+    if (!tcLayer<false>(sm, pipe, sm.w2, GUIDE_HIDDEN, GUIDE_HIDDEN, phase)) return false;
+    tcHiddenEpilogue(taddr, sm.b + GUIDE_HIDDEN);
+    if (!tcLayer<false>(sm, pipe, sm.w3, GUIDE_HIDDEN, GUIDE_HIDDEN, phase)) return false;
+    tcHiddenEpilogue(taddr, sm.b + 2 * GUIDE_HIDDEN);
+    if (!tcLayer<false>(sm, pipe, sm.w4, GUIDE_HIDDEN, GUIDE_OUTPUTS, phase)) return false;
     tmemLd32(taddr, o);
     tmemLd16(taddr + 32u, o + 32);
     tmemLdWait();
-    const float2 *b4 = reinterpret_cast<const float2 *>(sm.b + 3 * GUIDE_HIDDEN);
+    const float4 *b4 = reinterpret_cast<const float4 *>(sm.b + 3 * GUIDE_HIDDEN);
 #pragma unroll
-    for (int c = 0; c < GUIDE_OUTPUTS / 2; c++) addBias2(o[2 * c], o[2 * c + 1], b4[c]);
+    for (int c = 0; c < GUIDE_OUTPUTS / 4; c++) {
+        addBias2(o[4 * c], o[4 * c + 1], make_float2(b4[c].x, b4[c].y));
+        addBias2(o[4 * c + 2], o[4 * c + 3], make_float2(b4[c].z, b4[c].w));
+    }
     return true;
 }
 
@@ -965,6 +1023,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
 // coalesced 16-byte record per hit.
 __global__ void __launch_bounds__(256) k_guide_features(Context ctx, PathPool pool, Counters *cnt, uint32_t p,
                                                         uint32_t guideDepth) {
+    waitForPreviousKernel();
     const uint32_t nHit = cnt->nHit;
     const PathState S = pool.s[p];
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nHit; q += gridDim.x * blockDim.x) {
@@ -997,26 +1056,29 @@ __global__ void __launch_bounds__(kTcThreads) k_guide_infer(Counters *cnt, const
     extern __shared__ __align__(16) unsigned char smem[];
     TcSmem &sm = *reinterpret_cast<TcSmem *>(smem);
     tcSetup(sm, net);
+    waitForPreviousKernel();
     const int pipe = threadIdx.x / kTcPipeThreads, row = threadIdx.x & (kTcPipeThreads - 1);
     const uint32_t nHit = cnt->nHit;
     const uint32_t tiles = (nHit + kTcPipeThreads - 1) / kTcPipeThreads;
-    uint32_t phase = 0;
-    for (uint32_t tile = blockIdx.x * kTcPipes + pipe; tile < tiles; tile += gridDim.x * kTcPipes) {
-        const uint32_t q = tile * kTcPipeThreads + row;
-        uint4 packed = make_uint4(0u, 0u, 0u, 0xffff0000u);
-        if (q < nHit) packed = __ldcs(&features[q]);
+    uint32_t phase = tcStart(sm);
+    const uint32_t step = gridDim.x * kTcPipes * kTcPipeThreads;
+    const uint32_t first = pipe * gridDim.x + blockIdx.x;  // few tiles spread over all SMs
+    uint32_t q = first * kTcPipeThreads + row;
+    uint4 next = make_uint4(0u, 0u, 0u, 0xffff0000u);
+    if (q < nHit) next = __ldcs(&features[q]);
+    for (uint32_t tile = first; tile < tiles; tile += gridDim.x * kTcPipes, q += step) {
+        const uint4 packed = next;  // the next tile's are in flight meanwhile
+        if (q + step < nHit) next = __ldcs(&features[q + step]);
         const bool valid = q < nHit && (packed.w >> 16) < guideDepth;
         if (!pipeAny(pipe, valid)) continue;  // no guided vertex in this tile
         const GuideFeatures f = unpackFeatures(packed);
         float o[GUIDE_OUTPUTS];
-        if (!tcForward(sm, pipe, f, o, phase)) {
-            if (row == 0) atomicOr(&cnt->errors, ERR_GUIDE_TIMEOUT);
-            break;
-        }
+        if (!tcForward(sm, pipe, f, o, phase)) break;
         // Rows past the guided depth are written too; shading reads a mixture
         // only at guided depths.
         if (q < nHit) storeMixture(out + guideMixtureAt(q), pack(decode(o)));
     }
+    if (phase & kTcFailed) atomicOr(&cnt->errors, ERR_GUIDE_TIMEOUT);
     tcTeardown(sm, pipe, phase);
 }
 
@@ -1086,20 +1148,18 @@ __global__ void __launch_bounds__(kTcThreads) k_guide_forward_test(const float *
     tcSetup(sm, net);
     const int pipe = threadIdx.x / kTcPipeThreads, row = threadIdx.x & (kTcPipeThreads - 1);
     const uint32_t tiles = (n + kTcPipeThreads - 1) / kTcPipeThreads;
-    uint32_t phase = 0;
+    uint32_t phase = tcStart(sm);
     for (uint32_t tile = blockIdx.x * kTcPipes + pipe; tile < tiles; tile += gridDim.x * kTcPipes) {
         const uint32_t q = tile * kTcPipeThreads + row;
         GuideFeatures f = {};
         if (q < n)
             for (int k = 0; k < 7; k++) f.v[k] = features[7 * q + k];
         float o[GUIDE_OUTPUTS];
-        if (!tcForward(sm, pipe, f, o, phase)) {
-            if (row == 0) atomicExch(status, 1);
-            break;
-        }
+        if (!tcForward(sm, pipe, f, o, phase)) break;
         if (q < n)
             for (int c = 0; c < GUIDE_OUTPUTS; c++) out[GUIDE_OUTPUTS * q + c] = o[c];
     }
+    if (phase & kTcFailed) atomicExch(status, 1);
     tcTeardown(sm, pipe, phase);
 }
 
@@ -1149,24 +1209,6 @@ cudaError_t rmdGuideConfigure() {
                                 (int)rmdGuideSharedBytes(false));
 }
 
-cudaError_t rmdLaunchGuideInfer(const Context &ctx, const PathPool &pool, Counters *cnt, uint32_t cur,
-                                uint32_t guideDepth, const GuideNetView &net, uint4 *out, int blocks,
-                                cudaStream_t s) {
-    k_guide_features<<<pool.capacity / 256 < 1184u ? pool.capacity / 256 + 1 : 1184, 256, 0, s>>>(ctx, pool, cnt, cur,
-                                                                                              guideDepth);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_guide_infer<<<blocks, kTcThreads, rmdGuideSharedBytes(false), s>>>(cnt, pool.guideFeat, guideDepth, net, out);
-    return cudaGetLastError();
-}
-
-constexpr float kAdamBeta1 = 0.9f, kAdamBeta2 = 0.999f;
-// Adam's bias corrections 1 / (1 - beta^step)
-static void adamCorrections(int step, float &corr1, float &corr2) {
-    corr1 = 1.0f / (1.0f - powf(kAdamBeta1, (float)step));
-    corr2 = 1.0f / (1.0f - powf(kAdamBeta2, (float)step));
-}
-
 // Launches `kernel` allowed to start while the kernel before it in the
 // stream finishes (programmatic dependent launch); the kernel waits for that
 // grid before reading its results (gridDependencyWait).
@@ -1184,6 +1226,23 @@ static cudaError_t launchOverlapped(void (*kernel)(Params...), dim3 grid, dim3 b
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+cudaError_t rmdLaunchGuideInfer(const Context &ctx, const PathPool &pool, Counters *cnt, uint32_t cur,
+                                uint32_t guideDepth, const GuideNetView &net, uint4 *out, int blocks,
+                                cudaStream_t s) {
+    const uint32_t featureBlocks = pool.capacity / 256 < 1184u ? pool.capacity / 256 + 1 : 1184;
+    cudaError_t e = launchOverlapped(k_guide_features, dim3(featureBlocks), dim3(256), 0, s, ctx, pool, cnt, cur, guideDepth);
+    if (e != cudaSuccess) return e;
+    return launchOverlapped(k_guide_infer, dim3(blocks), dim3(kTcThreads), rmdGuideSharedBytes(false), s, cnt,
+                            pool.guideFeat, guideDepth, net, out);
+}
+
+constexpr float kAdamBeta1 = 0.9f, kAdamBeta2 = 0.999f;
+// Adam's bias corrections 1 / (1 - beta^step)
+static void adamCorrections(int step, float &corr1, float &corr2) {
+    corr1 = 1.0f / (1.0f - powf(kAdamBeta1, (float)step));
+    corr2 = 1.0f / (1.0f - powf(kAdamBeta2, (float)step));
 }
 
 cudaError_t rmdLaunchGuideTrain(const GuideRecord *rec, uint32_t total, uint32_t n, uint32_t seed, uint32_t steps,
