@@ -181,6 +181,18 @@ struct RecordBatch {
         h ^= h >> 16;
         return rec[h % total];
     }
+    // a record read from L2 (ahead of a wait for the kernel before)
+    __device__ GuideRecord load(uint32_t i) const {
+        union {
+            float4 q[3];
+            GuideRecord r;
+        } u;
+        static_assert(sizeof(GuideRecord) == sizeof(u.q), "a record is three 16-byte chunks");
+        const float4 *src = reinterpret_cast<const float4 *>(&pick(i));
+#pragma unroll
+        for (int k = 0; k < 3; k++) u.q[k] = __ldcg(&src[k]);
+        return u.r;
+    }
 };
 
 // one-blob value of bin `bin` of a feature with `bins` bins
@@ -266,13 +278,6 @@ __device__ __forceinline__ uint32_t biasReluBf16x2(float lo, float hi, float2 bi
         "cvt.rn.relu.bf16x2.f32 %0, h, l;\n}\n"
         : "=r"(r)
         : "f"(lo), "f"(hi), "f"(bias.x), "f"(bias.y));
-    return r;
-}
-
-// BF16 of a float, round to nearest even
-__device__ __forceinline__ uint16_t cvtBf16(float x) {
-    uint16_t r;
-    asm("cvt.rn.bf16.f32 %0, %1;\n" : "=h"(r) : "f"(x));
     return r;
 }
 
@@ -424,7 +429,7 @@ __device__ void tcSetup(TcSmem &sm, const GuideNetView &net) {
     }
     for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) {
         const int l = min(i / GUIDE_HIDDEN, 3);
-        sm.b[i] = __ldg(&net.b[l][i - l * GUIDE_HIDDEN]);
+        sm.b[i] = __ldcg(&net.b[l][i - l * GUIDE_HIDDEN]);
     }
     if ((threadIdx.x >> 5) == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemU32(&sm.tmemBase)),
@@ -590,7 +595,8 @@ __device__ __forceinline__ bool tcForward(TcSmem &sm, int pipe, const GuideFeatu
 // deltas) are reduced across each warp with shuffles into shared memory.  At
 // the end warps 0 and 1 (lanes 0..63, the output features) read the CTA's
 // weight gradient out of tensor memory into the CTA's slot of net.partials.
-constexpr int kTrThreads = 128;
+constexpr int kTrRows = 128;                // records of a tile (M of the forward layers)
+constexpr int kTrThreads = 2 * kTrRows;     // two threads per record, each one half of a layer's columns
 constexpr uint32_t kTrTmemCols = 512;
 // tensor-memory column of dW_l: dW0 at 64 (160 wide), dW1 224, dW2 288, dW3 352
 __device__ __forceinline__ uint32_t trColDw(int l) { return l == 0 ? 64u : 224u + 64u * (uint32_t)(l - 1); }
@@ -600,15 +606,14 @@ struct TrainSmem {
     uint16_t w1[GUIDE_HIDDEN * GUIDE_HIDDEN];
     uint16_t w2[GUIDE_HIDDEN * GUIDE_HIDDEN];
     uint16_t w3[GUIDE_OUTPUTS * GUIDE_HIDDEN];
-    uint16_t d[2][kTrThreads * GUIDE_HIDDEN];  // delta rows [record][feature], ping-pong (delta_3 is 48 wide)
-    uint16_t x[kTrThreads * GUIDE_INPUTS];     // one-blob input rows; follows the deltas (see above)
-    uint16_t h[3][kTrThreads * GUIDE_HIDDEN];  // hidden activation rows, the inputs of layers 1..3
+    uint16_t d[2][kTrRows * GUIDE_HIDDEN];  // delta rows [record][feature], ping-pong (delta_3 is 48 wide)
+    uint16_t x[kTrRows * GUIDE_INPUTS];     // one-blob input rows; follows the deltas (see above)
+    uint16_t h[3][kTrRows * GUIDE_HIDDEN];  // hidden activation rows, the inputs of layers 1..3
     float b[3 * GUIDE_HIDDEN + GUIDE_OUTPUTS];
     float db[3 * GUIDE_HIDDEN + GUIDE_OUTPUTS];  // the CTA's bias gradient
     float reduce[8];                             // per warp: loss sums
     unsigned long long mbar;
     uint32_t tmemBase;
-    int failed;
 };
 static_assert(sizeof(TrainSmem) <= 232448, "training shared memory exceeds the per-CTA limit");
 static_assert(GUIDE_PARAMS % 4 == 0 && (GUIDE_HIDDEN * GUIDE_INPUTS + GUIDE_HIDDEN) % 4 == 0 &&
@@ -622,8 +627,8 @@ static_assert(offsetof(TrainSmem, w0) == 0 && kImageBytes % 16 == 0 &&
 // An MN-major A of M = 128 over a delta buffer of width F reads up to byte
 // 15 * 16F + 2047 from its start (16 record groups of 16F bytes, 16 chunks of
 // 128 bytes): at most 2 KB past the buffer, which must stay inside TrainSmem.
-static_assert(offsetof(TrainSmem, x) == offsetof(TrainSmem, d) + sizeof(uint16_t) * 2 * kTrThreads * GUIDE_HIDDEN &&
-                  sizeof(uint16_t) * kTrThreads * GUIDE_INPUTS >= 2048,
+static_assert(offsetof(TrainSmem, x) == offsetof(TrainSmem, d) + sizeof(uint16_t) * 2 * kTrRows * GUIDE_HIDDEN &&
+                  sizeof(uint16_t) * kTrRows * GUIDE_INPUTS >= 2048,
               "the padded delta rows of a weight gradient must read inside shared memory");
 
 // Sum over the warp's 32 lanes of each of v[0..31]: afterwards lane l holds
@@ -664,87 +669,75 @@ __device__ __forceinline__ TrOperand mnMajor(const void *rows, int F) {
 
 // issues D (tmem) = A . B^T over K, N columns (accumulating if asked); committed later
 __device__ __forceinline__ void trMma(uint32_t tmem, TrOperand a, TrOperand b, int K, int N, bool accumulate) {
-    const uint32_t idesc = ummaInstr(kTrThreads, N) | (a.mnMajor << 15) | (b.mnMajor << 16);
+    const uint32_t idesc = ummaInstr(kTrRows, N) | (a.mnMajor << 15) | (b.mnMajor << 16);
     for (int kb = 0; kb < K / 16; kb++)
         umma(tmem, ummaDesc(a.addr + kb * a.kStep, a.lbo, a.sbo), ummaDesc(b.addr + kb * b.kStep, b.lbo, b.sbo),
              idesc, (accumulate || kb > 0) ? 1u : 0u);
 }
 
-// makes the threads' shared-memory writes visible to the tensor core and syncs the CTA
-__device__ __forceinline__ void trPublish() {
+// makes the threads' shared-memory writes visible to the tensor core and syncs
+// the CTA; false if a thread's wait has expired (all of them then stop)
+__device__ __forceinline__ bool trPublish(bool failed) {
     asyncProxyFence();
     tcFenceBefore();
-    __syncthreads();
+    const bool any = __syncthreads_or(failed);
+    tcFenceAfter();
+    return !any;
+}
+
+// waits for the MMAs that thread 0 issued and committed; notes an expired wait
+__device__ __forceinline__ void trWait(TrainSmem &sm, uint32_t &phase, bool &failed) {
+    if (mbarWait(smemU32(&sm.mbar), phase)) phase ^= 1u;  // else the teardown waits for the work in flight
+    else failed = true;
+    __syncwarp();
     tcFenceAfter();
 }
 
-// thread 0 commits the issued MMAs; everyone waits.  False if the wait expired.
-__device__ bool trCommitWait(TrainSmem &sm, uint32_t &phase) {
-    const uint32_t mbar = smemU32(&sm.mbar);
-    if (threadIdx.x == 0) ummaCommit(mbar);
-    const bool ok = mbarWait(mbar, phase);
-    if (ok) phase ^= 1u;  // else the teardown waits for the commit in flight
-    tcFenceAfter();
-    if (!ok) atomicExch(&sm.failed, 1);
-    __syncthreads();
-    return sm.failed == 0;
-}
-
-// Epilogue of a forward hidden layer: bias + ReLU of the thread's row of the
-// accumulator, written as the next layer's A row (kept for the backward
-// pass); returns the ReLU mask (bit c: column c positive).
-// The epilogues run three times per tile, and a CTA traces its code once per
-// Adam step: kept out of line and not unrolled over the two column halves, so
-// the second and later calls find their instructions cached (instruction
-// fetch, not the tensor cores, bounds a step).
-__device__ __noinline__ uint64_t trHiddenEpilogue(uint32_t taddr, const float *bias, uint16_t *rowOut, int row) {
-    uint64_t mask = 0;
+// Epilogue of a forward hidden layer: bias + ReLU of 32 columns of the row of
+// the accumulator, written as those of the next layer's A row (kept for the
+// backward pass); returns their ReLU mask (bit c: column c positive).
+// `first`: their first column.
+__device__ __forceinline__ uint32_t trHiddenEpilogue(uint32_t taddr, const float *bias, uint16_t *rowOut, int row,
+                                                     int first) {
+    uint32_t mask = 0;
     float v[32];
-#pragma unroll 1
-    for (int half = 0; half < 2; half++) {
-        tmemLd32(taddr + 32u * half, v);
-        tmemLdWait();
+    tmemLd32(taddr + (uint32_t)first, v);
+    tmemLdWait();
 #pragma unroll
-        for (int c = 0; c < 32; c += 8) {
-            uint32_t q[4];
+    for (int c = 0; c < 32; c += 8) {
+        uint32_t q[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                q[k] = biasReluBf16x2(v[c + 2 * k], v[c + 2 * k + 1],
-                                      *reinterpret_cast<const float2 *>(&bias[32 * half + c + 2 * k]));
-            *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(rowOut) +
-                                       canonOffset(row, 32 * half + c, GUIDE_HIDDEN)) = make_uint4(q[0], q[1], q[2], q[3]);
+        for (int k = 0; k < 4; k++)
+            q[k] = biasReluBf16x2(v[c + 2 * k], v[c + 2 * k + 1], *reinterpret_cast<const float2 *>(&bias[first + c + 2 * k]));
+        *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(rowOut) + canonOffset(row, first + c, GUIDE_HIDDEN)) =
+            make_uint4(q[0], q[1], q[2], q[3]);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int col = 32 * half + c + 2 * k;
-                mask |= (uint64_t)((q[k] & 0xffffu) != 0u) << col;
-                mask |= (uint64_t)((q[k] >> 16) != 0u) << (col + 1);
-            }
+        for (int k = 0; k < 4; k++) {
+            mask |= (uint32_t)((q[k] & 0xffffu) != 0u) << (c + 2 * k);
+            mask |= (uint32_t)((q[k] >> 16) != 0u) << (c + 2 * k + 1);
         }
     }
     return mask;
 }
 
-// Epilogue of a backward layer: the thread's row of delta . W masked by the
-// ReLU mask, as BF16 delta rows; bias gradient into db[0..64).
-__device__ __noinline__ void trDeltaEpilogue(uint32_t taddr, uint64_t mask, uint16_t *rowOut, float *db, int row,
-                                             int lane) {
-    float v[32];
-#pragma unroll 1
-    for (int half = 0; half < 2; half++) {
-        tmemLd32(taddr + 32u * half, v);
-        tmemLdWait();
+// Epilogue of a backward layer: 32 columns of the row of delta . W masked by
+// the ReLU mask, as BF16 delta rows; leaves the rounded deltas in v.
+__device__ __forceinline__ void trDeltaEpilogue(uint32_t taddr, uint32_t mask, uint16_t *rowOut, int row, int first,
+                                                float *v) {
+    tmemLd32(taddr + (uint32_t)first, v);
+    tmemLdWait();
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-            const int col = 32 * half + c;
-            const float a = ((mask >> col) & 1u) ? v[c] : 0.0f;
-            const float b = ((mask >> (col + 1)) & 1u) ? v[c + 1] : 0.0f;
-            const uint16_t lo = cvtBf16(a), hi = cvtBf16(b);
-            *reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(rowOut) +
-                                          canonOffset(row, col, GUIDE_HIDDEN)) = (uint32_t)lo | ((uint32_t)hi << 16);
-            v[c] = fromBf16(lo);  // the bias gradient sums the rounded deltas the MMAs use
-            v[c + 1] = fromBf16(hi);
+    for (int c = 0; c < 32; c += 8) {
+        uint32_t q[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int col = c + 2 * k;
+            q[k] = cvtBf16x2(((mask >> col) & 1u) ? v[col] : 0.0f, ((mask >> (col + 1)) & 1u) ? v[col + 1] : 0.0f);
+            v[col] = bf16Lo(q[k]);  // the bias gradient sums the rounded deltas the MMAs use
+            v[col + 1] = bf16Hi(q[k]);
         }
-        addBiasGrad(db, 32 * half, v, lane);
+        *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(rowOut) + canonOffset(row, first + c, GUIDE_HIDDEN)) =
+            make_uint4(q[0], q[1], q[2], q[3]);
     }
 }
 
@@ -777,166 +770,146 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
                                                                 GuideNetView net, uint32_t *errors) {
     extern __shared__ __align__(16) unsigned char smem[];
     TrainSmem &sm = *reinterpret_cast<TrainSmem *>(smem);
-    const int row = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    gridDependencyWait();  // the previous Adam step's weights (launched overlapped with it)
-    // set-up: the weights (forward and transposed, already in their shared-
-    // memory layout) arrive by one bulk copy on the mbarrier's phase 0 while
-    // the biases load, the tensor memory is allocated and the inputs encode
+    const int row = threadIdx.x & (kTrRows - 1), half = threadIdx.x / kTrRows;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Set-up, while the previous Adam step (launched before, overlapped) still
+    // runs: nothing up to gridDependencyWait depends on it.
     if (threadIdx.x == 0) {
-        sm.failed = 0;
-        const uint32_t mbar = smemU32(&sm.mbar);
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(1) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smemU32(&sm.mbar)), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(kImageBytes)
-                     : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                         smemU32(sm.w0)),
-                     "l"(net.image), "r"(kImageBytes), "r"(mbar)
-                     : "memory");
     }
-    for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) {
-        const int l = min(i / GUIDE_HIDDEN, 3);
-        sm.b[i] = __ldg(&net.b[l][i - l * GUIDE_HIDDEN]);
-        sm.db[i] = 0.0f;
-    }
+    for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) sm.db[i] = 0.0f;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemU32(&sm.tmemBase)),
                      "r"(kTrTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    trPublish();
+    trPublish(false);
     const uint32_t tmem = sm.tmemBase;
     const uint32_t taddr = tmem + ((uint32_t)(row & ~31) << 16);  // this warp's lanes, work columns
     const uint32_t n = batch.n;
     const float scale = 1.0f / (float)n;
-    const float invMeanY = sumY[0] > 0.0f ? (float)n / sumY[0] : 0.0f;
-    const uint32_t tiles = (n + kTrThreads - 1) / kTrThreads;
+    float invMeanY = 0.0f;
+    const uint32_t tiles = (n + kTrRows - 1) / kTrRows;
     float lossSum = 0.0f;
     uint32_t phase = 0;
-    bool first = true, ok = true;
-    {  // the weight image (phase 0); the MMA commits follow on phase 1, 0, ...
-        const bool arrived = mbarWait(smemU32(&sm.mbar), phase);
-        if (arrived) phase ^= 1u;  // else the teardown waits for the copy in flight
-        else atomicExch(&sm.failed, 1);
-        __syncthreads();
-        ok = sm.failed == 0;
-    }
-    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const uint32_t r = tile * kTrThreads + row;
-        GuideRecord rc = {};
+    bool first = true, failed = false, waited = false;
+    auto weights = [&](int l) { return l == 0 ? sm.w0 : sm.w1 + (l - 1) * GUIDE_HIDDEN * GUIDE_HIDDEN; };
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t r = tile * kTrRows + row;
         const bool valid = r < n;
-        if (valid) rc = batch.pick(r);
-        // inputs: one-blob rows (two non-zero bins per feature)
+        const GuideRecord rc = valid ? batch.load(r) : GuideRecord{};
+        // inputs: one-blob rows (zero for the padding rows of the last tile: no column is near -1)
         unsigned char *xRow = reinterpret_cast<unsigned char *>(sm.x);
+        if (half == 0) {
 #pragma unroll
-        for (int c = 0; c < GUIDE_INPUTS / 8; c++)
-            *reinterpret_cast<uint4 *>(xRow + canonOffset(row, 8 * c, GUIDE_INPUTS)) = make_uint4(0u, 0u, 0u, 0u);
-        if (valid) {
-#pragma unroll
-            for (int feature = 0; feature < 7; feature++) {
-                const int bins = feature < 3 ? 32 : 16;
-                const int firstCol = feature < 3 ? 32 * feature : 96 + 16 * (feature - 3);
-                const float v = rc.features[feature];
-                const int b = (int)floorf(v * (float)bins - 0.5f);
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const int bin = b + k;
-                    if (bin >= 0 && bin < bins)
-                        *reinterpret_cast<uint16_t *>(xRow + canonOffset(row, firstCol + bin, GUIDE_INPUTS)) =
-                            cvtBf16(oneBlob(v, bins, bin));
-                }
-            }
-        }
-        // forward: every layer's input rows stay for the backward pass
-        trPublish();
-        if (threadIdx.x == 0)
-            trMma(tmem, kMajor(sm.x, GUIDE_INPUTS), kMajor(sm.w0, GUIDE_INPUTS), GUIDE_INPUTS, GUIDE_HIDDEN, false);
-        if (!(ok = trCommitWait(sm, phase))) break;
-        const uint64_t m0 = trHiddenEpilogue(taddr, sm.b, sm.h[0], row);
-        trPublish();
-        if (threadIdx.x == 0)
-            trMma(tmem, kMajor(sm.h[0], GUIDE_HIDDEN), kMajor(sm.w1, GUIDE_HIDDEN), GUIDE_HIDDEN, GUIDE_HIDDEN, false);
-        if (!(ok = trCommitWait(sm, phase))) break;
-        const uint64_t m1 = trHiddenEpilogue(taddr, sm.b + GUIDE_HIDDEN, sm.h[1], row);
-        trPublish();
-        if (threadIdx.x == 0)
-            trMma(tmem, kMajor(sm.h[1], GUIDE_HIDDEN), kMajor(sm.w2, GUIDE_HIDDEN), GUIDE_HIDDEN, GUIDE_HIDDEN, false);
-        if (!(ok = trCommitWait(sm, phase))) break;
-        const uint64_t m2 = trHiddenEpilogue(taddr, sm.b + 2 * GUIDE_HIDDEN, sm.h[2], row);
-        trPublish();
-        if (threadIdx.x == 0)
-            trMma(tmem, kMajor(sm.h[2], GUIDE_HIDDEN), kMajor(sm.w3, GUIDE_HIDDEN), GUIDE_HIDDEN, GUIDE_OUTPUTS, false);
-        if (!(ok = trCommitWait(sm, phase))) break;
-        float o[GUIDE_OUTPUTS];
-        tmemLd32(taddr, o);
-        tmemLd16(taddr + 32u, o + 32);
-        tmemLdWait();
-        const float2 *b4 = reinterpret_cast<const float2 *>(sm.b + 3 * GUIDE_HIDDEN);
-#pragma unroll
-        for (int c = 0; c < GUIDE_OUTPUTS / 2; c++) addBias2(o[2 * c], o[2 * c + 1], b4[c]);
-        // loss gradient of the record (zero for the padding rows of the last tile)
-        uint16_t d3[GUIDE_OUTPUTS];
-        if (valid) {
-            const float y = fminf(rc.y * invMeanY, 100.0f);
-            lossSum += lossGradient(o, make_float3(rc.dir[0], rc.dir[1], rc.dir[2]), rc.pdfBsdf, y, scale, d3);
+            for (int k = 0; k < 3; k++) oneBlobColumns<32>(xRow, row, 32 * k, valid ? rc.features[k] : -1.0f);
         } else {
 #pragma unroll
-            for (int c = 0; c < GUIDE_OUTPUTS; c++) d3[c] = 0;
+            for (int k = 0; k < 4; k++) oneBlobColumns<16>(xRow, row, 96 + 16 * k, valid ? rc.features[3 + k] : -1.0f);
         }
-        {  // delta_3 rows (48 wide) into d[0], and its bias gradient
+        if (!waited) {
+            gridDependencyWait();  // the previous Adam step's weights
+            waited = true;
+            // the weights, already in their shared-memory layout, arrive by one bulk copy (phase 0 of the
+            // mbarrier; the MMA commits follow on phase 1, 0, ...)
+            if (threadIdx.x == 0) {
+                const uint32_t mbar = smemU32(&sm.mbar);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(kImageBytes)
+                             : "memory");
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                                 smemU32(sm.w0)),
+                             "l"(net.image), "r"(kImageBytes), "r"(mbar)
+                             : "memory");
+            }
+            for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) {
+                const int l = min(i / GUIDE_HIDDEN, 3);
+                sm.b[i] = __ldg(&net.b[l][i - l * GUIDE_HIDDEN]);
+            }
+            const float sum = __ldcg(sumY);
+            invMeanY = sum > 0.0f ? (float)n / sum : 0.0f;
+            trWait(sm, phase, failed);
+        }
+        // forward: every layer's input rows stay for the backward pass.  The loops over the layers stay
+        // rolled: a CTA runs this code once per Adam step, so a layer after the first finds it cached.
+        uint32_t mask[3] = {0u, 0u, 0u};
+        float o[GUIDE_OUTPUTS];
+#pragma unroll 1
+        for (int l = 0; l < 4; l++) {
+            if (!trPublish(failed)) goto stop;
+            if (threadIdx.x == 0) {
+                const int width = l == 0 ? GUIDE_INPUTS : GUIDE_HIDDEN;
+                trMma(tmem, kMajor(l == 0 ? sm.x : sm.h[l - 1], width), kMajor(weights(l), width), width,
+                      l == 3 ? GUIDE_OUTPUTS : GUIDE_HIDDEN, false);
+                ummaCommit(smemU32(&sm.mbar));
+            }
+            trWait(sm, phase, failed);
+            if (l == 3) break;
+            const uint32_t m = trHiddenEpilogue(taddr, sm.b + GUIDE_HIDDEN * l, sm.h[l], row, 32 * half);
+            mask[0] = l == 0 ? m : mask[0];
+            mask[1] = l == 1 ? m : mask[1];
+            mask[2] = m;
+        }
+        float v[32];
+        uint16_t d3[GUIDE_OUTPUTS];
+        if (half == 0) {
+            tmemLd32(taddr, o);
+            tmemLd16(taddr + 32u, o + 32);
+            tmemLdWait();
+            const float2 *b4 = reinterpret_cast<const float2 *>(sm.b + 3 * GUIDE_HIDDEN);
+#pragma unroll
+            for (int c = 0; c < GUIDE_OUTPUTS / 2; c++) addBias2(o[2 * c], o[2 * c + 1], b4[c]);
+            // loss gradient of the record (zero for the padding rows of the last tile)
+            if (valid) {
+                const float y = fminf(rc.y * invMeanY, 100.0f);
+                lossSum += lossGradient(o, make_float3(rc.dir[0], rc.dir[1], rc.dir[2]), rc.pdfBsdf, y, scale, d3);
+            } else {
+#pragma unroll
+                for (int c = 0; c < GUIDE_OUTPUTS; c++) d3[c] = 0;
+            }
+            // delta_3 rows (48 wide) into d[0]
             unsigned char *dRow = reinterpret_cast<unsigned char *>(sm.d[0]);
 #pragma unroll
             for (int c = 0; c < GUIDE_OUTPUTS; c += 8)
                 *reinterpret_cast<uint4 *>(dRow + canonOffset(row, c, GUIDE_OUTPUTS)) =
                     make_uint4(pack2(d3[c], d3[c + 1]), pack2(d3[c + 2], d3[c + 3]), pack2(d3[c + 4], d3[c + 5]),
                                pack2(d3[c + 6], d3[c + 7]));
-            float v[32];
+        }
+        // backward, layer 3 to 0: dW_l, and for l > 0 delta_(l-1).  The weight gradients read delta and
+        // activation rows MN-major (K = the records), delta . W_l reads the forward W_l MN-major (as W_l^T).
+        // A layer's bias gradient (column sums) is taken while its MMAs run.
+#pragma unroll 1
+        for (int l = 3; l >= 0; l--) {
+            uint16_t *d = sm.d[(3 - l) & 1];
+            if (l < 3) trDeltaEpilogue(taddr, l == 2 ? mask[2] : l == 1 ? mask[1] : mask[0], d, row, 32 * half, v);
+            if (!trPublish(failed)) goto stop;
+            if (threadIdx.x == 0) {
+                const int outs = l == 3 ? GUIDE_OUTPUTS : GUIDE_HIDDEN, width = l == 0 ? GUIDE_INPUTS : GUIDE_HIDDEN;
+                trMma(tmem + trColDw(l), mnMajor(d, outs), mnMajor(l == 0 ? sm.x : sm.h[l - 1], width), kTrRows, width,
+                      !first);
+                if (l > 0) trMma(tmem, kMajor(d, outs), mnMajor(weights(l), GUIDE_HIDDEN), outs, GUIDE_HIDDEN, false);
+                ummaCommit(smemU32(&sm.mbar));
+            }
+            __syncwarp();
+            if (l < 3) {
+                addBiasGrad(sm.db + GUIDE_HIDDEN * l, 32 * half, v, lane);
+            } else if (half == 0) {
 #pragma unroll
-            for (int c = 0; c < 32; c++) v[c] = fromBf16(d3[c]);
-            addBiasGrad(sm.db + 3 * GUIDE_HIDDEN, 0, v, lane);
+                for (int c = 0; c < 32; c++) v[c] = fromBf16(d3[c]);
+                addBiasGrad(sm.db + 3 * GUIDE_HIDDEN, 0, v, lane);
 #pragma unroll
-            for (int c = 0; c < 32; c++) v[c] = c < GUIDE_OUTPUTS - 32 ? fromBf16(d3[32 + c]) : 0.0f;
-            const float sum = warpColumnSums(v, lane);
-            if (lane < GUIDE_OUTPUTS - 32) atomicAdd(&sm.db[3 * GUIDE_HIDDEN + 32 + lane], sum);
+                for (int c = 0; c < 32; c++) v[c] = c < GUIDE_OUTPUTS - 32 ? fromBf16(d3[32 + c]) : 0.0f;
+                const float sum = warpColumnSums(v, lane);
+                if (lane < GUIDE_OUTPUTS - 32) atomicAdd(&sm.db[3 * GUIDE_HIDDEN + 32 + lane], sum);
+            }
+            trWait(sm, phase, failed);
         }
-        // backward: layer 3 (dW3, delta2), 2 (dW2, delta1), 1 (dW1, delta0), 0 (dW0); the weight
-        // gradients read delta and activation rows MN-major (K = the records), delta . W_l reads
-        // the forward W_l MN-major (as W_l^T)
-        trPublish();
-        if (threadIdx.x == 0) {
-            trMma(tmem + trColDw(3), mnMajor(sm.d[0], GUIDE_OUTPUTS), mnMajor(sm.h[2], GUIDE_HIDDEN), kTrThreads,
-                  GUIDE_HIDDEN, !first);
-            trMma(tmem, kMajor(sm.d[0], GUIDE_OUTPUTS), mnMajor(sm.w3, GUIDE_HIDDEN), GUIDE_OUTPUTS, GUIDE_HIDDEN,
-                  false);
-        }
-        if (!(ok = trCommitWait(sm, phase))) break;
-        trDeltaEpilogue(taddr, m2, sm.d[1], sm.db + 2 * GUIDE_HIDDEN, row, lane);
-        trPublish();
-        if (threadIdx.x == 0) {
-            trMma(tmem + trColDw(2), mnMajor(sm.d[1], GUIDE_HIDDEN), mnMajor(sm.h[1], GUIDE_HIDDEN), kTrThreads,
-                  GUIDE_HIDDEN, !first);
-            trMma(tmem, kMajor(sm.d[1], GUIDE_HIDDEN), mnMajor(sm.w2, GUIDE_HIDDEN), GUIDE_HIDDEN, GUIDE_HIDDEN,
-                  false);
-        }
-        if (!(ok = trCommitWait(sm, phase))) break;
-        trDeltaEpilogue(taddr, m1, sm.d[0], sm.db + GUIDE_HIDDEN, row, lane);
-        trPublish();
-        if (threadIdx.x == 0) {
-            trMma(tmem + trColDw(1), mnMajor(sm.d[0], GUIDE_HIDDEN), mnMajor(sm.h[0], GUIDE_HIDDEN), kTrThreads,
-                  GUIDE_HIDDEN, !first);
-            trMma(tmem, kMajor(sm.d[0], GUIDE_HIDDEN), mnMajor(sm.w1, GUIDE_HIDDEN), GUIDE_HIDDEN, GUIDE_HIDDEN,
-                  false);
-        }
-        if (!(ok = trCommitWait(sm, phase))) break;
-        trDeltaEpilogue(taddr, m0, sm.d[1], sm.db, row, lane);
-        trPublish();
-        if (threadIdx.x == 0)
-            trMma(tmem + trColDw(0), mnMajor(sm.d[1], GUIDE_HIDDEN), mnMajor(sm.x, GUIDE_INPUTS), kTrThreads,
-                  GUIDE_INPUTS, !first);
-        if (!(ok = trCommitWait(sm, phase))) break;
         first = false;
     }
+stop:
+    if (!waited) gridDependencyWait();
+    const bool ok = !__syncthreads_or(failed);  // and no MMA reads the staging area below any more
     gridDependentsMayLaunch();  // the Adam step's blocks may be scheduled (they wait for this grid's gradient)
     // the CTA's gradient: weights from tensor memory (lanes = output features), biases from shared memory.
     // A warp's 32 rows x 32 columns go through shared memory (the input rows, free once the last MMA has
@@ -944,11 +917,12 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
     // 128-byte row pieces per store instruction instead of 32 scattered 16-byte pieces.
     float *part = net.partials + (size_t)blockIdx.x * GUIDE_PARAMS;
     const bool have = ok && !first;
-    if (warp < 2) {
-        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+    const int quarter = warp & 3;  // of the tensor memory's lanes
+    if (quarter < 2) {
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
         constexpr int kPitch = 36;  // floats per staged row
-        static_assert(2 * 32 * kPitch * sizeof(float) <= sizeof(TrainSmem::x), "gradient staging fits the input rows");
-        float *stage = reinterpret_cast<float *>(sm.x) + warp * 32 * kPitch;
+        static_assert(kTrThreads / 64 * 2 * 32 * kPitch * sizeof(float) <= sizeof(TrainSmem::x), "gradient staging fits the input rows");
+        float *stage = reinterpret_cast<float *>(sm.x) + (2 * half + quarter) * 32 * kPitch;
         // the 11 blocks of 32 columns: layer 0 (160 inputs) five, layers 1-3 two each
         auto layerOf = [](int q) { return q < 5 ? 0 : 1 + (q - 5) / 2; };
         auto colOf = [](int q) { return q < 5 ? 32 * q : 32 * ((q - 5) & 1); };
@@ -971,7 +945,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 const int r = 4 * k + (lane >> 3), c = 4 * (lane & 7);
-                const int o = warp * 32 + r;  // output feature
+                const int o = quarter * 32 + r;  // output feature
                 if (o < outs)
                     *reinterpret_cast<float4 *>(part + net.wOffset[l] + o * width + c0 + c) =
                         *reinterpret_cast<const float4 *>(stage + r * kPitch + c);
@@ -979,17 +953,17 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
             __syncwarp();
         };
         // the next block's tensor-memory load is in flight while this one is stored
-        constexpr int kBlocks = 11;
+        const int begin = half ? 6 : 0, end = half ? 11 : 6;
         float va[32], vb[32];
-        load(0, va);
+        load(begin, va);
         tmemLdWaitFor(va);
 #pragma unroll 1
-        for (int q = 0; q < kBlocks; q += 2) {
-            if (q + 1 < kBlocks) load(q + 1, vb);
+        for (int q = begin; q < end; q += 2) {
+            if (q + 1 < end) load(q + 1, vb);
             store(q, va);
             tmemLdWaitFor(vb);
-            if (q + 2 < kBlocks) load(q + 2, va);
-            if (q + 1 < kBlocks) store(q + 1, vb);
+            if (q + 2 < end) load(q + 2, va);
+            if (q + 1 < end) store(q + 1, vb);
             tmemLdWaitFor(va);
         }
     }
@@ -999,14 +973,14 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
         part[net.bOffset[l] + i - l * GUIDE_HIDDEN] = have ? sm.db[i] : 0.0f;
     }
     for (int off = 16; off > 0; off >>= 1) lossSum += __shfl_xor_sync(0xffffffffu, lossSum, off);
-    if (lane == 0) sm.reduce[warp] = lossSum;
+    if (lane == 0 && half == 0) sm.reduce[warp] = lossSum;
     __syncthreads();
     if (threadIdx.x == 0)
         net.partials[GUIDE_PARTIAL_LOSS + blockIdx.x] =
             ok ? (sm.reduce[0] + sm.reduce[1] + sm.reduce[2] + sm.reduce[3]) * scale : 0.0f;
     if (!ok && threadIdx.x == 0 && errors) atomicOr(errors, ERR_GUIDE_TIMEOUT);
     // teardown: a last bounded wait for work in flight after an expired wait, then free tensor memory
-    if (!ok) mbarWait(smemU32(&sm.mbar), phase);
+    if (failed) mbarWait(smemU32(&sm.mbar), phase);
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
@@ -1111,32 +1085,54 @@ __device__ __forceinline__ void storeBf16Weight(const GuideNetView &net, int i, 
 
 static_assert(GUIDE_INPUTS == 5 * 32 && GUIDE_HIDDEN == 2 * 32 && GUIDE_OUTPUTS <= GUIDE_HIDDEN,
               "the gradient write-out walks 5 + 2 + 2 + 2 blocks of 32 columns");
-constexpr int kAdamSplit = 8;  // a power of two, at most 32 (one warp's lanes)
+constexpr int kAdamSplit = 8, kAdamParams = 32;  // warps and parameters of a block
 // Adam step on every parameter; refreshes the bf16 weight copies and clears
-// the gradient.  kAdamSplit threads per parameter (neighbouring lanes) each
-// sum every kAdamSplit-th of the blocks' gradient slots, so a thread waits
-// on a fraction of the loads.
-__global__ void k_guide_adam(GuideNetView net, int blocks, float lr, float beta1, float beta2, float eps, float corr1,
-                             float corr2, float *lossOut) {
+// the gradient.  A block takes kAdamParams parameters: warp w sums every
+// kAdamSplit-th of the training blocks' gradient slots from slot w on (a
+// thread per parameter, so that a slot's values arrive as whole lines), the
+// first warp the kAdamSplit sums.  What the step before left (moments, master
+// weights) is loaded ahead of the wait for the training kernel.
+__global__ void __launch_bounds__(kAdamSplit * 32) k_guide_adam(GuideNetView net, int blocks, float lr, float beta1,
+                                                                float beta2, float eps, float corr1, float corr2,
+                                                                float *lossOut) {
+    __shared__ float sums[kAdamSplit][kAdamParams];
+    const int part = threadIdx.x >> 5, i = blockIdx.x * kAdamParams + (threadIdx.x & 31);
+    const bool mine = part == 0 && i < GUIDE_PARAMS;
+    float m0 = 0.0f, v0 = 0.0f, w0 = 0.0f, g0 = 0.0f;
+    if (mine) {
+        m0 = __ldcg(&net.adamM[i]);
+        v0 = __ldcg(&net.adamV[i]);
+        w0 = __ldcg(&net.master[i]);
+        g0 = __ldcg(&net.grad[i]);
+    }
     gridDependencyWait();  // the training blocks' gradient slots (launched overlapped with them)
     gridDependentsMayLaunch();
-    sumLoss(net, blocks, lossOut);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / kAdamSplit, part = t % kAdamSplit;
     float gr = 0.0f;
-    if (i < GUIDE_PARAMS)
-        for (int b = part; b < blocks; b += kAdamSplit) gr += net.partials[(size_t)b * GUIDE_PARAMS + i];
-    for (int off = 1; off < kAdamSplit; off <<= 1) gr += __shfl_xor_sync(0xffffffffu, gr, off);
-    if (i >= GUIDE_PARAMS || part != 0) return;
-    gr += net.grad[i];
-    const float m = beta1 * net.adamM[i] + (1.0f - beta1) * gr;
-    const float v = beta2 * net.adamV[i] + (1.0f - beta2) * gr * gr;
+    if (i < GUIDE_PARAMS) {
+#pragma unroll 8
+        for (int b = part; b < blocks; b += kAdamSplit) gr += __ldcg(&net.partials[(size_t)b * GUIDE_PARAMS + i]);
+    }
+    sums[part][threadIdx.x & 31] = gr;
+    __syncthreads();
+    if (!mine) return;
+    float t[kAdamSplit];
+#pragma unroll
+    for (int k = 0; k < kAdamSplit; k++) t[k] = sums[k][threadIdx.x & 31];
+#pragma unroll
+    for (int n = kAdamSplit / 2; n > 0; n >>= 1) {
+#pragma unroll
+        for (int k = 0; k < n; k++) t[k] = t[2 * k] + t[2 * k + 1];
+    }
+    gr = t[0] + g0;
+    const float m = beta1 * m0 + (1.0f - beta1) * gr;
+    const float v = beta2 * v0 + (1.0f - beta2) * gr * gr;
     net.adamM[i] = m;
     net.adamV[i] = v;
-    const float w = net.master[i] - lr * (m * corr1) / (sqrtf(v * corr2) + eps);
+    const float w = w0 - lr * (m * corr1) / (sqrtf(v * corr2) + eps);
     net.master[i] = w;
     net.grad[i] = 0.0f;
     storeBf16Weight(net, i, w);
+    sumLoss(net, blocks, lossOut);
 }
 
 // Test hook: forward pass of explicit feature vectors through the inference
@@ -1254,7 +1250,7 @@ cudaError_t rmdLaunchGuideTrain(const GuideRecord *rec, uint32_t total, uint32_t
     if (total == 0) return cudaSuccess;
     RecordBatch batch{rec, total, std::min(n, total), seed};
     // one CTA per tile of 128 records, at most `blocks` (each CTA then takes several tiles)
-    const int tiles = (int)((batch.n + kTrThreads - 1) / kTrThreads);
+    const int tiles = (int)((batch.n + kTrRows - 1) / kTrRows);
     blocks = std::max(1, std::min(std::min(blocks, tiles), GUIDE_TRAIN_MAX_BLOCKS));
     cudaError_t e = cudaSuccess;
     for (uint32_t k = 0; k < steps; k++) {
@@ -1272,7 +1268,7 @@ cudaError_t rmdLaunchGuideTrain(const GuideRecord *rec, uint32_t total, uint32_t
             return e;
         float corr1, corr2;
         adamCorrections(step + (int)k, corr1, corr2);
-        if ((e = launchOverlapped(k_guide_adam, dim3((kAdamSplit * GUIDE_PARAMS + 255) / 256), dim3(256), 0, s, net,
+        if ((e = launchOverlapped(k_guide_adam, dim3((GUIDE_PARAMS + kAdamParams - 1) / kAdamParams), dim3(kAdamSplit * 32), 0, s, net,
                                   blocks, lr, kAdamBeta1, kAdamBeta2, 1e-8f, corr1, corr2, scratch + 1)) != cudaSuccess)
             return e;
     }
@@ -1283,7 +1279,7 @@ cudaError_t rmdLaunchGuideAdam(const GuideNetView &net, int blocks, float lr, in
                                cudaStream_t s) {
     float corr1, corr2;
     adamCorrections(step, corr1, corr2);
-    k_guide_adam<<<(kAdamSplit * GUIDE_PARAMS + 255) / 256, 256, 0, s>>>(net, blocks, lr, kAdamBeta1, kAdamBeta2, 1e-8f,
+    k_guide_adam<<<(GUIDE_PARAMS + kAdamParams - 1) / kAdamParams, kAdamSplit * 32, 0, s>>>(net, blocks, lr, kAdamBeta1, kAdamBeta2, 1e-8f,
                                                                          corr1, corr2, lossOut);
     return cudaGetLastError();
 }
@@ -1304,7 +1300,7 @@ cudaError_t rmdLaunchGuideGradientTest(const GuideRecord *rec, uint32_t n, const
     RecordBatch batch{rec, n, n, 0};
     k_guide_sum_y<<<1, kSumThreads, 0, s>>>(batch, scratch);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int tiles = (int)((n + kTrThreads - 1) / kTrThreads);
+    const int tiles = (int)((n + kTrRows - 1) / kTrRows);
     blocks = std::max(1, std::min(std::min(blocks, tiles), GUIDE_TRAIN_MAX_BLOCKS));
     k_guide_train_tc<<<blocks, kTrThreads, rmdGuideSharedBytes(true), s>>>(batch, scratch, net,
                                                                            reinterpret_cast<uint32_t *>(scratch + 2));
