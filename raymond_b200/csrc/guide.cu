@@ -566,14 +566,15 @@ __device__ __forceinline__ bool tcForward(TcSmem &sm, int pipe, const GuideFeatu
 }
 
 // ------------------------------------------------- tcgen05 training core
-// Training on the 5th-generation tensor cores.  A CTA of 128 threads takes
-// tiles of 128 records, one thread per record (M = 128).  Per tile:
+// Training on the 5th-generation tensor cores.  A CTA takes tiles of 128
+// records (M = 128), two threads per record.  Per tile:
 //
 //   forward   4 layers as in inference (A = the previous layer's rows, B = W);
 //             every layer's input rows stay in shared memory for the
-//             backward pass, and every thread keeps its record's ReLU masks
-//   loss      each thread the gradient of its record's loss with respect to
-//             the 48 raw outputs (CUDA cores), as delta rows
+//             backward pass, and every thread keeps the ReLU masks of its
+//             half of its record's columns
+//   loss      the gradient of each record's loss with respect to the 48 raw
+//             outputs (CUDA cores, one thread per record), as delta rows
 //   backward  per layer l = 3..0: dW_l += delta_l^T . a_(l-1), contracting
 //             the 128 records, accumulated in tensor memory over the CTA's
 //             tiles; and delta_(l-1) = (delta_l . W_l) masked by ReLU',
@@ -592,9 +593,19 @@ __device__ __forceinline__ bool tcForward(TcSmem &sm, int pipe, const GuideFeatu
 // buffer, then the input rows) and land in tensor-memory lanes that are
 // never read.  Tensor memory: columns 0..63 the layer accumulator, then dW0
 // (160), dW1, dW2, dW3 (64 each).  Bias gradients (column sums of the
-// deltas) are reduced across each warp with shuffles into shared memory.  At
-// the end warps 0 and 1 (lanes 0..63, the output features) read the CTA's
-// weight gradient out of tensor memory into the CTA's slot of net.partials.
+// deltas) are reduced across each warp with shuffles into shared memory while
+// the layer's MMAs run.  At the end the four warps of lanes 0..63 (the output
+// features) read the CTA's weight gradient out of tensor memory into the CTA's
+// slot of net.partials.
+//
+// A step is the serial chain of one tile on 64 SMs, then the sum of the 64
+// slots.  Per Adam step (2^13 records, both kernels) on the 640 x 360 room:
+// 25.8 us with one thread per record, set-up after the wait for the previous
+// step, two barriers per layer, the gradient staged and written row by row by
+// two warps, and the slots read 16 bytes at a time; 20.3 us now.  Of it the
+// weights take 0.7 us, the forward layers 3.2, the loss 2.0, the backward
+// layers 4.4, the write-out 2.2 and the Adam kernel about 2.2; the rest is the
+// two kernels' hand-over.
 constexpr int kTrRows = 128;                // records of a tile (M of the forward layers)
 constexpr int kTrThreads = 2 * kTrRows;     // two threads per record, each one half of a layer's columns
 constexpr uint32_t kTrTmemCols = 512;
@@ -619,6 +630,14 @@ static_assert(sizeof(TrainSmem) <= 232448, "training shared memory exceeds the p
 static_assert(GUIDE_PARAMS % 4 == 0 && (GUIDE_HIDDEN * GUIDE_INPUTS + GUIDE_HIDDEN) % 4 == 0 &&
                   (GUIDE_HIDDEN * GUIDE_HIDDEN + GUIDE_HIDDEN) % 4 == 0,
               "a CTA's gradient slot and its layers start on 16-byte boundaries");
+// width (inputs) and outputs of layer l, and where the gradient of its weight
+// (output o, input c) lies in a training CTA's slot: outputs contiguous, as the
+// CTA's lanes hold them (biases lie where they do among the parameters)
+__host__ __device__ constexpr int layerWidth(int l) { return l == 0 ? GUIDE_INPUTS : GUIDE_HIDDEN; }
+__host__ __device__ constexpr int layerOutputs(int l) { return l == 3 ? GUIDE_OUTPUTS : GUIDE_HIDDEN; }
+__device__ __forceinline__ int slotIndex(const GuideNetView &net, int l, int o, int c) {
+    return net.wOffset[l] + c * layerOutputs(l) + o;
+}
 // the weight image (GuideNetView::image) is TrainSmem's leading weight region
 constexpr uint32_t kImageBytes = (uint32_t)offsetof(TrainSmem, d);
 static_assert(offsetof(TrainSmem, w0) == 0 && kImageBytes % 16 == 0 &&
@@ -911,18 +930,14 @@ stop:
     if (!waited) gridDependencyWait();
     const bool ok = !__syncthreads_or(failed);  // and no MMA reads the staging area below any more
     gridDependentsMayLaunch();  // the Adam step's blocks may be scheduled (they wait for this grid's gradient)
-    // the CTA's gradient: weights from tensor memory (lanes = output features), biases from shared memory.
-    // A warp's 32 rows x 32 columns go through shared memory (the input rows, free once the last MMA has
-    // read them; rows padded to 36 floats, so neither side meets a bank conflict) and leave as four
-    // 128-byte row pieces per store instruction instead of 32 scattered 16-byte pieces.
+    // the CTA's gradient into its slot: a lane of tensor memory is an output feature, so each column leaves
+    // as a warp's consecutive values
     float *part = net.partials + (size_t)blockIdx.x * GUIDE_PARAMS;
     const bool have = ok && !first;
     const int quarter = warp & 3;  // of the tensor memory's lanes
     if (quarter < 2) {
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-        constexpr int kPitch = 36;  // floats per staged row
-        static_assert(kTrThreads / 64 * 2 * 32 * kPitch * sizeof(float) <= sizeof(TrainSmem::x), "gradient staging fits the input rows");
-        float *stage = reinterpret_cast<float *>(sm.x) + (2 * half + quarter) * 32 * kPitch;
+        const int o = 32 * quarter + lane;
         // the 11 blocks of 32 columns: layer 0 (160 inputs) five, layers 1-3 two each
         auto layerOf = [](int q) { return q < 5 ? 0 : 1 + (q - 5) / 2; };
         auto colOf = [](int q) { return q < 5 ? 32 * q : 32 * ((q - 5) & 1); };
@@ -935,22 +950,11 @@ stop:
             }
         };
         auto store = [&](int q, const float *v) {
-            const int l = layerOf(q), c0 = colOf(q);
-            const int width = l == 0 ? GUIDE_INPUTS : GUIDE_HIDDEN, outs = l == 3 ? GUIDE_OUTPUTS : GUIDE_HIDDEN;
-            float4 *mine = reinterpret_cast<float4 *>(stage + lane * kPitch);
+            const int l = layerOf(q);
+            if (o >= layerOutputs(l)) return;
+            float *to = part + slotIndex(net, l, o, colOf(q));
 #pragma unroll
-            for (int c = 0; c < 32; c += 4) mine[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-            __syncwarp();
-            // 16-byte pieces: every layer offset, row width and column block is a multiple of 4 floats
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int r = 4 * k + (lane >> 3), c = 4 * (lane & 7);
-                const int o = quarter * 32 + r;  // output feature
-                if (o < outs)
-                    *reinterpret_cast<float4 *>(part + net.wOffset[l] + o * width + c0 + c) =
-                        *reinterpret_cast<const float4 *>(stage + r * kPitch + c);
-            }
-            __syncwarp();
+            for (int c = 0; c < 32; c++) to[c * layerOutputs(l)] = v[c];
         };
         // the next block's tensor-memory load is in flight while this one is stored
         const int begin = half ? 6 : 0, end = half ? 11 : 6;
@@ -961,17 +965,17 @@ stop:
         for (int q = begin; q < end; q += 2) {
             if (q + 1 < end) load(q + 1, vb);
             store(q, va);
+            __syncwarp();
             tmemLdWaitFor(vb);
             if (q + 2 < end) load(q + 2, va);
             if (q + 1 < end) store(q + 1, vb);
+            __syncwarp();
             tmemLdWaitFor(va);
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) {
-        const int l = min(i / GUIDE_HIDDEN, 3);
-        part[net.bOffset[l] + i - l * GUIDE_HIDDEN] = have ? sm.db[i] : 0.0f;
-    }
+    if (threadIdx.x < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS)
+        part[net.bOffset[threadIdx.x / GUIDE_HIDDEN] + threadIdx.x % GUIDE_HIDDEN] = have ? sm.db[threadIdx.x] : 0.0f;
     for (int off = 16; off > 0; off >>= 1) lossSum += __shfl_xor_sync(0xffffffffu, lossSum, off);
     if (lane == 0 && half == 0) sm.reduce[warp] = lossSum;
     __syncthreads();
@@ -1070,8 +1074,13 @@ __global__ void k_guide_reduce(GuideNetView net, int blocks, float *lossOut) {
     sumLoss(net, blocks, lossOut);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= GUIDE_PARAMS) return;
+    int slot = i;
+    for (int l = 0; l < 4; l++) {
+        const int k = i - net.wOffset[l], width = layerWidth(l);
+        if (k >= 0 && k < layerOutputs(l) * width) slot = slotIndex(net, l, k / width, k % width);
+    }
     float g = 0.0f;
-    for (int b = 0; b < blocks; b++) g += net.partials[(size_t)b * GUIDE_PARAMS + i];
+    for (int b = 0; b < blocks; b++) g += net.partials[(size_t)b * GUIDE_PARAMS + slot];
     net.grad[i] += g;
 }
 
@@ -1085,19 +1094,34 @@ __device__ __forceinline__ void storeBf16Weight(const GuideNetView &net, int i, 
 
 static_assert(GUIDE_INPUTS == 5 * 32 && GUIDE_HIDDEN == 2 * 32 && GUIDE_OUTPUTS <= GUIDE_HIDDEN,
               "the gradient write-out walks 5 + 2 + 2 + 2 blocks of 32 columns");
-constexpr int kAdamSplit = 8, kAdamParams = 32;  // warps and parameters of a block
 // Adam step on every parameter; refreshes the bf16 weight copies and clears
-// the gradient.  A block takes kAdamParams parameters: warp w sums every
-// kAdamSplit-th of the training blocks' gradient slots from slot w on (a
-// thread per parameter, so that a slot's values arrive as whole lines), the
-// first warp the kAdamSplit sums.  What the step before left (moments, master
-// weights) is loaded ahead of the wait for the training kernel.
-__global__ void __launch_bounds__(kAdamSplit * 32) k_guide_adam(GuideNetView net, int blocks, float lr, float beta1,
-                                                                float beta2, float eps, float corr1, float corr2,
-                                                                float *lossOut) {
-    __shared__ float sums[kAdamSplit][kAdamParams];
-    const int part = threadIdx.x >> 5, i = blockIdx.x * kAdamParams + (threadIdx.x & 31);
-    const bool mine = part == 0 && i < GUIDE_PARAMS;
+// the gradient.  A block takes 32 outputs x 4 inputs of a layer (the last
+// blocks 128 biases each): its warp w sums every kAdamSplit-th of the training
+// CTAs' gradient slots from slot w on, a column of 32 outputs per load, and
+// leaves its sums in shared memory; then a thread per parameter, 4 inputs in a
+// row.  What the step before left is loaded ahead of the wait for the training
+// kernel.  8 inputs make 89 blocks, too few to draw the 5.5 MB of slots from L2
+// (21.8 us per step instead of 20.3); 2 and 4 are equal.
+constexpr int kAdamSplit = 8, kAdamColumns = 4, kAdamThreads = 32 * kAdamSplit;
+constexpr int kAdamTiles0 = 2 * GUIDE_INPUTS / kAdamColumns, kAdamTiles = 2 * GUIDE_HIDDEN / kAdamColumns;
+constexpr int kBiases = 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS;
+constexpr int kAdamBiasTile = kAdamTiles0 + 3 * kAdamTiles;  // the first block of biases
+constexpr int kAdamBlocks = kAdamBiasTile + (kBiases + 32 * kAdamColumns - 1) / (32 * kAdamColumns);
+__global__ void __launch_bounds__(kAdamThreads) k_guide_adam(GuideNetView net, int blocks, float lr, float beta1,
+                                                             float beta2, float eps, float corr1, float corr2,
+                                                             float *lossOut) {
+    __shared__ float sums[kAdamSplit][kAdamColumns][33];
+    const int t = threadIdx.x, part = t >> 5, lane = t & 31, tile = blockIdx.x;
+    const bool bias = tile >= kAdamBiasTile;
+    const int l = tile < kAdamTiles0 ? 0 : 1 + (tile - kAdamTiles0) / kAdamTiles;  // weights only
+    const int k = l == 0 ? tile : (tile - kAdamTiles0) % kAdamTiles;
+    const int o0 = 32 * (k & 1), c0 = kAdamColumns * (k >> 1);
+    auto biasIndex = [&](int j) { return net.bOffset[j / GUIDE_HIDDEN] + j % GUIDE_HIDDEN; };
+    const int j0 = 32 * kAdamColumns * (tile - kAdamBiasTile);
+    // this thread's parameter
+    const int o = o0 + t / kAdamColumns, c = c0 + t % kAdamColumns;
+    const bool mine = t < 32 * kAdamColumns && (bias ? j0 + t < kBiases : o < layerOutputs(l));
+    const int i = !mine ? 0 : bias ? biasIndex(j0 + t) : net.wOffset[l] + o * layerWidth(l) + c;
     float m0 = 0.0f, v0 = 0.0f, w0 = 0.0f, g0 = 0.0f;
     if (mine) {
         m0 = __ldcg(&net.adamM[i]);
@@ -1107,31 +1131,45 @@ __global__ void __launch_bounds__(kAdamSplit * 32) k_guide_adam(GuideNetView net
     }
     gridDependencyWait();  // the training blocks' gradient slots (launched overlapped with them)
     gridDependentsMayLaunch();
-    float gr = 0.0f;
-    if (i < GUIDE_PARAMS) {
+    float s[kAdamColumns];
+    int slot[kAdamColumns];
+#pragma unroll
+    for (int q = 0; q < kAdamColumns; q++) {
+        const int j = j0 + 32 * q + lane;
+        s[q] = 0.0f;
+        slot[q] = bias ? (j < kBiases ? biasIndex(j) : -1)
+                       : (o0 + lane < layerOutputs(l) ? slotIndex(net, l, o0 + lane, c0 + q) : -1);
+    }
 #pragma unroll 8
-        for (int b = part; b < blocks; b += kAdamSplit) gr += __ldcg(&net.partials[(size_t)b * GUIDE_PARAMS + i]);
+    for (int b = part; b < blocks; b += kAdamSplit) {
+        const float *p = net.partials + (size_t)b * GUIDE_PARAMS;
+#pragma unroll
+        for (int q = 0; q < kAdamColumns; q++)
+            if (slot[q] >= 0) s[q] += __ldcg(&p[slot[q]]);
     }
-    sums[part][threadIdx.x & 31] = gr;
+#pragma unroll
+    for (int q = 0; q < kAdamColumns; q++) sums[part][q][lane] = s[q];
     __syncthreads();
-    if (!mine) return;
-    float t[kAdamSplit];
+    if (mine) {
+        const int q = bias ? t >> 5 : t % kAdamColumns, at = bias ? lane : t / kAdamColumns;
+        float a[kAdamSplit];
 #pragma unroll
-    for (int k = 0; k < kAdamSplit; k++) t[k] = sums[k][threadIdx.x & 31];
+        for (int n = 0; n < kAdamSplit; n++) a[n] = sums[n][q][at];
 #pragma unroll
-    for (int n = kAdamSplit / 2; n > 0; n >>= 1) {
+        for (int n = kAdamSplit / 2; n > 0; n >>= 1) {
 #pragma unroll
-        for (int k = 0; k < n; k++) t[k] = t[2 * k] + t[2 * k + 1];
+            for (int h = 0; h < n; h++) a[h] = a[2 * h] + a[2 * h + 1];
+        }
+        const float gr = a[0] + g0;
+        const float m = beta1 * m0 + (1.0f - beta1) * gr;
+        const float v = beta2 * v0 + (1.0f - beta2) * gr * gr;
+        net.adamM[i] = m;
+        net.adamV[i] = v;
+        const float w = w0 - lr * (m * corr1) / (sqrtf(v * corr2) + eps);
+        net.master[i] = w;
+        net.grad[i] = 0.0f;
+        storeBf16Weight(net, i, w);
     }
-    gr = t[0] + g0;
-    const float m = beta1 * m0 + (1.0f - beta1) * gr;
-    const float v = beta2 * v0 + (1.0f - beta2) * gr * gr;
-    net.adamM[i] = m;
-    net.adamV[i] = v;
-    const float w = w0 - lr * (m * corr1) / (sqrtf(v * corr2) + eps);
-    net.master[i] = w;
-    net.grad[i] = 0.0f;
-    storeBf16Weight(net, i, w);
     sumLoss(net, blocks, lossOut);
 }
 
@@ -1268,7 +1306,7 @@ cudaError_t rmdLaunchGuideTrain(const GuideRecord *rec, uint32_t total, uint32_t
             return e;
         float corr1, corr2;
         adamCorrections(step + (int)k, corr1, corr2);
-        if ((e = launchOverlapped(k_guide_adam, dim3((GUIDE_PARAMS + kAdamParams - 1) / kAdamParams), dim3(kAdamSplit * 32), 0, s, net,
+        if ((e = launchOverlapped(k_guide_adam, dim3(kAdamBlocks), dim3(kAdamThreads), 0, s, net,
                                   blocks, lr, kAdamBeta1, kAdamBeta2, 1e-8f, corr1, corr2, scratch + 1)) != cudaSuccess)
             return e;
     }
@@ -1279,7 +1317,7 @@ cudaError_t rmdLaunchGuideAdam(const GuideNetView &net, int blocks, float lr, in
                                cudaStream_t s) {
     float corr1, corr2;
     adamCorrections(step, corr1, corr2);
-    k_guide_adam<<<(GUIDE_PARAMS + kAdamParams - 1) / kAdamParams, kAdamSplit * 32, 0, s>>>(net, blocks, lr, kAdamBeta1, kAdamBeta2, 1e-8f,
+    k_guide_adam<<<kAdamBlocks, kAdamThreads, 0, s>>>(net, blocks, lr, kAdamBeta1, kAdamBeta2, 1e-8f,
                                                                          corr1, corr2, lossOut);
     return cudaGetLastError();
 }
