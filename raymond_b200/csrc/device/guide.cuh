@@ -46,8 +46,10 @@ struct alignas(16) GuideMixture {
     float pad[2];
 };
 constexpr uint32_t GUIDE_MIX_STRIDE = 32;  // 16-byte chunks between two chunks of one mixture
-// a mixture's first chunk: hit `q` in shading order
-RMD_HD size_t guideMixtureAt(uint32_t q) { return (size_t)(q >> 5) * (8u * GUIDE_MIX_STRIDE) + (q & 31u); }
+// a mixture's first chunk, hit `q` in shading order: (q / 32) * 256 + q % 32
+// (2^29 hits, where it would leave 32 bits, are 64 GB of mixtures beside 140 GB
+// of paths)
+RMD_HD uint32_t guideMixtureAt(uint32_t q) { return q + 7u * (q & ~31u); }
 RMD_HD void storeMixture(uint4 *dst, const GuideMixture &m) {
 #pragma unroll
     for (int j = 0; j < GUIDE_LOBES / 2; j++)
