@@ -800,11 +800,13 @@ struct Workspace {
     cudaStream_t stream;
     char *base = nullptr;
     size_t used = 0;
-    explicit Workspace(cudaStream_t s) : stream(s) {}
+    size_t allocated = 0;
+    const rmdhost::DeviceMemory &memory;
+    Workspace(cudaStream_t s, const rmdhost::DeviceMemory &m) : stream(s), memory(m) {}
     ~Workspace() {
         if (!base) return;
         cudaStreamSynchronize(stream);  // after an error its kernels may still run
-        cudaFree(base);
+        memory.free(base, allocated);
     }
     template <class T>
     T *take(size_t count) {  // null while only sizes are counted
@@ -846,14 +848,14 @@ namespace rmdhost {
 using namespace rmd;
 
 cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, const uint32_t *inst,
-                            const uint32_t *prim, uint32_t n, cudaStream_t s, const DeviceAlloc &alloc, GpuBvhResult &out) {
+                            const uint32_t *prim, uint32_t n, cudaStream_t s, const DeviceMemory &memory, GpuBvhResult &out) {
     out = GpuBvhResult();
     if (n == 0) return cudaSuccess;  // no nodes: everything misses
     if (n > kGpuBvhMaxTriangles) {
         out.error = "the device BVH builder takes at most 2^24 triangles";
         return cudaErrorInvalidValue;
     }
-    Workspace S(s);
+    Workspace S(s, memory);
     float4 *triLo, *triHi, *nodeLo, *nodeHi, *clLo[2], *clHi[2];
     int2 *nodeChild;
     uint64_t *keys[2];
@@ -905,9 +907,10 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
         planPos = S.take<uint2>(n);
     };
     carve();
-    BVH_TRY(alloc(reinterpret_cast<void **>(&S.base), S.used));
+    S.allocated = S.used;
+    BVH_TRY(memory.alloc(reinterpret_cast<void **>(&S.base), S.allocated));
     carve();
-    BVH_TRY(alloc(&out.tris, (size_t)n * TRI_FLOAT4 * sizeof(float4)));
+    BVH_TRY(memory.alloc(&out.tris, (size_t)n * TRI_FLOAT4 * sizeof(float4)));
     float4 *tris = static_cast<float4 *>(out.tris);
 
     // 1. boxes and centroid bounds
@@ -990,9 +993,9 @@ cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, c
                     " triangles";
         return cudaErrorInvalidValue;
     }
-    BVH_TRY(alloc(&out.nodes, (size_t)wideCount * sizeof(GpuWideNode)));
-    BVH_TRY(cudaMemcpyAsync(out.nodes, wide, (size_t)wideCount * sizeof(GpuWideNode), cudaMemcpyDeviceToDevice, s));
+    BVH_TRY(memory.alloc(&out.nodes, (size_t)wideCount * sizeof(GpuWideNode)));
     out.nodeCount = wideCount;
+    BVH_TRY(cudaMemcpyAsync(out.nodes, wide, (size_t)wideCount * sizeof(GpuWideNode), cudaMemcpyDeviceToDevice, s));
     out.levels = level;
     return cudaStreamSynchronize(s);
 }

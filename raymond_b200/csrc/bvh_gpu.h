@@ -9,8 +9,11 @@
 
 namespace rmdhost {
 
-// allocates device memory that cudaFree frees
-using DeviceAlloc = std::function<cudaError_t(void **, size_t)>;
+// where the builder's device memory comes from and goes to (free: with the size allocated)
+struct DeviceMemory {
+    std::function<cudaError_t(void **, size_t)> alloc;
+    std::function<void(void *, size_t)> free;
+};
 
 struct GpuBvhResult {
     void *nodes = nullptr;   // nodeCount x 80 B (GpuWideNode), allocated, owned by the caller
@@ -30,6 +33,6 @@ constexpr uint32_t kGpuBvhMaxTriangles = 1u << 24;
 // triangle).  Returns cudaErrorInvalidValue with `error` set when the input
 // is out of range or the tree would be deeper than the traversal stack.
 cudaError_t buildWideBvhGpu(const float *v0, const float *v1, const float *v2, const uint32_t *inst,
-                            const uint32_t *prim, uint32_t n, cudaStream_t s, const DeviceAlloc &alloc, GpuBvhResult &out);
+                            const uint32_t *prim, uint32_t n, cudaStream_t s, const DeviceMemory &memory, GpuBvhResult &out);
 
 }  // namespace rmdhost

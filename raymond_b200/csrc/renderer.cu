@@ -9,6 +9,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -94,50 +95,85 @@ static int defaultShadeMinBlocks() {
 
 // A context's device memory: blocks that its scenes, renderers and batches free
 // stay with it for the next ones, up to kMemoryKept bytes; beyond that, and
-// with the context, they go back to the device.  cudaMalloc and cudaFree of
-// the 10-500 MB blocks that a scene and its renderer take cost 1-10 ms each,
-// and now and then hundreds (the 852 k-triangle scene: 20 ms to 4 s of a
-// creation); a block that the pool holds costs microseconds.  Any thread may
+// with the context and its last object, they go back to the device.  cudaMalloc
+// and cudaFree of the 10-500 MB blocks that a scene and its renderer take cost
+// 1-10 ms each, and now and then hundreds (the 852 k-triangle scene: 20 ms to
+// 4 s of a creation).  A driver pool maps its memory anew whenever a block fits
+// no hole (2-3 ms for the tree's workspace and for the paths, in one of four
+// creations 40-1,200 ms); a kept block is handed out as it is.  Sizes below
+// 1 GiB are rounded up to an eighth of their power of two, so that a scene a
+// little larger than the one before takes the same blocks.  Any thread may
 // allocate and free.
 struct DevPool {
-    static constexpr uint64_t kMemoryKept = 2ull << 30;
-    cudaMemPool_t pool = nullptr;
-    cudaStream_t stream = nullptr;  // orders the allocations alone; waited for by each
-    cudaError_t create(int device) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaError_t e = cudaMemPoolCreate(&pool, &props);
-        uint64_t kept = kMemoryKept;
-        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    static constexpr size_t kMemoryKept = size_t(2) << 30;
+    std::mutex mutex;
+    std::multimap<size_t, void *> kept;  // free blocks by size
+    size_t keptBytes = 0;
+    static size_t rounded(size_t n) {
+        size_t step = 512;
+        if (n < (size_t(1) << 30))
+            while (step * 16 <= n) step *= 2;
+        return (n + step - 1) / step * step;
+    }
+    // a block of the current device, which has to be the context's
+    cudaError_t alloc(void **p, size_t n) {
+        const size_t size = rounded(n);
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            const auto it = kept.find(size);
+            if (it != kept.end()) {
+                *p = it->second;
+                keptBytes -= size;
+                kept.erase(it);
+                return cudaSuccess;
+            }
+        }
+        cudaError_t e = cudaMalloc(p, size);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            giveBack();
+            e = cudaMalloc(p, size);
+        }
         return e;
     }
-    // The block may be used on any stream at once: its allocation has completed.
-    cudaError_t alloc(void **p, size_t n) const {
-        cudaError_t e = cudaMallocFromPoolAsync(p, n, pool, stream);
-        return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+    // takes back a block that alloc gave for n bytes; no work may use it any more
+    void free(void *p, size_t n) {
+        const size_t size = rounded(n);
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            if (keptBytes + size <= kMemoryKept) {
+                kept.emplace(size, p);
+                keptBytes += size;
+                return;
+            }
+        }
+        cudaFree(p);
     }
-    ~DevPool() {  // blocks in use stay valid; the pool goes with the last of them
-        if (stream) cudaStreamDestroy(stream);
-        if (pool) cudaMemPoolDestroy(pool);
+    void giveBack() {
+        std::lock_guard<std::mutex> lock(mutex);
+        for (auto &block : kept) cudaFree(block.second);
+        kept.clear();
+        keptBytes = 0;
     }
+    ~DevPool() { giveBack(); }
 };
 
 // Device buffer owned by a scene, renderer or batch, from its context's pool
-// where one is set.  Whoever frees it has waited for the work that uses it:
-// cudaFree of a pool's block does not.
+// where one is set.  Whoever frees it has waited for the work that uses it: the
+// pool does not.
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
-    const DevPool *from = nullptr;
+    std::shared_ptr<DevPool> from;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }
     void release() {
-        if (ptr) cudaFree(ptr);
+        if (ptr) {
+            if (from) from->free(ptr, bytes);
+            else cudaFree(ptr);
+        }
         ptr = nullptr;
         bytes = 0;
     }
@@ -147,7 +183,7 @@ struct DevBuf {
         if (n == 0) return cudaSuccess;
         return from ? from->alloc(&ptr, n) : cudaMalloc(&ptr, n);
     }
-    void adopt(void *p, size_t n) {  // takes ownership of an allocated block
+    void adopt(void *p, size_t n) {  // takes ownership of a block allocated as alloc(n) does
         release();
         ptr = p;
         bytes = n;
@@ -186,7 +222,7 @@ struct rmd_context {
     int smCount = 148;
     cudaStream_t stream = nullptr;
     uint32_t bvhBuilder = RMD_BVH_HOST;  // builder of the scenes created next
-    DevPool memory;
+    std::shared_ptr<DevPool> memory = std::make_shared<DevPool>();
 };
 
 struct rmd_scene {
@@ -212,11 +248,11 @@ struct rmd_scene {
     int shadeBlocks = 0, traceBlocks = 0, regenBlocks = 0;
     int defaultMinBlocks = 1;
     bool ownsModule = true;  // false for the scenes of a batch (the batch owns the shared module)
-    void takeMemoryFrom(const DevPool &p) {
+    void takeMemoryFrom(const std::shared_ptr<DevPool> &p) {
         for (DevBuf *b : {&vertices, &normals, &texcoords, &faces, &instances, &lightFaces, &envPdfs, &envMipmap, &areaLights,
                           &pointLights, &sunLights, &spotLights, &shapeLights, &surfaceTable, &lightTable, &materialParams,
                           &bvhNodes, &bvhTris, &textureTexels, &textureViews})
-            b->from = &p;
+            b->from = p;
     }
     ~rmd_scene() {
         waitForDevice(device);
@@ -236,8 +272,8 @@ struct GuideState {
     uint32_t recordCapacity = 0;  // nonzero-target records the replay ring holds
     bool initialised = false;
     float3 frameMin = {0, 0, 0}, frameInvExtent = {1, 1, 1};  // position encoding frame (scene bounds)
-    void takeMemoryFrom(const DevPool &p) {
-        for (DevBuf *b : {&mixtures, &features, &rec, &finRec, &shRec, &records}) b->from = &p;
+    void takeMemoryFrom(const std::shared_ptr<DevPool> &p) {
+        for (DevBuf *b : {&mixtures, &features, &rec, &finRec, &shRec, &records}) b->from = p;
     }
 };
 
@@ -473,7 +509,6 @@ rmd_status rmd_context_create(int32_t device, rmd_context **out) {
     c->device = device;
     RMD_CUDA(cudaSetDevice(device));
     RMD_CUDA(cudaDeviceGetAttribute(&c->smCount, cudaDevAttrMultiProcessorCount, device));
-    RMD_CUDA(c->memory.create(device));
     RMD_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     const rmd_status ns = rmdhost::noallocSetup(device);
     if (ns != RMD_OK) {
@@ -660,7 +695,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         if (k % 5 == 4 && sh.num_faces) std::memcpy(hostMat + 2 * f, sh.materials, 2 * (size_t)sh.num_faces);
     }
     DevBuf staged;
-    staged.from = &ctx->memory;
+    staged.from = ctx->memory;
     RMD_CUDA(staged.upload(mesh.get(), meshBytes, st));
     RMD_CUDA(s->vertices.alloc(numVertices * sizeof(float4)));
     RMD_CUDA(s->normals.alloc(numVertices * sizeof(float4)));
@@ -757,7 +792,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     s->bvhStats.builder = ctx->bvhBuilder;
     if (ctx->bvhBuilder == RMD_BVH_GPU) {
         DevBuf world;  // three vertices, instance and primitive per triangle, then the bounds
-        world.from = &ctx->memory;
+        world.from = ctx->memory;
         RMD_CUDA(world.alloc(numTriangles * 44 + 6 * sizeof(uint32_t)));
         float *w0 = world.as<float>(), *w1 = w0 + 3 * numTriangles, *w2 = w1 + 3 * numTriangles;
         uint32_t *wInst = reinterpret_cast<uint32_t *>(w2 + 3 * numTriangles), *wPrim = wInst + numTriangles;
@@ -771,7 +806,8 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         }
         rmdhost::GpuBvhResult g;
         const cudaError_t e = rmdhost::buildWideBvhGpu(
-            w0, w1, w2, wInst, wPrim, n, st, [&](void **p, size_t bytes) { return ctx->memory.alloc(p, bytes); }, g);
+            w0, w1, w2, wInst, wPrim, n, st, {[&](void **p, size_t bytes) { return ctx->memory->alloc(p, bytes); },
+             [&](void *p, size_t bytes) { ctx->memory->free(p, bytes); }}, g);
         s->bvhNodes.adopt(g.nodes, g.nodeCount * sizeof(rmdhost::GpuWideNode));
         s->bvhTris.adopt(g.tris, numTriangles * TRI_FLOAT4 * sizeof(float4));
         if (e != cudaSuccess) {
@@ -895,7 +931,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     }
     if (s->triangles && ctx->bvhBuilder != RMD_BVH_GPU) {  // the traversal kernels read three rotated copies of each triangle (device/traverse.cuh)
         DevBuf rotated;
-        rotated.from = &ctx->memory;
+        rotated.from = ctx->memory;
         RMD_CUDA(rotated.alloc(s->triangles * TRI_FLOAT4 * sizeof(float4)));
         RMD_CUDA(rmdLaunchRotateTriangles(s->bvhTris.as<float4>(), rotated.as<float4>(), (uint32_t)s->triangles, st));
         RMD_CUDA(cudaStreamSynchronize(st));
@@ -1188,7 +1224,7 @@ rmd_status rmd_renderer_create(rmd_scene *scene, uint32_t width, uint32_t height
     auto r = std::make_unique<rmd_renderer>();
     r->scene = scene;
     // not the film, whose address callers get (rmd_film_device)
-    for (DevBuf *b : {&r->pool, &r->counters, &r->resolve, &r->film64}) b->from = &scene->ctx->memory;
+    for (DevBuf *b : {&r->pool, &r->counters, &r->resolve, &r->film64}) b->from = scene->ctx->memory;
     r->device = scene->ctx->device;
     r->guide.takeMemoryFrom(scene->ctx->memory);
     r->dctx = scene->dctx;
@@ -1901,7 +1937,7 @@ rmd_status rmd_batch_create(rmd_context *ctx, const rmd_scene_desc *descs, int32
     RMD_CUDA(cudaSetDevice(ctx->device));
     auto b = std::make_unique<rmd_batch>();
     b->ctx = ctx;
-    for (DevBuf *m : {&b->viewTable, &b->pool, &b->counters, &b->resolve, &b->film, &b->film64}) m->from = &ctx->memory;
+    for (DevBuf *m : {&b->viewTable, &b->pool, &b->counters, &b->resolve, &b->film, &b->film64}) m->from = ctx->memory;
     b->device = ctx->device;
     b->guide.takeMemoryFrom(ctx->memory);
     b->useGraph = !(flags & RMD_BATCH_NO_GRAPH);
