@@ -139,15 +139,15 @@ struct DevPool {
     // takes back a block that alloc gave for n bytes; no work may use it any more
     void free(void *p, size_t n) {
         const size_t size = rounded(n);
-        {
-            std::lock_guard<std::mutex> lock(mutex);
-            if (keptBytes + size <= kMemoryKept) {
-                kept.emplace(size, p);
-                keptBytes += size;
-                return;
-            }
+        std::lock_guard<std::mutex> lock(mutex);
+        kept.emplace(size, p);
+        keptBytes += size;
+        while (keptBytes > kMemoryKept) {  // the largest go first: small ones are asked for on every read-out
+            const auto largest = std::prev(kept.end());
+            cudaFree(largest->second);
+            keptBytes -= largest->first;
+            kept.erase(largest);
         }
-        cudaFree(p);
     }
     void giveBack() {
         std::lock_guard<std::mutex> lock(mutex);
