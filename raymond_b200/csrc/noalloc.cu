@@ -70,10 +70,12 @@ rmd_status noallocSetup(int device) {
     std::lock_guard<std::mutex> lock(g_mutex);
     g_scratch[device] = ptr;
     HostSide &h = g_host[device];
-    if (h.events[0] && cudaEventQuery(h.events[0]) != cudaSuccess) {  // gone with a device reset
-        cudaGetLastError();
+    // Made anew only if they went with a device reset: a call that renders on another thread leaves its event
+    // pending (cudaErrorNotReady), and goes on using these.
+    const cudaError_t alive = h.events[0] ? cudaEventQuery(h.events[0]) : cudaSuccess;
+    if (alive != cudaSuccess) cudaGetLastError();
+    if (alive == cudaErrorInvalidResourceHandle || alive == cudaErrorContextIsDestroyed || alive == cudaErrorDeviceUninitialized)
         h = HostSide();
-    }
     for (cudaEvent_t &ev : h.events)
         if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
             return cudaFail(e, "cudaEventCreate");
@@ -105,13 +107,13 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
     if (e != cudaSuccess) return cudaFail(e, "cudaSetDevice");
 
     void *base;
-    HostSide *host;
+    HostSide host;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         base = g_scratch[v.device];  // set when the scene's context was created
-        host = &g_host[v.device];
+        host = g_host[v.device];
     }
-    if (!base) return rmdhost::setLastError(RMD_ERROR_CUDA, "rmd_render_noalloc: scratch array not set up");
+    if (!base || !host.counters) return rmdhost::setLastError(RMD_ERROR_CUDA, "rmd_render_noalloc: scratch array not set up");
     const uint32_t P = pool_size ? pool_size : kMaxPaths;
     Counters *cnt = static_cast<Counters *>(base);
     const PathPool pool = carvePathPool(static_cast<unsigned char *>(base) + kCountersBytes, P);
@@ -167,7 +169,7 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
             status = rmdhost::setLastError(RMD_ERROR_WATCHDOG, "rmd_render_noalloc: render did not drain");
         return status != RMD_OK || h.pathsDone >= numPaths;
     };
-    e = rmdhost::driveWavefront(cnt, numPaths, P, host->counters, host->events, st, iterate, check);
+    e = rmdhost::driveWavefront(cnt, numPaths, P, host.counters, host.events, st, iterate, check);
     if (e != cudaSuccess) return cudaFail(e, "wavefront");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cudaFail(e, "synchronize");
     if (status != RMD_OK) return status;
