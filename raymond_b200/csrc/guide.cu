@@ -1375,7 +1375,7 @@ void GuideNet::release() {
     imageIndex = nullptr;
 }
 
-cudaError_t GuideNet::allocate() {
+cudaError_t GuideNet::allocate(cudaStream_t s) {
     release();
     const size_t pb = GUIDE_PARAMS * sizeof(float);
     cudaError_t e;
@@ -1402,8 +1402,9 @@ cudaError_t GuideNet::allocate() {
                 idx[p] = qOff[l] + o * in[l] + k;
                 img[p] = (int)((fwd[l] + canonOffset(o, k, in[l])) / sizeof(uint16_t));  // row o, K = inputs
             }
-    if ((e = cudaMemcpy(bf16Index, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(imageIndex, img.data(), img.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess)
+    if ((e = cudaMemcpyAsync(bf16Index, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(imageIndex, img.data(), img.size() * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return e;
     return rmdGuideConfigure();
 }
@@ -1507,7 +1508,7 @@ extern "C" rmd_status rmd_test_guide_forward(const float *params, const float *f
         return rmdhost::setLastError(RMD_ERROR_INVALID_ARGUMENT, "rmd_test_guide_forward: invalid arguments");
     rmdhost::GuideNet net;
     cudaError_t e;
-    if ((e = net.allocate()) != cudaSuccess) return guideFail(e, "guide allocate");
+    if ((e = net.allocate(0)) != cudaSuccess) return guideFail(e, "guide allocate");
     if ((e = net.setParams(params, 0)) != cudaSuccess) return guideFail(e, "guide params");
     DeviceArray f, o, st;
     const int zero = 0;
@@ -1533,7 +1534,7 @@ extern "C" rmd_status rmd_test_guide_gradient(const float *params, const float *
     static_assert(sizeof(GuideRecord) == 12 * sizeof(float), "GuideRecord is 12 floats");
     rmdhost::GuideNet net;
     cudaError_t e;
-    if ((e = net.allocate()) != cudaSuccess) return guideFail(e, "guide allocate");
+    if ((e = net.allocate(0)) != cudaSuccess) return guideFail(e, "guide allocate");
     if ((e = net.setParams(params, 0)) != cudaSuccess) return guideFail(e, "guide params");
     DeviceArray r;
     if ((e = r.upload(records, (size_t)n * sizeof(GuideRecord))) != cudaSuccess) return guideFail(e, "guide records");
@@ -1562,7 +1563,7 @@ extern "C" rmd_status rmd_test_guide_adam(const float *params, const float *grad
     rmdhost::GuideNet net;
     cudaError_t e;
     const size_t pb = GUIDE_PARAMS * sizeof(float);
-    if ((e = net.allocate()) != cudaSuccess) return guideFail(e, "guide allocate");
+    if ((e = net.allocate(0)) != cudaSuccess) return guideFail(e, "guide allocate");
     if ((e = net.setParams(params, 0)) != cudaSuccess) return guideFail(e, "guide params");
     if ((e = cudaMemcpy(net.grad, grad, pb, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(net.adamM, m, pb, cudaMemcpyHostToDevice)) != cudaSuccess ||

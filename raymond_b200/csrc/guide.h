@@ -82,7 +82,7 @@ struct GuideNet {
     ~GuideNet() { release(); }
     void release();
     bool allocated() const { return master != nullptr; }
-    cudaError_t allocate();
+    cudaError_t allocate(cudaStream_t s);  // `s`: the stream that will use it
     // upload FP32 parameters (refreshes the BF16 copy, clears Adam and the gradient)
     cudaError_t setParams(const float *host, cudaStream_t s);
     cudaError_t getParams(float *host, cudaStream_t s) const;

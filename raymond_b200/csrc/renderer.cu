@@ -160,7 +160,9 @@ struct DevPool {
 
 // Device buffer owned by a scene, renderer or batch, from its context's pool
 // where one is set.  Whoever frees it has waited for the work that uses it: the
-// pool does not.
+// pool does not.  A new one may hold what a block's last owner left, so it is
+// cleared and filled on the stream that uses it (the legacy stream is not
+// ordered with a context's).
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
@@ -1055,7 +1057,7 @@ static void guideFrame(const rmd_scene *s, float3 &lo, float3 &invExtent);
 static rmd_status allocatePool(rmd_renderer *r) {
     RMD_CUDA(r->pool.alloc(pathPoolBytes(r->capacity)));
     RMD_CUDA(r->counters.alloc(sizeof(Counters)));
-    RMD_CUDA(cudaMemset(r->counters.ptr, 0, sizeof(Counters)));
+    RMD_CUDA(cudaMemsetAsync(r->counters.ptr, 0, sizeof(Counters), r->scene->ctx->stream));
     return ensureGuideBuffers(r);
 }
 
@@ -1097,7 +1099,7 @@ static void guideFrame(const rmd_scene *s, float3 &lo, float3 &invExtent) {
 }
 
 // (re)allocates the guide's buffers for a pool of `capacity` paths
-static rmd_status guideBuffers(GuideState &g, uint32_t capacity, Counters *counters) {
+static rmd_status guideBuffers(GuideState &g, uint32_t capacity, Counters *counters, cudaStream_t stream) {
     if (!g.settings.sampling && !g.settings.training) return RMD_OK;
     if (g.pathCapacity < capacity) {
         g.pathCapacity = 0;
@@ -1122,13 +1124,13 @@ static rmd_status guideBuffers(GuideState &g, uint32_t capacity, Counters *count
         g.recordCapacity = 0;
         RMD_CUDA(g.records.alloc((size_t)want * sizeof(GuideRecord)));
         g.recordCapacity = want;
-        RMD_CUDA(cudaMemset(&counters->numRecords, 0, 2 * sizeof(uint32_t)));
+        RMD_CUDA(cudaMemsetAsync(&counters->numRecords, 0, 2 * sizeof(uint32_t), stream));
     }
     return RMD_OK;
 }
 
 static rmd_status ensureGuideBuffers(rmd_renderer *r) {
-    return guideBuffers(r->guide, r->capacity, r->counters.as<Counters>());
+    return guideBuffers(r->guide, r->capacity, r->counters.as<Counters>(), r->scene->ctx->stream);
 }
 
 // Adam steps due after a counter check: one per `batch_size` samples (times
@@ -1175,7 +1177,7 @@ static rmd_status setGuide(GuideState &g, const rmd_guide_settings *settings, cu
     if (next.replay_records == 0) next.replay_records = 1u << 18;
     if (next.steps_per_batch == 0) next.steps_per_batch = 8;
     if (next.guided_depth == 0) next.guided_depth = 65535;
-    if (!g.net.allocated()) RMD_CUDA(g.net.allocate());
+    if (!g.net.allocated()) RMD_CUDA(g.net.allocate(stream));
     if (!g.initialised || next.reset) {
         std::vector<float> params(GUIDE_PARAMS);
         rmdhost::GuideNet::initParams(params.data(), next.seed);
@@ -1183,7 +1185,7 @@ static rmd_status setGuide(GuideState &g, const rmd_guide_settings *settings, cu
         g.initialised = true;
         g.stats = rmd_guide_stats{};
         // records gathered by an earlier network are dropped with it
-        RMD_CUDA(cudaMemset(&counters->numRecords, 0, 2 * sizeof(uint32_t)));
+        RMD_CUDA(cudaMemsetAsync(&counters->numRecords, 0, 2 * sizeof(uint32_t), stream));
     }
     next.reset = 0;
     g.settings = next;
@@ -1191,7 +1193,7 @@ static rmd_status setGuide(GuideState &g, const rmd_guide_settings *settings, cu
 }
 
 static rmd_status guideParams(GuideState &g, float *params, int32_t write, cudaStream_t stream) {
-    if (!g.net.allocated()) RMD_CUDA(g.net.allocate());
+    if (!g.net.allocated()) RMD_CUDA(g.net.allocate(stream));
     if (write) {
         for (int i = 0; i < GUIDE_PARAMS; i++)
             if (!std::isfinite(params[i])) return fail(RMD_ERROR_INVALID_ARGUMENT, "non-finite guide parameter");
@@ -1762,7 +1764,7 @@ rmd_status rmd_test_trace(const rmd_scene *s, const float *rays, int32_t n, int3
     RMD_CUDA(dout.alloc((size_t)std::max(1, n) * 4 * sizeof(float)));
     RMD_CUDA(dinst.alloc((size_t)std::max(1, n) * sizeof(uint32_t)));
     RMD_CUDA(derr.alloc(sizeof(uint32_t)));
-    RMD_CUDA(cudaMemset(derr.ptr, 0, sizeof(uint32_t)));
+    RMD_CUDA(cudaMemsetAsync(derr.ptr, 0, sizeof(uint32_t), s->ctx->stream));
     if (n > 0)
         RMD_CUDA(rmdLaunchDebugTrace(s->bvhNodes.as<WideNode>(), s->bvhTris.as<float4>(), dr.as<float>(), n, any,
                                      dout.as<float>(), dinst.as<uint32_t>(), derr.as<uint32_t>(), s->ctx->stream));
@@ -1874,8 +1876,8 @@ static rmd_status batchAllocatePool(rmd_batch *b) {
     b->graphKey.clear();
     RMD_CUDA(b->pool.alloc(pathPoolBytes(b->capacity)));
     RMD_CUDA(b->counters.alloc(sizeof(Counters)));
-    RMD_CUDA(cudaMemset(b->counters.ptr, 0, sizeof(Counters)));
-    return guideBuffers(b->guide, b->capacity, b->counters.as<Counters>());
+    RMD_CUDA(cudaMemsetAsync(b->counters.ptr, 0, sizeof(Counters), b->ctx->stream));
+    return guideBuffers(b->guide, b->capacity, b->counters.as<Counters>(), b->ctx->stream);
 }
 
 static PathPool batchPoolView(const rmd_batch *b) {
@@ -2030,7 +2032,7 @@ rmd_status rmd_batch_create(rmd_context *ctx, const rmd_scene_desc *descs, int32
     b->totalPixels = offset;
     RMD_CUDA(b->viewTable.upload(table.data(), table.size() * sizeof(BatchView), ctx->stream));
     RMD_CUDA(b->film.alloc((size_t)offset * sizeof(float4)));
-    RMD_CUDA(cudaMemset(b->film.ptr, 0, b->film.bytes));
+    RMD_CUDA(cudaMemsetAsync(b->film.ptr, 0, b->film.bytes, ctx->stream));
     RMD_CUDA(b->resolve.alloc((size_t)offset * 3 * sizeof(float)));
     b->capacity = poolSize ? poolSize : (1u << 21);
     if (b->capacity > BATCH_MAX_CAPACITY) return fail(RMD_ERROR_INVALID_ARGUMENT, "batch pools hold at most 2^22 paths");
@@ -2116,7 +2118,7 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
     }
     GuideNetView net{};
     if (guide.settings.sampling || guide.settings.training) {
-        rmd_status gs = guideBuffers(guide, b->capacity, b->counters.as<Counters>());
+        rmd_status gs = guideBuffers(guide, b->capacity, b->counters.as<Counters>(), st);
         if (gs != RMD_OK) return gs;
         net = guide.net.view(guide.frameMin, guide.frameInvExtent);
         fp.guideDepth = guide.settings.sampling ? guide.settings.guided_depth : 0u;
@@ -2252,7 +2254,7 @@ rmd_status rmd_batch_set_guide(rmd_batch *b, const rmd_guide_settings *settings)
         b->graphExec = nullptr;
     }
     b->graphKey.clear();
-    return guideBuffers(b->guide, b->capacity, b->counters.as<Counters>());
+    return guideBuffers(b->guide, b->capacity, b->counters.as<Counters>(), b->ctx->stream);
 }
 
 rmd_status rmd_batch_guide_stats(const rmd_batch *b, rmd_guide_stats *out) {

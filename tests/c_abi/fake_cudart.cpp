@@ -227,9 +227,11 @@ cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t s) {
     std::memset(p, v, n);
     return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind kind) {
     ASK("cudaMemcpy", d, n);
+    enqueue(nullptr);  // from pageable memory it may return before the last bytes have arrived
     std::memcpy(d, s, n);
+    if (kind == cudaMemcpyDeviceToHost) g_legacy.done = g_legacy.enqueued;
     return cudaSuccess;
 }
 // the hook gets the source
