@@ -44,13 +44,6 @@ static __device__ __align__(256) unsigned char g_noallocScratch[kScratchBytes];
 
 std::mutex g_mutex;
 void *g_scratch[64] = {};  // device address of g_noallocScratch per device, set by noallocSetup
-// Pinned counters and events of the render loop, per device, made with the
-// first context (2 x sizeof(Counters)) and kept: like the array, shared by all calls.
-struct HostSide {
-    Counters *counters = nullptr;
-    cudaEvent_t events[2] = {};
-};
-HostSide g_host[64];
 
 rmd_status cudaFail(cudaError_t e, const char *what) {
     std::string msg = std::string("rmd_render_noalloc: ") + what + ": " + cudaGetErrorString(e);
@@ -65,22 +58,10 @@ namespace rmdhost {
 rmd_status noallocSetup(int device) {
     if (device < 0 || device >= 64) return RMD_OK;  // rmd_render_noalloc rejects such devices
     void *ptr = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&ptr, g_noallocScratch);
+    const cudaError_t e = cudaGetSymbolAddress(&ptr, g_noallocScratch);
     if (e != cudaSuccess) return cudaFail(e, "cudaGetSymbolAddress");
     std::lock_guard<std::mutex> lock(g_mutex);
     g_scratch[device] = ptr;
-    HostSide &h = g_host[device];
-    // Made anew only if they went with a device reset: a call that renders on another thread leaves its event
-    // pending (cudaErrorNotReady), and goes on using these.
-    const cudaError_t alive = h.events[0] ? cudaEventQuery(h.events[0]) : cudaSuccess;
-    if (alive != cudaSuccess) cudaGetLastError();
-    if (alive == cudaErrorInvalidResourceHandle || alive == cudaErrorContextIsDestroyed || alive == cudaErrorDeviceUninitialized)
-        h = HostSide();
-    for (cudaEvent_t &ev : h.events)
-        if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
-            return cudaFail(e, "cudaEventCreate");
-    if (!h.counters && (e = cudaMallocHost((void **)&h.counters, 2 * sizeof(Counters))) != cudaSuccess)
-        return cudaFail(e, "cudaMallocHost");
     return RMD_OK;
 }
 
@@ -107,13 +88,11 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
     if (e != cudaSuccess) return cudaFail(e, "cudaSetDevice");
 
     void *base;
-    HostSide host;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         base = g_scratch[v.device];  // set when the scene's context was created
-        host = g_host[v.device];
     }
-    if (!base || !host.counters) return rmdhost::setLastError(RMD_ERROR_CUDA, "rmd_render_noalloc: scratch array not set up");
+    if (!base) return rmdhost::setLastError(RMD_ERROR_CUDA, "rmd_render_noalloc: scratch array not set up");
     const uint32_t P = pool_size ? pool_size : kMaxPaths;
     Counters *cnt = static_cast<Counters *>(base);
     const PathPool pool = carvePathPool(static_cast<unsigned char *>(base) + kCountersBytes, P);
@@ -169,7 +148,7 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
             status = rmdhost::setLastError(RMD_ERROR_WATCHDOG, "rmd_render_noalloc: render did not drain");
         return status != RMD_OK || h.pathsDone >= numPaths;
     };
-    e = rmdhost::driveWavefront(cnt, numPaths, P, host.counters, host.events, st, iterate, check);
+    e = rmdhost::driveWavefront(cnt, numPaths, P, v.loop->counters, v.loop->events, st, iterate, check);
     if (e != cudaSuccess) return cudaFail(e, "wavefront");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cudaFail(e, "synchronize");
     if (status != RMD_OK) return status;

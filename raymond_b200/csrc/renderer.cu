@@ -225,6 +225,7 @@ struct rmd_context {
     cudaStream_t stream = nullptr;
     uint32_t bvhBuilder = RMD_BVH_HOST;  // builder of the scenes created next
     std::shared_ptr<DevPool> memory = std::make_shared<DevPool>();
+    rmdhost::LoopHost noallocLoop;
 };
 
 struct rmd_scene {
@@ -485,6 +486,7 @@ bool sceneView(const rmd_scene *s, SceneView &v) {
     v.shade = s->jit.shade;
     v.shadeBlocks = s->shadeBlocks;
     v.stream = s->ctx->stream;
+    v.loop = &s->ctx->noallocLoop;
     v.device = s->ctx->device;
     v.smCount = s->ctx->smCount;
     return true;
@@ -511,6 +513,7 @@ rmd_status rmd_context_create(int32_t device, rmd_context **out) {
     c->device = device;
     RMD_CUDA(cudaSetDevice(device));
     RMD_CUDA(cudaDeviceGetAttribute(&c->smCount, cudaDevAttrMultiProcessorCount, device));
+    RMD_CUDA(c->noallocLoop.create());
     RMD_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     const rmd_status ns = rmdhost::noallocSetup(device);
     if (ns != RMD_OK) {

@@ -8,6 +8,25 @@
 
 namespace rmdhost {
 
+// Pinned counters (two) and events of rmd_render_noalloc's loop, which may not
+// allocate them.  A context has its own: they come with it, nothing replaces
+// them under a call, and a context made after a device reset has new ones.
+struct LoopHost {
+    rmd::Counters *counters = nullptr;
+    cudaEvent_t events[2] = {};
+    cudaError_t create() {
+        cudaError_t e = cudaMallocHost((void **)&counters, 2 * sizeof(rmd::Counters));
+        for (cudaEvent_t &ev : events)
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        return e;
+    }
+    ~LoopHost() {
+        for (cudaEvent_t ev : events)
+            if (ev) cudaEventDestroy(ev);
+        if (counters) cudaFreeHost(counters);
+    }
+};
+
 struct SceneView {
     rmd::Context ctx;              // device view of geometry, lights, materials, camera
     const rmd::WideNode *nodes;     // nullptr for a scene without triangles
@@ -15,6 +34,7 @@ struct SceneView {
     cudaKernel_t shade;            // shading megakernel of the scene's material module
     int shadeBlocks;
     cudaStream_t stream;
+    LoopHost *loop;                // of the scene's context
     int device;
     int smCount;
 };

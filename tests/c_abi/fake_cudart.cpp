@@ -23,11 +23,13 @@ struct Stream {
 struct Event {
     Stream *stream = nullptr;  // null: never recorded
     unsigned long long at = 0;
+    int life = 0;  // the device's when it was made
 };
 using Hook = int (*)(const char *name, void *ptr, size_t size, void *stream);
 
 std::recursive_mutex g_mutex;
 Hook g_hook = nullptr;
+int g_life = 0, g_staleUses = 0;
 Stream g_legacy;
 std::map<Stream *, bool> g_streams;  // made by the library
 std::map<void *, size_t> g_blocks;   // cudaMalloc'd
@@ -86,6 +88,13 @@ cudaError_t launch(const void *kernel, cudaStream_t s) {
     return e;
 }
 
+// the event, noting the use of one that went with a device reset (undefined in the real runtime)
+Event *eventOf(cudaEvent_t e) {
+    Event *x = reinterpret_cast<Event *>(e);
+    if (x->life != g_life) g_staleUses++;
+    return x;
+}
+
 #define ASK(...)                                        \
     do {                                                \
         const cudaError_t e_ = ask(__VA_ARGS__);        \
@@ -113,6 +122,9 @@ unsigned long long fake_pending(void *stream) {
     Stream *s = of((cudaStream_t)stream);
     return s->enqueued - s->done;
 }
+// as a device reset: events made before are gone; and how often one was used all the same
+void fake_reset_device(void) { g_life++; }
+int fake_stale_uses(void) { return g_staleUses; }
 void fake_set_capturing(void *stream, int on) { of((cudaStream_t)stream)->capturing = on != 0; }
 
 // ------------------------------------------------------------- registration
@@ -271,7 +283,9 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) {
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
     ASK("cudaEventCreate");
-    *e = (cudaEvent_t) new Event;
+    Event *x = new Event;
+    x->life = g_life;
+    *e = (cudaEvent_t)x;
     return cudaSuccess;
 }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e, 0); }
@@ -279,7 +293,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }  // the object
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
     ASK("cudaEventRecord", e, 0, s);
     Lock lock(g_mutex);
-    Event *x = reinterpret_cast<Event *>(e);
+    Event *x = eventOf(e);
     x->stream = of(s);
     x->at = of(s)->enqueued;
     return cudaSuccess;
@@ -287,14 +301,14 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
 cudaError_t cudaEventSynchronize(cudaEvent_t e) {
     ASK("cudaEventSynchronize", e);
     Lock lock(g_mutex);
-    Event *x = reinterpret_cast<Event *>(e);
+    Event *x = eventOf(e);
     if (x->stream && x->stream->done < x->at) x->stream->done = x->at;
     return cudaSuccess;
 }
 cudaError_t cudaEventQuery(cudaEvent_t e) {
     ASK("cudaEventQuery", e);
     Lock lock(g_mutex);
-    const Event *x = reinterpret_cast<Event *>(e);
+    const Event *x = eventOf(e);
     return x->stream && x->stream->done < x->at ? result(cudaErrorNotReady) : cudaSuccess;
 }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
