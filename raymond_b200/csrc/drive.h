@@ -15,18 +15,21 @@ namespace rmdhost {
 // its grids need to cover); check(counters, iterations) returns whether the
 // render is over (done, or failed).
 //
-// The first counters are read once every path has been handed out and could
-// have ended, and then after every second iteration, two iterations behind the
-// ones being enqueued: the device never waits for the host, for at most four
-// empty iterations at the end.  (Reading them after every fourth iteration and
-// waiting left a gap of 10-20 us each time.)  `slots`: two Counters in pinned
-// memory; `events`: two events.  On return the last iterations may still run.
+// The counters are read after every eighth iteration until every path has been
+// handed out and could have ended, and then after every second, each read
+// looked at once the iterations up to the next are enqueued: the device never
+// waits for the host, for at most four empty iterations at the end, and a
+// device error ends a render of any length within 16 iterations.  (Reading them
+// after every fourth iteration and waiting left a gap of 10-20 us each time.)
+// `slots`: two Counters in pinned memory; `events`: two events.  On return the
+// last iterations may still run.
 template <class Iterate, class Check>
 cudaError_t driveWavefront(const rmd::Counters *cnt, uint64_t numPaths, uint32_t capacity, rmd::Counters *slots,
                            cudaEvent_t *events, cudaStream_t st, Iterate iterate, Check check) {
     uint64_t it = 0, paths = std::min<uint64_t>(numPaths, capacity);
-    uint64_t next = ((numPaths + capacity - 1) / capacity + 3) & ~uint64_t(1);
-    for (uint32_t k = 0;; k++, next += 2) {
+    const uint64_t handedOut = ((numPaths + capacity - 1) / capacity + 3) & ~uint64_t(1);
+    uint64_t next = std::min<uint64_t>(handedOut, 8);
+    for (uint32_t k = 0;; k++, next = next < handedOut ? std::min(handedOut, next + 8) : next + 2) {
         cudaError_t e;
         for (; it < next; it++)
             if ((e = iterate((uint32_t)(it & 1u), paths)) != cudaSuccess) return e;

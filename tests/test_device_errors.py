@@ -1,0 +1,62 @@
+"""A device error ends a render within a few iterations (host side, the device's part played by the test)."""
+import numpy as np
+import pytest
+
+from host_runtime import ERRORS, PATHS_DONE, fake  # noqa: F401
+from raymond_b200 import scenes
+from raymond_b200._abi import SceneDesc
+
+W, H, SPP, POOL = 64, 48, 64, 64  # 3,072 pools of paths
+
+
+def _render(fake, call, see_counters):
+    api = fake.api
+    desc = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
+    ctx = api.Context(0)
+    if call == "batch":
+        b = api.Batch(ctx, [desc], [{"scene": 0, "width": W, "height": H}], pool_size=POOL, graph=False)
+        run = lambda: b.render(spp=SPP, max_depth=4, first_sample=0)
+    elif call == "noalloc":
+        scene, film = api.Scene(ctx, desc), np.zeros((H, W, 4), np.float32)
+        run = lambda: api.render_noalloc(scene, desc.scene["camera"], W, H, film.ctypes.data, spp=SPP, first_sample=0,
+                                         max_depth=4, pool_size=POOL)
+    else:
+        r = api.Renderer(api.Scene(ctx, desc), W, H, pool_size=POOL)
+        if call == "guided":
+            r.set_guide(sampling=True, training=False)
+        run = lambda: r.render(spp=SPP, max_depth=4, first_sample=0)
+    iterations = [0]
+
+    def see(name, ptr, size, stream):
+        if name == "launch:rmd_shade":
+            iterations[0] += 1
+        elif fake.is_counters(name, size):
+            fake.counter(ptr, ERRORS, 32).value = 0  # the kernel that clears them does nothing here
+            see_counters(ptr, iterations[0])
+
+    with fake.on(see):
+        run()
+    return iterations[0]
+
+
+@pytest.mark.parametrize("call", ["render", "guided", "noalloc", "batch"])
+def test_errors_are_seen_early(fake, call):
+    seen = []
+
+    def error(ptr, iterations):
+        seen.append(iterations)
+        fake.counter(ptr, ERRORS, 32).value = 2
+
+    with pytest.raises(fake.api.RmdError, match="error flags"):
+        _render(fake, call, error)
+    assert seen[0] <= 16 and seen[-1] <= 32
+
+
+@pytest.mark.parametrize("call", ["render", "noalloc", "batch"])
+@pytest.mark.parametrize("ends", [3074, 3081, 4000])
+def test_the_end_is_seen_soon(fake, call, ends):
+    """A render ends within six iterations of its last path (the counters of iteration i are read after i + 2)."""
+    def play(ptr, iterations):
+        fake.counter(ptr, PATHS_DONE).value = W * H * SPP if iterations >= ends else 0
+
+    assert ends <= _render(fake, call, play) <= ends + 6
