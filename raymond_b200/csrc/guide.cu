@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_guide_train_tc(RecordBatch ba
             }
             for (int i = threadIdx.x; i < 3 * GUIDE_HIDDEN + GUIDE_OUTPUTS; i += blockDim.x) {
                 const int l = min(i / GUIDE_HIDDEN, 3);
-                sm.b[i] = __ldg(&net.b[l][i - l * GUIDE_HIDDEN]);
+                sm.b[i] = __ldcg(&net.b[l][i - l * GUIDE_HIDDEN]);
             }
             const float sum = __ldcg(sumY);
             invMeanY = sum > 0.0f ? (float)n / sum : 0.0f;
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(256) k_guide_features(Context ctx, PathPool po
         GuideFeatures f = {};
         if (depth < guideDepth) {  // only guided vertices need the features
             // a batch path's scene is its view's (the view in the top bits of its sample word)
-            const Context &c = pool.views ? pool.views[__ldg(&S.id[idx].y) >> BATCH_SAMPLE_BITS].ctx : ctx;
+            const Context &c = pool.views ? pool.views[__ldcg(&S.id[idx].y) >> BATCH_SAMPLE_BITS].ctx : ctx;
             const float4 o = __ldcs(&S.rayO[idx]), dd = __ldcs(&S.rayD[idx]), h = pool.hit[idx];
             const PerInstanceData &inst = c.instances[pool.hitInst[idx]];
             const uint4 face = c.faces[inst.faceOffset + __float_as_uint(h.w)];

@@ -159,7 +159,7 @@ template <bool BATCH>
 __device__ __forceinline__ void closestRay(const PathPool &pool, const PathState &S, uint32_t idx, const WideNode *&nodes,
                                            const float4 *&tris, float4 &o, float4 &d) {
     if constexpr (BATCH) {
-        const BatchView &bv = pool.views[__ldg(&S.id[idx].y) >> BATCH_SAMPLE_BITS];
+        const BatchView &bv = pool.views[__ldcg(&S.id[idx].y) >> BATCH_SAMPLE_BITS];
         nodes = static_cast<const WideNode *>(bv.nodes);
         tris = bv.tris;
     }
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, 8) k_trace(const WideNode *__re
                     beginTraversal(s, nodes, xyz(o), xyz(d), SHADOW_EPS, o.w);
                     traverse<true>(s, stack, nodes, tris, &cnt->errors);
                     if (s.hitTri < 0)
-                        unoccluded<BATCH>(pool, cnt, q, idx, __float_as_uint(__ldg(&pool.shD[idx].w)));
+                        unoccluded<BATCH>(pool, cnt, q, idx, __float_as_uint(__ldcg(&pool.shD[idx].w)));
                 }
             }
             __syncwarp();
