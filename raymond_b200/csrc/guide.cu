@@ -21,6 +21,7 @@
 #include "device/scene.cuh"
 #include "device/wavefront.cuh"
 #include "guide.h"
+#include "memory.h"
 
 namespace rmd {
 namespace {
@@ -1379,14 +1380,11 @@ cudaError_t GuideNet::allocate(cudaStream_t s) {
     release();
     const size_t pb = GUIDE_PARAMS * sizeof(float);
     cudaError_t e;
-    if ((e = cudaMalloc(&master, pb)) != cudaSuccess || (e = cudaMalloc(&adamM, pb)) != cudaSuccess ||
-        (e = cudaMalloc(&adamV, pb)) != cudaSuccess || (e = cudaMalloc(&grad, pb)) != cudaSuccess ||
-        (e = cudaMalloc(&scratch, 64 * sizeof(float))) != cudaSuccess ||
-        (e = cudaMalloc(&partials, (size_t)GUIDE_TRAIN_MAX_BLOCKS * (pb + sizeof(float)))) != cudaSuccess ||
-        (e = cudaMalloc(&weightsBf16, GUIDE_WEIGHTS * sizeof(uint16_t))) != cudaSuccess ||
-        (e = cudaMalloc(&bf16Index, GUIDE_PARAMS * sizeof(int))) != cudaSuccess ||
-        (e = cudaMalloc(&image, kImageBytes)) != cudaSuccess ||
-        (e = cudaMalloc(&imageIndex, GUIDE_PARAMS * sizeof(int))) != cudaSuccess)
+    const auto alloc = [&](auto *&p, size_t n) { return (e = rmdhost::deviceAlloc((void **)&p, n)) == cudaSuccess; };
+    if (!alloc(master, pb) || !alloc(adamM, pb) || !alloc(adamV, pb) || !alloc(grad, pb) ||
+        !alloc(scratch, 64 * sizeof(float)) || !alloc(partials, (size_t)GUIDE_TRAIN_MAX_BLOCKS * (pb + sizeof(float))) ||
+        !alloc(weightsBf16, GUIDE_WEIGHTS * sizeof(uint16_t)) || !alloc(bf16Index, GUIDE_PARAMS * sizeof(int)) ||
+        !alloc(image, kImageBytes) || !alloc(imageIndex, GUIDE_PARAMS * sizeof(int)))
         return e;
     std::vector<int> idx(GUIDE_PARAMS, -1), img(GUIDE_PARAMS, -1);
     int wOff[4], bOff[4], qOff[4];
@@ -1493,11 +1491,11 @@ struct DeviceArray {
         if (p) cudaFree(p);
     }
     cudaError_t upload(const void *h, size_t n) {
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 16));
+        cudaError_t e = alloc(n);
         if (e != cudaSuccess || n == 0) return e;
         return cudaMemcpy(p, h, n, cudaMemcpyHostToDevice);
     }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 16)); }
+    cudaError_t alloc(size_t n) { return rmdhost::deviceAlloc(&p, std::max<size_t>(n, 16)); }
 };
 }  // namespace
 

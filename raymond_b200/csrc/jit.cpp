@@ -1,6 +1,8 @@
 // NVRTC driver for the material module.
 #include "jit.h"
 
+#include "memory.h"
+
 #include <nvrtc.h>
 
 #include <chrono>
@@ -71,7 +73,7 @@ std::string compileModule(const std::string &source, JitModule &out, const std::
     const auto t0 = std::chrono::steady_clock::now();
     std::string err = compileCubin(source, cubin, out.log, out.fromCache, extraDefines);
     if (!err.empty()) return err;
-    cudaError_t e = cudaLibraryLoadData(&out.library, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
+    cudaError_t e = loadLibrary(&out.library, cubin.data());
     if (e != cudaSuccess) return std::string("cudaLibraryLoadData: ") + cudaGetErrorString(e);
     if ((e = cudaLibraryGetKernel(&out.shade, out.library, "rmd_shade")) != cudaSuccess ||
         (e = cudaLibraryGetKernel(&out.envmapBuild, out.library, "rmd_envmap_build")) != cudaSuccess ||

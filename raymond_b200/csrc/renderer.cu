@@ -9,7 +9,6 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -25,9 +24,12 @@
 #include "guide.h"
 #include "jit.h"
 #include "kernels.h"
+#include "memory.h"
 #include "scene_view.h"
 
 using namespace rmd;
+using rmdhost::DevBuf;
+using rmdhost::DevPool;
 
 // The host-facing records keep the layout of the reference's DEVICE_STRUCTs
 // (raymond/bridge/Camera.hpp, PerInstanceData.hpp, Uniforms.hpp, lights/ *.hpp)
@@ -93,116 +95,6 @@ static int defaultShadeMinBlocks() {
     return v >= 1 && v <= 16 ? v : 5;
 }
 
-// A context's device memory: blocks that its scenes, renderers and batches free
-// stay with it for the next ones, up to kMemoryKept bytes; beyond that, and
-// with the context and its last object, they go back to the device.  cudaMalloc
-// and cudaFree of the 10-500 MB blocks that a scene and its renderer take cost
-// 1-10 ms each, and now and then hundreds (the 852 k-triangle scene: 20 ms to
-// 4 s of a creation).  A driver pool maps its memory anew whenever a block fits
-// no hole (2-3 ms for the tree's workspace and for the paths, in one of four
-// creations 40-1,200 ms); a kept block is handed out as it is.  Sizes below
-// 1 GiB are rounded up to an eighth of their power of two, so that a scene a
-// little larger than the one before takes the same blocks.  Any thread may
-// allocate and free.
-struct DevPool {
-    static constexpr size_t kMemoryKept = size_t(2) << 30;
-    std::mutex mutex;
-    std::multimap<size_t, void *> kept;  // free blocks by size
-    size_t keptBytes = 0;
-    static size_t rounded(size_t n) {
-        size_t step = 512;
-        if (n < (size_t(1) << 30))
-            while (step * 16 <= n) step *= 2;
-        return (n + step - 1) / step * step;
-    }
-    // a block of the current device, which has to be the context's
-    cudaError_t alloc(void **p, size_t n) {
-        const size_t size = rounded(n);
-        {
-            std::lock_guard<std::mutex> lock(mutex);
-            const auto it = kept.find(size);
-            if (it != kept.end()) {
-                *p = it->second;
-                keptBytes -= size;
-                kept.erase(it);
-                return cudaSuccess;
-            }
-        }
-        cudaError_t e = cudaMalloc(p, size);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            giveBack();
-            e = cudaMalloc(p, size);
-        }
-        return e;
-    }
-    // takes back a block that alloc gave for n bytes; no work may use it any more
-    void free(void *p, size_t n) {
-        const size_t size = rounded(n);
-        std::lock_guard<std::mutex> lock(mutex);
-        kept.emplace(size, p);
-        keptBytes += size;
-        while (keptBytes > kMemoryKept) {  // the largest go first: small ones are asked for on every read-out
-            const auto largest = std::prev(kept.end());
-            cudaFree(largest->second);
-            keptBytes -= largest->first;
-            kept.erase(largest);
-        }
-    }
-    void giveBack() {
-        std::lock_guard<std::mutex> lock(mutex);
-        for (auto &block : kept) cudaFree(block.second);
-        kept.clear();
-        keptBytes = 0;
-    }
-    ~DevPool() { giveBack(); }
-};
-
-// Device buffer owned by a scene, renderer or batch, from its context's pool
-// where one is set.  Whoever frees it has waited for the work that uses it: the
-// pool does not.  A new one may hold what a block's last owner left, so it is
-// cleared and filled on the stream that uses it (the legacy stream is not
-// ordered with a context's).
-struct DevBuf {
-    void *ptr = nullptr;
-    size_t bytes = 0;
-    std::shared_ptr<DevPool> from;
-    DevBuf() = default;
-    DevBuf(const DevBuf &) = delete;
-    DevBuf &operator=(const DevBuf &) = delete;
-    ~DevBuf() { release(); }
-    void release() {
-        if (ptr) {
-            if (from) from->free(ptr, bytes);
-            else cudaFree(ptr);
-        }
-        ptr = nullptr;
-        bytes = 0;
-    }
-    cudaError_t alloc(size_t n) {
-        release();
-        bytes = n;
-        if (n == 0) return cudaSuccess;
-        return from ? from->alloc(&ptr, n) : cudaMalloc(&ptr, n);
-    }
-    void adopt(void *p, size_t n) {  // takes ownership of a block allocated as alloc(n) does
-        release();
-        ptr = p;
-        bytes = n;
-    }
-    cudaError_t upload(const void *src, size_t n, cudaStream_t s) {
-        cudaError_t e = alloc(n);
-        if (e != cudaSuccess || n == 0) return e;
-        e = cudaMemcpyAsync(ptr, src, n, cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return e;
-        return cudaStreamSynchronize(s);
-    }
-    template <class T>
-    T *as() const {
-        return static_cast<T *>(ptr);
-    }
-};
-
 struct HostMat4 {
     float c[4][4];  // columns
 };
@@ -224,7 +116,7 @@ struct rmd_context {
     int smCount = 148;
     cudaStream_t stream = nullptr;
     uint32_t bvhBuilder = RMD_BVH_HOST;  // builder of the scenes created next
-    std::shared_ptr<DevPool> memory = std::make_shared<DevPool>();
+    std::shared_ptr<DevPool> memory;
     rmdhost::LoopHost noallocLoop;
 };
 
@@ -511,6 +403,7 @@ rmd_status rmd_context_create(int32_t device, rmd_context **out) {
     if (device < 0 || device >= count) return fail(RMD_ERROR_INVALID_ARGUMENT, "device index out of range");
     auto c = std::make_unique<rmd_context>();
     c->device = device;
+    c->memory = std::make_shared<DevPool>(device);
     RMD_CUDA(cudaSetDevice(device));
     RMD_CUDA(cudaDeviceGetAttribute(&c->smCount, cudaDevAttrMultiProcessorCount, device));
     RMD_CUDA(c->noallocLoop.create());
@@ -1600,7 +1493,7 @@ static rmd_status ensureVariants(rmd_scene *s, const std::vector<int> &minBlocks
     for (size_t i = 0; i < missing.size(); i++) {
         if (!errs[i].empty()) return fail(RMD_ERROR_NVRTC, errs[i]);
         auto m = std::make_unique<rmdhost::JitModule>();
-        RMD_CUDA(cudaLibraryLoadData(&m->library, cubins[i].data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+        RMD_CUDA(rmdhost::loadLibrary(&m->library, cubins[i].data()));
         RMD_CUDA(cudaLibraryGetKernel(&m->shade, m->library, "rmd_shade"));
         s->variants[shadeVariantKey(missing[i], guided)] = std::move(m);
     }
@@ -1751,7 +1644,7 @@ rmd_status rmd_renderer_guide_params(rmd_renderer *r, float *params, int32_t wri
 rmd_status rmd_test_prng(uint32_t mode, uint64_t a, uint64_t b, int32_t n, float *out) {
     if (!out || n < 0) return fail(RMD_ERROR_INVALID_ARGUMENT, "invalid arguments");
     float *d = nullptr;
-    RMD_CUDA(cudaMalloc(&d, std::max<int>(1, n) * sizeof(float)));
+    RMD_CUDA(rmdhost::deviceAlloc((void **)&d, std::max<int>(1, n) * sizeof(float)));
     cudaError_t e = rmdLaunchDebugPrng(mode, a, b, n, d, 0);
     if (e == cudaSuccess) e = cudaMemcpy(out, d, n * sizeof(float), cudaMemcpyDeviceToHost);
     cudaFree(d);
@@ -2176,7 +2069,7 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
             cudaError_t endErr = cudaStreamEndCapture(st, &captured);
             RMD_CUDA(ce);
             RMD_CUDA(endErr);
-            RMD_CUDA(cudaGraphInstantiate(&b->graphExec, b->graph, 0));
+            RMD_CUDA(rmdhost::withKeptMemory([&] { return cudaGraphInstantiate(&b->graphExec, b->graph, 0); }));
             b->graphKey = key;
         }
         RMD_CUDA(cudaGraphLaunch(b->graphExec, st));

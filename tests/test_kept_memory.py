@@ -1,0 +1,94 @@
+"""A context's kept blocks and the allocations that find the device full (host
+side, on a device whose size the test sets)."""
+import pytest
+
+from host_runtime import OUT_OF_MEMORY, fake  # noqa: F401
+from raymond_b200 import scenes
+from raymond_b200._abi import SceneDesc
+
+W, H = 512, 512
+DESC = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
+
+
+def _full_device(fake, ctx, blocks=3):
+    """Blocks of ~0.5 GB kept by `ctx`, and nothing else free on the device."""
+    api = fake.api
+    scene = api.Scene(ctx, DESC)
+    renderers = [api.Renderer(scene, 16, 16, pool_size=1 << 21) for _ in range(blocks)]
+    for r in renderers:
+        r.close()
+    assert fake.lib.fake_allocated() > blocks * (500 << 20)
+    fake.lib.fake_set_capacity(fake.lib.fake_allocated() + (1 << 20))
+    return scene
+
+
+def test_film_takes_what_the_context_keeps(fake):
+    scene = _full_device(fake, fake.api.Context(0))
+    r = fake.api.Renderer(scene, W, H, pool_size=1 << 12)  # 4 MB of film, outside the pool
+    r.set_size(2 * W, 2 * H)
+    r.close()
+
+
+def test_network_takes_what_the_context_keeps(fake):
+    api = fake.api
+    ctx = api.Context(0)
+    r = api.Renderer(api.Scene(ctx, DESC), 16, 16, pool_size=1 << 12)
+    _full_device(fake, ctx)
+    r.set_guide(sampling=True, training=True)  # the gradient slots of the network: 27 MB
+    assert len(r.guide_params()) == api.guide_param_count()
+    r.close()
+
+
+def test_another_context_takes_what_a_context_keeps(fake):
+    api = fake.api
+    scene = _full_device(fake, api.Context(0))
+    r = api.Renderer(api.Scene(api.Context(0), DESC), W, H, pool_size=1 << 20)
+    r.close(), scene.close()
+
+
+@pytest.mark.parametrize("call", ["cudaLibraryLoadData", "cudaGraphInstantiate"])
+def test_modules_and_graphs_take_what_a_context_keeps(fake, call):
+    api = fake.api
+    ctx = api.Context(0)
+    scene = _full_device(fake, ctx)
+    kept = fake.lib.fake_allocated()
+    failed = []
+
+    def see(name, ptr, size, stream):
+        if name == call and not failed:
+            failed.append(fake.lib.fake_allocated())
+            return OUT_OF_MEMORY
+
+    with fake.on(see):
+        b = api.Batch(ctx, [DESC], [{"scene": 0, "width": 8, "height": 8}], pool_size=1 << 10)
+        if call == "cudaGraphInstantiate":
+            b.render(spp=1, max_depth=2, first_sample=0)
+    assert failed and fake.lib.fake_allocated() < kept - (1 << 30)
+    b.close(), scene.close()
+
+
+def test_out_of_memory_is_reported_when_nothing_is_kept(fake):
+    api = fake.api
+    scene = api.Scene(api.Context(0), DESC)
+    fake.lib.fake_set_capacity(fake.lib.fake_allocated() + (1 << 20))
+    with pytest.raises(api.RmdError, match="OUT_OF_MEMORY"):
+        api.Renderer(scene, W, H, pool_size=1 << 20)
+    fake.lib.fake_set_capacity(180 << 30)
+    api.Renderer(scene, W, H, pool_size=1 << 20).close()  # and the failure is forgotten
+    scene.close()
+
+
+def test_the_bound_holds_and_all_goes_with_the_context(fake):
+    api = fake.api
+    before = fake.lib.fake_allocated()
+    ctx = api.Context(0)
+    scene = api.Scene(ctx, DESC)
+    base = fake.lib.fake_allocated()
+    renderers = [api.Renderer(scene, 16, 16, pool_size=1 << 21) for _ in range(6)]
+    for r in renderers:
+        r.close()
+    assert base < fake.lib.fake_allocated() <= base + (2 << 30)
+    scene.close()
+    ctx.close()
+    del scene
+    assert fake.lib.fake_allocated() == before
