@@ -125,6 +125,19 @@ inline bool giveBackKept(int device) {
         if (p->device == device && p->giveBack()) any = true;
     return any;
 }
+// Free memory of the current device, the kept blocks included.
+inline cudaError_t freeMemory(size_t &bytes) {
+    size_t total = 0;
+    int device = 0;
+    cudaError_t e = cudaMemGetInfo(&bytes, &total);
+    if (e != cudaSuccess || (e = cudaGetDevice(&device)) != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(poolList().mutex);
+    for (DevPool *p : poolList().pools) {
+        std::lock_guard<std::mutex> poolLock(p->mutex);
+        if (p->device == device) bytes += p->keptBytes;
+    }
+    return e;
+}
 
 // Device buffer owned by a scene, renderer or batch, from its context's pool
 // where one is set.  Whoever frees it has waited for the work that uses it: the

@@ -1577,8 +1577,8 @@ rmd_status rmd_renderer_autotune(rmd_renderer *r, const rmd_render_settings *set
     // 3) paths in flight (queue sizes)
     uint32_t bestCap = cap0;
     for (uint32_t cap : caps) {
-        size_t freeB = 0, totalB = 0;
-        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess || pathPoolBytes(cap) > freeB / 2) continue;
+        size_t freeB = 0;
+        if (rmdhost::freeMemory(freeB) != cudaSuccess || pathPoolBytes(cap) > freeB / 2) continue;
         r->capacity = cap;
         if ((st = allocatePool(r)) != RMD_OK) return st;
         double ms;
@@ -2263,8 +2263,8 @@ rmd_status rmd_batch_autotune(rmd_batch *b, const rmd_render_settings *settings,
     b->traceBlocksPerSm = bestTb;
     uint32_t bestCap = cap0;
     for (uint32_t cap : caps) {
-        size_t freeB = 0, totalB = 0;
-        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess || pathPoolBytes(cap) > freeB / 2) continue;
+        size_t freeB = 0;
+        if (rmdhost::freeMemory(freeB) != cudaSuccess || pathPoolBytes(cap) > freeB / 2) continue;
         b->capacity = cap;
         if ((st = batchAllocatePool(b)) != RMD_OK) return st;
         double ms;

@@ -2,7 +2,7 @@
 side, on a device whose size the test sets)."""
 import pytest
 
-from host_runtime import OUT_OF_MEMORY, fake  # noqa: F401
+from host_runtime import OUT_OF_MEMORY, PATHS_DONE, fake  # noqa: F401
 from raymond_b200 import scenes
 from raymond_b200._abi import SceneDesc
 
@@ -92,3 +92,24 @@ def test_the_bound_holds_and_all_goes_with_the_context(fake):
     ctx.close()
     del scene
     assert fake.lib.fake_allocated() == before
+
+
+def test_autotune_counts_kept_memory_as_free(fake):
+    """Pools are tried if they fit into half of the free memory; blocks that contexts keep are free."""
+    api = fake.api
+    ctx = api.Context(0)
+    scene = api.Scene(ctx, DESC)
+    r = api.Renderer(scene, 16, 16, pool_size=1 << 16)
+    _full_device(fake, ctx).close()
+    tried = []
+
+    def see(name, ptr, size, stream):
+        if name == "cudaMalloc" and size > 1 << 24:
+            tried.append(size)
+        elif fake.is_counters(name, size):
+            fake.counter(ptr, PATHS_DONE).value = 1 << 40
+
+    with fake.on(see):
+        r.autotune(spp=1, max_depth=2)
+    assert len(tried) >= 2  # twice and four times the paths
+    r.close(), scene.close()
