@@ -40,7 +40,8 @@ inline cudaError_t loadLibrary(cudaLibrary_t *library, const void *code) {
 // no hole (2-3 ms for the tree's workspace and for the paths, in one of four
 // creations 40-1,200 ms); a kept block is handed out as it is.  Sizes below
 // 1 GiB are rounded up to an eighth of their power of two, so that a scene a
-// little larger than the one before takes the same blocks.  Any thread may
+// little larger than the one before takes the same blocks; a size that only fits
+// as it is gets such a block, which is not kept.  Any thread may
 // allocate and free.  Kept blocks are free memory to every allocation of the
 // library: one that finds the device full has all contexts of the device give
 // theirs back (withKeptMemory).
@@ -50,6 +51,7 @@ struct DevPool {
     std::mutex mutex;
     std::multimap<size_t, void *> kept;  // free blocks by size
     size_t keptBytes = 0;
+    std::set<void *> unrounded;  // blocks in use that are smaller than their rounded size
     explicit DevPool(int device);
     ~DevPool();
     DevPool(const DevPool &) = delete;
@@ -73,12 +75,21 @@ struct DevPool {
                 return cudaSuccess;
             }
         }
-        return deviceAlloc(p, size);
+        cudaError_t e = deviceAlloc(p, size);
+        if (e == cudaErrorMemoryAllocation && n < size && (e = deviceAlloc(p, n)) == cudaSuccess) {
+            std::lock_guard<std::mutex> lock(mutex);
+            unrounded.insert(*p);
+        }
+        return e;
     }
     // takes back a block that alloc gave for n bytes; no work may use it any more
     void free(void *p, size_t n) {
         const size_t size = rounded(n);
         std::lock_guard<std::mutex> lock(mutex);
+        if (unrounded.erase(p)) {
+            cudaFree(p);
+            return;
+        }
         kept.emplace(size, p);
         keptBytes += size;
         while (keptBytes > kMemoryKept) {  // the largest go first: small ones are asked for on every read-out
