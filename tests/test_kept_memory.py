@@ -119,17 +119,17 @@ def test_a_size_that_fits_only_unrounded(fake):
     """Sizes are rounded up to make kept blocks useful again, not at the price of an allocation that fits."""
     api = fake.api
     scene = api.Scene(api.Context(0), DESC)
-    paths, more = 2_000_000, 2_020_000  # 520 and 525 MB, both rounded up to 537
+    paths, more = 2_000_000, 2_020_000  # 264 bytes each: 528 and 533 MB, both rounded up to 537
     asked = []
 
     def see(name, ptr, size, stream):
         if name == "cudaMalloc" and size > 1 << 28:
             asked.append(size)
 
-    fake.lib.fake_set_capacity(fake.lib.fake_allocated() + 260 * paths + (2 << 20))
+    fake.lib.fake_set_capacity(fake.lib.fake_allocated() + 264 * paths + (2 << 20))
     api.Renderer(scene, 64, 64, pool_size=paths).close()
     fake.lib.fake_set_capacity(180 << 30)
     with fake.on(see):
         api.Renderer(scene, 64, 64, pool_size=more).close()
-    assert asked and asked[0] >= 260 * more  # not the smaller block
+    assert asked and asked[0] >= 264 * more  # not the smaller block
     scene.close()
