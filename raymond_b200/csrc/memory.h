@@ -5,6 +5,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <set>
 
 namespace rmdhost {
@@ -78,19 +79,30 @@ struct DevPool {
         cudaError_t e = deviceAlloc(p, size);
         if (e == cudaErrorMemoryAllocation && n < size && (e = deviceAlloc(p, n)) == cudaSuccess) {
             std::lock_guard<std::mutex> lock(mutex);
-            unrounded.insert(*p);
+            try {
+                unrounded.insert(*p);
+            } catch (const std::bad_alloc &) {
+                cudaFree(*p);
+                *p = nullptr;
+                return cudaErrorMemoryAllocation;
+            }
         }
         return e;
     }
     // takes back a block that alloc gave for n bytes; no work may use it any more
-    void free(void *p, size_t n) {
+    void free(void *p, size_t n) noexcept {
         const size_t size = rounded(n);
         std::lock_guard<std::mutex> lock(mutex);
         if (unrounded.erase(p)) {
             cudaFree(p);
             return;
         }
-        kept.emplace(size, p);
+        try {
+            kept.emplace(size, p);
+        } catch (const std::bad_alloc &) {  // objects free their buffers where nothing may be thrown
+            cudaFree(p);
+            return;
+        }
         keptBytes += size;
         while (keptBytes > kMemoryKept) {  // the largest go first: small ones are asked for on every read-out
             const auto largest = std::prev(kept.end());

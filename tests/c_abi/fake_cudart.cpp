@@ -6,11 +6,13 @@
 // first and can make it fail.
 #include <cuda_runtime_api.h>
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -101,11 +103,23 @@ Event *eventOf(cudaEvent_t e) {
         if (e_ != cudaSuccess) return e_;               \
     } while (0)
 
+std::atomic<int> g_newFails{0};  // how many of the next allocations by `new` fail
+
 }  // namespace
+
+void *operator new(size_t n) {
+    if (g_newFails > 0 && g_newFails-- > 0) throw std::bad_alloc();
+    void *p = std::malloc(n ? n : 1);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 extern "C" {
 
 // ------------------------------------------------------------- for the tests
+void fake_fail_new(int times) { g_newFails = times; }
 void fake_set_hook(Hook hook) {
     Lock lock(g_mutex);
     g_hook = hook;

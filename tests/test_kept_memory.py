@@ -1,5 +1,9 @@
 """A context's kept blocks and the allocations that find the device full (host
 side, on a device whose size the test sets)."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 
 from host_runtime import OUT_OF_MEMORY, PATHS_DONE, fake  # noqa: F401
@@ -133,3 +137,28 @@ def test_a_size_that_fits_only_unrounded(fake):
         api.Renderer(scene, 64, 64, pool_size=more).close()
     assert asked and asked[0] >= 264 * more  # not the smaller block
     scene.close()
+
+
+def test_host_memory_runs_out_while_a_block_is_kept(fake):
+    """A handle's destruction reports nothing, so it may not throw either (in a process of its own: it would abort)."""
+    code = f"""
+import sys
+from pathlib import Path
+sys.path[:0] = [{str(Path(__file__).parent)!r}, {str(Path(__file__).parent.parent)!r}]
+from host_runtime import FakeRuntime
+from test_kept_memory import DESC
+rt = FakeRuntime(Path({str(fake.path)!r}))
+scene = rt.api.Scene(rt.api.Context(0), DESC)
+before = rt.lib.fake_allocated()
+r = rt.api.Renderer(scene, 64, 64, pool_size=1 << 20)
+rt.lib.fake_fail_new(100)
+rt.lib.rmd_renderer_destroy(r.h)
+rt.lib.fake_fail_new(0)
+r.h = type(r.h)()
+assert rt.lib.fake_allocated() == before, (rt.lib.fake_allocated(), before)  # freed, as nothing could be kept
+rt.api.Renderer(scene, 64, 64, pool_size=1 << 20).close()
+scene.close()
+print("done")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
