@@ -1384,8 +1384,10 @@ cudaError_t GuideNet::allocate(cudaStream_t s) {
     if (!alloc(master, pb) || !alloc(adamM, pb) || !alloc(adamV, pb) || !alloc(grad, pb) ||
         !alloc(scratch, 64 * sizeof(float)) || !alloc(partials, (size_t)GUIDE_TRAIN_MAX_BLOCKS * (pb + sizeof(float))) ||
         !alloc(weightsBf16, GUIDE_WEIGHTS * sizeof(uint16_t)) || !alloc(bf16Index, GUIDE_PARAMS * sizeof(int)) ||
-        !alloc(image, kImageBytes) || !alloc(imageIndex, GUIDE_PARAMS * sizeof(int)))
+        !alloc(image, kImageBytes) || !alloc(imageIndex, GUIDE_PARAMS * sizeof(int))) {
+        release();  // all or nothing: allocated() looks at one of them
         return e;
+    }
     std::vector<int> idx(GUIDE_PARAMS, -1), img(GUIDE_PARAMS, -1);
     int wOff[4], bOff[4], qOff[4];
     layout(wOff, bOff, qOff);
@@ -1402,9 +1404,9 @@ cudaError_t GuideNet::allocate(cudaStream_t s) {
             }
     if ((e = cudaMemcpyAsync(bf16Index, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(imageIndex, img.data(), img.size() * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return e;
-    return rmdGuideConfigure();
+        (e = cudaStreamSynchronize(s)) != cudaSuccess || (e = rmdGuideConfigure()) != cudaSuccess)
+        release();
+    return e;
 }
 
 cudaError_t GuideNet::setParams(const float *host, cudaStream_t s) {

@@ -1005,11 +1005,11 @@ static rmd_status guideBuffers(GuideState &g, uint32_t capacity, Counters *count
         g.finRec.release();
         g.shRec.release();
     }
-    if (g.settings.sampling && !g.mixtures.ptr) {
+    if (g.settings.sampling && !g.features.ptr) {  // the last of these: the earlier ones may be left from a full device
         RMD_CUDA(g.mixtures.alloc(((size_t)capacity + 31u) / 32u * 32u * sizeof(GuideMixture)));
         RMD_CUDA(g.features.alloc((size_t)capacity * sizeof(uint4)));
     }
-    if (g.settings.training && !g.rec.ptr) {
+    if (g.settings.training && !g.shRec.ptr) {
         RMD_CUDA(g.rec.alloc((size_t)capacity * 2 * 4 * sizeof(float4)));
         RMD_CUDA(g.finRec.alloc((size_t)capacity * 4 * sizeof(float4)));
         RMD_CUDA(g.shRec.alloc((size_t)capacity * 2 * sizeof(float4)));

@@ -162,3 +162,49 @@ print("done")
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
     assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("kind", ["renderer", "batch"])
+def test_a_guide_that_ran_out_of_memory_is_set_up_whole(fake, kind):
+    """Wherever set_guide runs out of memory, the next call allocates what is missing: no kernel gets a null buffer."""
+    api = fake.api
+
+    def make():
+        ctx = api.Context(0)  # nothing kept
+        if kind == "batch":
+            return api.Batch(ctx, [DESC], [{"scene": 0, "width": 8, "height": 8}], pool_size=1 << 12)
+        return api.Renderer(api.Scene(ctx, DESC), 8, 8, pool_size=1 << 12)
+
+    def set_guide(x, fail_from):
+        calls = 0
+
+        def see(name, ptr, size, stream):
+            nonlocal calls
+            if name == "cudaMalloc":
+                calls += 1
+                return OUT_OF_MEMORY if fail_from <= calls else 0
+
+        with fake.on(see):
+            x.set_guide(sampling=True, training=True, replay_records=1 << 12)
+        return calls
+
+    def begin():
+        x = make()
+        with pytest.raises(api.RmdError, match="OUT_OF_MEMORY"):
+            set_guide(x, 1)  # gives back what the context keeps
+        return x, fake.lib.fake_allocated()
+
+    x, base = begin()
+    calls = set_guide(x, 1000)
+    whole = fake.lib.fake_allocated() - base
+    x.close()
+    del x  # with its scene and context
+    assert calls >= 16
+    for k in range(1, calls + 1):
+        x, base = begin()
+        with pytest.raises(api.RmdError, match="OUT_OF_MEMORY"):
+            set_guide(x, k)
+        set_guide(x, 1000)
+        assert fake.lib.fake_allocated() - base == whole, k
+        x.close()
+        del x
