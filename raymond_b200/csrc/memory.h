@@ -46,6 +46,12 @@ inline cudaError_t loadLibrary(cudaLibrary_t *library, const void *code) {
 // allocate and free.  Kept blocks are free memory to every allocation of the
 // library: one that finds the device full has all contexts of the device give
 // theirs back (withKeptMemory).
+//
+// A context's blocks are used on its stream alone, so what is enqueued on a block
+// comes after all that its last owner enqueued, waited for or not (cudaFree waits
+// by itself).  No wait stands in an object's end: it would have to be for a stream
+// or a device that another thread may be capturing on, which refuses it and spoils
+// the capture.
 struct DevPool {
     static constexpr size_t kMemoryKept = size_t(2) << 30;
     const int device;
@@ -89,7 +95,7 @@ struct DevPool {
         }
         return e;
     }
-    // takes back a block that alloc gave for n bytes; no work may use it any more
+    // takes back a block that alloc gave for n bytes
     void free(void *p, size_t n) noexcept {
         const size_t size = rounded(n);
         std::lock_guard<std::mutex> lock(mutex);
@@ -163,10 +169,9 @@ inline cudaError_t freeMemory(size_t &bytes) {
 }
 
 // Device buffer owned by a scene, renderer or batch, from its context's pool
-// where one is set.  Whoever frees it has waited for the work that uses it: the
-// pool does not.  A new one may hold what a block's last owner left, so it is
-// cleared and filled on the stream that uses it (the legacy stream is not
-// ordered with a context's).
+// where one is set.  A new one may hold what a block's last owner left, so it is
+// cleared and filled on the context's stream (the legacy stream is not ordered
+// with it).
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;

@@ -101,16 +101,6 @@ struct HostMat4 {
 
 }  // namespace
 
-// Waits for all work of `device` (an object's last, so its memory may go back to
-// the pool), whichever device the calling thread has current.
-static void waitForDevice(int device) {
-    int current = device;
-    if (device < 0 || cudaGetDevice(&current) != cudaSuccess) return;
-    if (device != current) cudaSetDevice(device);
-    cudaDeviceSynchronize();
-    if (device != current) cudaSetDevice(current);
-}
-
 struct rmd_context {
     int device = 0;
     int smCount = 148;
@@ -122,7 +112,6 @@ struct rmd_context {
 
 struct rmd_scene {
     rmd_context *ctx = nullptr;
-    int device = -1;  // set with the first work
     Context dctx{};  // device view
     DevBuf vertices, normals, texcoords, faces, instances, lightFaces, envPdfs, envMipmap;
     DevBuf areaLights, pointLights, sunLights, spotLights, shapeLights;
@@ -150,7 +139,6 @@ struct rmd_scene {
             b->from = p;
     }
     ~rmd_scene() {
-        waitForDevice(device);
         for (auto &kv : variants) rmdhost::unloadModule(*kv.second);
         if (ownsModule) rmdhost::unloadModule(jit);
     }
@@ -173,7 +161,6 @@ struct GuideState {
 };
 
 struct rmd_renderer {
-    int device = -1;  // set with the first work
     rmd_scene *scene = nullptr;
     uint32_t width = 0, height = 0, capacity = 0;
     // launch choices (rmd_renderer_autotune)
@@ -194,7 +181,6 @@ struct rmd_renderer {
     std::vector<int> stageOf;              // stage of the interval that ends at each event
     GuideState guide;  // learned path guiding
     ~rmd_renderer() {
-        waitForDevice(device);
         if (hostCounters) cudaFreeHost(hostCounters);
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
@@ -218,7 +204,6 @@ struct rmd_renderer {
 // stage), the whole render one CUDA-graph launch whose while loop the device
 // drives.
 struct rmd_batch {
-    int device = -1;  // set with the first work
     rmd_context *ctx = nullptr;
     std::vector<std::unique_ptr<rmd_scene>> scenes;
     rmdhost::JitModule jit;  // the merged material module of all scenes (batch shading kernel)
@@ -245,7 +230,6 @@ struct rmd_batch {
     cudaGraphExec_t graphExec = nullptr;
     std::vector<uint64_t> graphKey;
     ~rmd_batch() {
-        waitForDevice(device);
         if (graphExec) cudaGraphExecDestroy(graphExec);
         if (graph) cudaGraphDestroy(graph);
         if (hostCounters) cudaFreeHost(hostCounters);
@@ -499,7 +483,6 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
                                  const rmd_texture *textures, int numTextures) {
     cudaStream_t st = ctx->stream;
     s->ctx = ctx;
-    s->device = ctx->device;
     s->takeMemoryFrom(ctx->memory);
     s->numSurface = d->num_surface_materials;
     s->numLight = d->num_light_materials;
@@ -1123,7 +1106,6 @@ rmd_status rmd_renderer_create(rmd_scene *scene, uint32_t width, uint32_t height
     r->scene = scene;
     // not the film, whose address callers get (rmd_film_device)
     for (DevBuf *b : {&r->pool, &r->counters, &r->resolve, &r->film64}) b->from = scene->ctx->memory;
-    r->device = scene->ctx->device;
     r->guide.takeMemoryFrom(scene->ctx->memory);
     r->dctx = scene->dctx;
     r->shade = scene->jit.shade;
@@ -1836,7 +1818,6 @@ rmd_status rmd_batch_create(rmd_context *ctx, const rmd_scene_desc *descs, int32
     auto b = std::make_unique<rmd_batch>();
     b->ctx = ctx;
     for (DevBuf *m : {&b->viewTable, &b->pool, &b->counters, &b->resolve, &b->film, &b->film64}) m->from = ctx->memory;
-    b->device = ctx->device;
     b->guide.takeMemoryFrom(ctx->memory);
     b->useGraph = !(flags & RMD_BATCH_NO_GRAPH);
     // one material module for all scenes: their materials concatenated
