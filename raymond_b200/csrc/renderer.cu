@@ -229,9 +229,11 @@ struct rmd_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
     std::vector<uint64_t> graphKey;
+    cudaStream_t captureStream = nullptr;  // not the context's: other objects' work there would be captured with it
     ~rmd_batch() {
         if (graphExec) cudaGraphExecDestroy(graphExec);
         if (graph) cudaGraphDestroy(graph);
+        if (captureStream) cudaStreamDestroy(captureStream);
         if (hostCounters) cudaFreeHost(hostCounters);
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
@@ -2041,13 +2043,15 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
             RMD_CUDA(cudaGraphAddNode(&loop, b->graph, nullptr, 0, &cp));
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             // the body: two iterations (both parities) and the condition kernel
-            RMD_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+            if (!b->captureStream) RMD_CUDA(cudaStreamCreateWithFlags(&b->captureStream, cudaStreamNonBlocking));
+            const cudaStream_t cs = b->captureStream;
+            RMD_CUDA(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             cudaError_t ce = cudaSuccess;
             for (uint32_t cur = 0; cur < 2 && ce == cudaSuccess; cur++)
-                ce = batchEnqueueIteration(b, pool, fp, sp, net, cur, allPaths, st);
-            if (ce == cudaSuccess) ce = rmdLaunchLoopCondition(cnt, handle, 2, (uint32_t)maxIters, st);
+                ce = batchEnqueueIteration(b, pool, fp, sp, net, cur, allPaths, cs);
+            if (ce == cudaSuccess) ce = rmdLaunchLoopCondition(cnt, handle, 2, (uint32_t)maxIters, cs);
             cudaGraph_t captured = nullptr;
-            cudaError_t endErr = cudaStreamEndCapture(st, &captured);
+            cudaError_t endErr = cudaStreamEndCapture(cs, &captured);
             RMD_CUDA(ce);
             RMD_CUDA(endErr);
             RMD_CUDA(rmdhost::withKeptMemory([&] { return cudaGraphInstantiate(&b->graphExec, b->graph, 0); }));

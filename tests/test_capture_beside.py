@@ -77,3 +77,29 @@ def test_batches_beside_renderers_that_go(gpu_ctx):
     assert not failed and made[0] > 3
     for d, f in films:
         np.testing.assert_array_equal(f, alone[d])
+
+
+def test_a_batch_captures_on_a_stream_of_its_own(fake):
+    """What other threads enqueue on the context's stream meanwhile is not captured with it."""
+    api = fake.api
+    desc = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
+    ctx = api.Context(0)
+    b = api.Batch(ctx, [desc], VIEWS, pool_size=2048)
+    r = api.Renderer(api.Scene(ctx, desc), 24, 16, pool_size=2048)
+    captured, launched, during = [], [], []
+
+    def see(name, ptr, size, stream):
+        if name == "cudaStreamBeginCaptureToGraph":
+            captured.append(stream)
+        elif name == "cudaGraphLaunch":
+            launched.append(stream)
+        elif name == "launch:rmd_shade" and captured and not launched:
+            during.append(stream)
+            r.reset()  # clears its film on the context's stream and waits for it
+
+    with fake.on(see):
+        b.render(spp=1, max_depth=2, first_sample=0)
+        b.render(spp=1, max_depth=3, first_sample=0)
+    assert len(captured) == len(launched) == 2 and during and set(during) <= set(captured)
+    assert not set(captured) & set(launched)
+    r.close(), b.close()
