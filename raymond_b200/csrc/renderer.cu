@@ -674,12 +674,14 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     const auto buildStart = std::chrono::steady_clock::now();
     s->bvhStats.builder = ctx->bvhBuilder;
     if (ctx->bvhBuilder == RMD_BVH_GPU) {
+        if (numTriangles > rmdhost::kGpuBvhMaxTriangles)  // before their memory, and the flattening's 32-bit indexes
+            return fail(RMD_ERROR_INVALID_ARGUMENT, "device BVH build: the device BVH builder takes at most 2^24 triangles");
         DevBuf world;  // three vertices, instance and primitive per triangle, then the bounds
         world.from = ctx->memory;
         RMD_CUDA(world.alloc(numTriangles * 44 + 6 * sizeof(uint32_t)));
         float *w0 = world.as<float>(), *w1 = w0 + 3 * numTriangles, *w2 = w1 + 3 * numTriangles;
         uint32_t *wInst = reinterpret_cast<uint32_t *>(w2 + 3 * numTriangles), *wPrim = wInst + numTriangles;
-        const uint32_t n = (uint32_t)std::min<size_t>(numTriangles, 0xffffffffu);
+        const uint32_t n = (uint32_t)numTriangles;
         if (n) {
             float bounds[6];
             RMD_CUDA(rmdLaunchFlatten(s->vertices.as<float4>(), s->faces.as<uint4>(), s->instances.as<PerInstanceData>(),

@@ -205,8 +205,10 @@ cudaError_t cudaMalloc(void **p, size_t n) {
     ASK("cudaMalloc", nullptr, n);
     Lock lock(g_mutex);
     if (g_bytes + n > g_capacity) return result(cudaErrorMemoryAllocation);
-    *p = std::calloc(1, n ? n : 1);
-    g_blocks[*p] = n;
+    void *block = std::calloc(1, n ? n : 1);
+    if (!block) return result(cudaErrorMemoryAllocation);
+    *p = block;
+    g_blocks[block] = n;
     g_bytes += n;
     return cudaSuccess;
 }
