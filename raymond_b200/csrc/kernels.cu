@@ -514,12 +514,12 @@ __global__ void k_rotate_triangles(const float4 *__restrict__ in, float4 *__rest
 // ------------------------------------------------------------- scene building
 // The meshes' packed arrays as the shading kernels read them: positions and
 // normals on 16 bytes, faces with their material.
-__global__ void k_pack_mesh(const float *__restrict__ pos, const float *__restrict__ nrm, uint32_t numVertices,
-                            const uint32_t *__restrict__ idx, const uint16_t *__restrict__ mat, uint32_t numFaces,
+__global__ void k_pack_mesh(const float *__restrict__ pos, const float *__restrict__ nrm, size_t numVertices,
+                            const uint32_t *__restrict__ idx, const uint16_t *__restrict__ mat, size_t numFaces,
                             float4 *__restrict__ vertices, float4 *__restrict__ normals, uint4 *__restrict__ faces) {
-    const uint32_t n = max(numVertices, numFaces);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const size_t k = 3 * (size_t)i;
+    const size_t n = max(numVertices, numFaces), step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+        const size_t k = 3 * i;
         if (i < numVertices) {
             vertices[i] = make_float4(pos[k], pos[k + 1], pos[k + 2], 0.0f);
             normals[i] = make_float4(nrm[k], nrm[k + 1], nrm[k + 2], 0.0f);
@@ -641,12 +641,12 @@ cudaError_t rmdLaunchDebugPrng(uint32_t mode, uint64_t a, uint64_t b, int n, flo
     k_debug_prng<<<1, 1, 0, s>>>(mode, a, b, n, out);
     return cudaGetLastError();
 }
-cudaError_t rmdLaunchPackMesh(const float *pos, const float *nrm, uint32_t numVertices, const uint32_t *idx,
-                              const uint16_t *mat, uint32_t numFaces, float4 *vertices, float4 *normals, uint4 *faces,
+cudaError_t rmdLaunchPackMesh(const float *pos, const float *nrm, size_t numVertices, const uint32_t *idx,
+                              const uint16_t *mat, size_t numFaces, float4 *vertices, float4 *normals, uint4 *faces,
                               cudaStream_t s) {
-    const uint32_t n = std::max(numVertices, numFaces);
+    const size_t n = std::max(numVertices, numFaces);
     if (n == 0) return cudaSuccess;
-    k_pack_mesh<<<std::min<uint32_t>((n + 255) / 256, 148u * 16u), 256, 0, s>>>(pos, nrm, numVertices, idx, mat, numFaces,
+    k_pack_mesh<<<(unsigned)std::min<size_t>((n + 255) / 256, 148u * 16u), 256, 0, s>>>(pos, nrm, numVertices, idx, mat, numFaces,
                                                                              vertices, normals, faces);
     return cudaGetLastError();
 }

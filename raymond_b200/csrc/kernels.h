@@ -34,8 +34,8 @@ cudaError_t rmdLaunchFilmResolve(const float4 *film, const double *film64, int f
                                  cudaStream_t s);
 cudaError_t rmdLaunchDebugPrng(uint32_t mode, uint64_t a, uint64_t b, int n, float *out, cudaStream_t s);
 // the packed mesh arrays as the shading kernels read them
-cudaError_t rmdLaunchPackMesh(const float *pos, const float *nrm, uint32_t numVertices, const uint32_t *idx,
-                              const uint16_t *mat, uint32_t numFaces, float4 *vertices, float4 *normals, uint4 *faces,
+cudaError_t rmdLaunchPackMesh(const float *pos, const float *nrm, size_t numVertices, const uint32_t *idx,
+                              const uint16_t *mat, size_t numFaces, float4 *vertices, float4 *normals, uint4 *faces,
                               cudaStream_t s);
 // world-space triangles of all instances (n in all) and their bounds (host; min xyz, max xyz), waiting for them
 cudaError_t rmdLaunchFlatten(const float4 *vertices, const uint4 *faces, const rmd::PerInstanceData *instances,

@@ -20,6 +20,7 @@
 #include "codegen.h"
 #include "drive.h"
 #include "exr.h"
+#include "face_runs.h"
 #include "device/wavefront.cuh"
 #include "guide.h"
 #include "jit.h"
@@ -513,18 +514,16 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     // count: none).  All cores go over the shapes' runs of 64 k faces; the
     // device packs the arrays.  One thread, appending to vectors element by
     // element, took 20-30 ms for 852 k faces.
-    constexpr uint32_t kRun = 1u << 16;
-    std::vector<std::pair<int, uint32_t>> runs;  // shape, first face
-    for (int si = 0; si < checked; si++)
-        for (uint32_t f = 0; f == 0 || f < d->shapes[si].num_faces; f += kRun) runs.push_back({si, f});
+    std::vector<rmdhost::FaceRun> runs;
+    for (int si = 0; si < checked; si++) rmdhost::appendFaceRuns(runs, si, d->shapes[si].num_faces);
     std::vector<uint32_t> badFace(runs.size(), 0xffffffffu);
     std::vector<uint8_t> emits(runs.size(), 0);
 #pragma omp parallel for schedule(dynamic, 1)
     for (int64_t k = 0; k < (int64_t)runs.size(); k++) {
-        const rmd_shape &sh = d->shapes[runs[k].first];
-        const uint32_t begin = runs[k].second, end = std::min(sh.num_faces, begin + kRun);
+        const rmd_shape &sh = d->shapes[runs[k].shape];
+        const uint32_t begin = runs[k].begin, end = runs[k].end;
         if (begin == 0) {
-            ShapeInfo &info = shapes[runs[k].first];
+            ShapeInfo &info = shapes[runs[k].shape];
             for (int c = 0; c < 3; c++) {
                 info.boundsMin[c] = INFINITY;
                 info.boundsMax[c] = -INFINITY;
@@ -549,7 +548,7 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
         }
     }
     for (size_t k = 0; k < runs.size(); k++) {
-        const int si = runs[k].first;
+        const int si = runs[k].shape;
         if (badFace[k] != 0xffffffffu) {
             const uint32_t *ix = d->shapes[si].indices + 3 * (size_t)badFace[k], n = d->shapes[si].num_vertices;
             const bool vertex = ix[0] >= n || ix[1] >= n || ix[2] >= n;
@@ -586,9 +585,9 @@ static rmd_status buildSceneData(rmd_context *ctx, const rmd_scene_desc *d, rmd_
     RMD_CUDA(s->faces.alloc(numFaces * sizeof(uint4)));
     const unsigned char *devPos = staged.as<unsigned char>();
     RMD_CUDA(rmdLaunchPackMesh(reinterpret_cast<const float *>(devPos), reinterpret_cast<const float *>(devPos + posBytes),
-                               (uint32_t)numVertices, reinterpret_cast<const uint32_t *>(devPos + 2 * posBytes + uvBytes),
+                               numVertices, reinterpret_cast<const uint32_t *>(devPos + 2 * posBytes + uvBytes),
                                reinterpret_cast<const uint16_t *>(devPos + 2 * posBytes + uvBytes + idxBytes),
-                               (uint32_t)numFaces, s->vertices.as<float4>(), s->normals.as<float4>(),
+                               numFaces, s->vertices.as<float4>(), s->normals.as<float4>(),
                                s->faces.as<uint4>(), st));
     if (uvBytes)
         RMD_CUDA(cudaMemcpyAsync(s->texcoords.ptr, devPos + 2 * posBytes, uvBytes, cudaMemcpyDeviceToDevice, st));

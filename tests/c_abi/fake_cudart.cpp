@@ -78,14 +78,16 @@ void finishAll() {
     g_legacy.done = g_legacy.enqueued;
     for (auto &s : g_streams) s.first->done = s.first->enqueued;
 }
-cudaError_t launch(const void *kernel, cudaStream_t s) {
+// the hook gets the grid's blocks as the size
+cudaError_t launch(const void *kernel, dim3 grid, cudaStream_t s) {
     std::string name = "launch:";
     {
         Lock lock(g_mutex);
         const auto it = kernels().find(kernel);
         name += it != kernels().end() ? it->second : "?";
     }
-    const cudaError_t e = ask(name.c_str(), kernel, 0, s);
+    const cudaError_t e = ask(name.c_str(), kernel, (size_t)grid.x * grid.y * grid.z, s);
+    if (grid.x == 0 || grid.y == 0 || grid.z == 0) return result(cudaErrorInvalidConfiguration);
     if (e == cudaSuccess) enqueue(s);
     return e;
 }
@@ -333,9 +335,9 @@ cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
 }
 
 // ------------------------------------------------------------- kernels, modules
-cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t s) { return launch(f, s); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) { return launch(f, c->stream); }
-cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t s) { return launch(f, s); }
+cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **, size_t, cudaStream_t s) { return launch(f, grid, s); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) { return launch(f, c->gridDim, c->stream); }
+cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3 grid, dim3, void **, size_t, cudaStream_t s) { return launch(f, grid, s); }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *, int, size_t) {
     *n = 4;
