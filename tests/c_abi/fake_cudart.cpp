@@ -52,6 +52,11 @@ std::map<const void *, std::string> &kernels() {
 
 using Lock = std::lock_guard<std::recursive_mutex>;
 
+constexpr size_t kArrayBytes = size_t(16) << 20;  // more than any __device__ array of the library
+void *scratchArray() {
+    static void *p = std::calloc(1, kArrayBytes);
+    return p;
+}
 Stream *of(cudaStream_t s) { return s ? reinterpret_cast<Stream *>(s) : &g_legacy; }
 cudaError_t result(cudaError_t e) {
     if (e != cudaSuccess) g_last = e;
@@ -126,6 +131,8 @@ void fake_set_hook(Hook hook) {
     Lock lock(g_mutex);
     g_hook = hook;
 }
+// clears the library's device arrays, as no kernel does
+void fake_clear_arrays(void) { std::memset(scratchArray(), 0, kArrayBytes); }
 // device memory there is, and how much of it is allocated
 void fake_set_capacity(size_t bytes) { g_capacity = bytes; }
 size_t fake_allocated(void) {
@@ -241,8 +248,7 @@ cudaError_t cudaMemGetInfo(size_t *free, size_t *total) {
     return cudaSuccess;
 }
 cudaError_t cudaGetSymbolAddress(void **p, const void *) {
-    static void *scratch = std::calloc(1, size_t(16) << 20);
-    *p = scratch;
+    *p = scratchArray();
     return cudaSuccess;
 }
 cudaError_t cudaMemset(void *p, int v, size_t n) {

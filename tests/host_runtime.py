@@ -52,6 +52,7 @@ class FakeRuntime:
         L.fake_set_capturing.argtypes = [C.c_void_p, C.c_int]
         L.fake_counters_layout.restype, L.fake_counters_layout.argtypes = C.c_size_t, [C.c_int]
         L.fake_set_hook.argtypes = [C.c_void_p]
+        L.fake_clear_arrays()
         self.layout = [L.fake_counters_layout(k) for k in range(5)]
 
     @contextlib.contextmanager
