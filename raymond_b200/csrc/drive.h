@@ -15,21 +15,22 @@ namespace rmdhost {
 // its grids need to cover); check(counters, iterations) returns whether the
 // render is over (done, or failed).
 //
-// The counters are read after every eighth iteration until every path has been
-// handed out and could have ended, and then after every second, each read
+// The counters are read after every sixteenth iteration until every path has
+// been handed out and could have ended, and then after every second, each read
 // looked at once the iterations up to the next are enqueued: the device never
 // waits for the host, for at most four empty iterations at the end, and a
-// device error ends a render of any length within 16 iterations.  (Reading them
-// after every fourth iteration and waiting left a gap of 10-20 us each time.)
-// `slots`: two Counters in pinned memory; `events`: two events.  On return the
-// last iterations may still run.
+// device error ends a render of any length within 32 iterations.  (Reading them
+// after every fourth iteration and waiting left a gap of 10-20 us each time; a
+// read breaks the overlap of two launches, 3-7 us: one more in the 10 iterations
+// of a 640 x 360 render cost 0.6 % of it.)  `slots`: two Counters in pinned
+// memory; `events`: two events.  On return the last iterations may still run.
 template <class Iterate, class Check>
 cudaError_t driveWavefront(const rmd::Counters *cnt, uint64_t numPaths, uint32_t capacity, rmd::Counters *slots,
                            cudaEvent_t *events, cudaStream_t st, Iterate iterate, Check check) {
     uint64_t it = 0, paths = std::min<uint64_t>(numPaths, capacity);
     const uint64_t handedOut = ((numPaths + capacity - 1) / capacity + 3) & ~uint64_t(1);
-    uint64_t next = std::min<uint64_t>(handedOut, 8);
-    for (uint32_t k = 0;; k++, next = next < handedOut ? std::min(handedOut, next + 8) : next + 2) {
+    uint64_t next = std::min<uint64_t>(handedOut, 16);
+    for (uint32_t k = 0;; k++, next = next < handedOut ? std::min(handedOut, next + 16) : next + 2) {
         cudaError_t e;
         for (; it < next; it++)
             if ((e = iterate((uint32_t)(it & 1u), paths)) != cudaSuccess) return e;
