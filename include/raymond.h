@@ -380,7 +380,8 @@ typedef struct rmd_renderer rmd_renderer;
 /* Device selection and stream.  Replaces MTLCreateSystemDefaultDevice and
  * the command queue of Renderer.init (Renderer.swift:319-325).  Device memory
  * that its scenes, renderers and batches free stays with the context for the
- * next ones, at most 2 GiB, until it is destroyed. */
+ * next ones, at most 2 GiB, until it and they are destroyed or the library
+ * finds the device full. */
 rmd_status rmd_context_create(int32_t device, rmd_context **out);
 void rmd_context_destroy(rmd_context *ctx);
 

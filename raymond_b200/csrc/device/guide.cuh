@@ -48,7 +48,9 @@ struct alignas(16) GuideMixture {
 constexpr uint32_t GUIDE_MIX_STRIDE = 32;  // 16-byte chunks between two chunks of one mixture
 // a mixture's first chunk, hit `q` in shading order: (q / 32) * 256 + q % 32
 // (2^29 hits, where it would leave 32 bits, are 64 GB of mixtures beside 140 GB
-// of paths)
+// of paths).  Written as q + 7 (q & ~31) and in 32 bits because the other forms
+// (64 bits; (q >> 5) * 256 + (q & 31)) had the compiler contract other
+// multiply-adds in some scenes' shading modules: films moved by an ulp.
 RMD_HD uint32_t guideMixtureAt(uint32_t q) { return q + 7u * (q & ~31u); }
 RMD_HD void storeMixture(uint4 *dst, const GuideMixture &m) {
 #pragma unroll

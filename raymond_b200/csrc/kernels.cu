@@ -294,8 +294,8 @@ __device__ __noinline__ void traceByGroups(const WideNode *__restrict__ sceneNod
 // slowest ray, and a group's steps are about four times shorter.
 //
 // B200, per render: 192 x 108 x 1 spp (20 k paths) traversal 0.33 -> 0.07 ms;
-// 1080p x 1 spp of the 852 k-triangle scene 2.71 -> 1.71 ms, most of it in the
-// last iterations; 1080p x 64 spp 83.0 -> 83.4 ms (bound by divergence and
+// 1080p x 1 spp of the 852 k-triangle scene 2.71 -> 1.74 ms (closest hits 1.11,
+// shadow rays 0.63), most of it in the last iterations; 1080p x 64 spp 83.0 -> 83.4 ms (bound by divergence and
 // issue there; 64 spilled bytes in the loop had cost 2.5 %).
 template <bool BATCH, bool CLOSEST, bool SHADOW>
 __global__ void __launch_bounds__(TRACE_THREADS, 8) k_trace(const WideNode *__restrict__ sceneNodes,
