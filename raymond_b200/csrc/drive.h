@@ -57,7 +57,9 @@ inline cudaError_t launchOverlapped(const void *kernel, int blocks, int threads,
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, kernel, args);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+    if (e != cudaSuccess) cudaGetLastError();  // the caller's to report, not the next launch check's
+    return e;
 }
 template <class... Params, class... Args>
 cudaError_t launchOverlapped(void (*kernel)(Params...), int blocks, int threads, cudaStream_t st, Args... values) {

@@ -1260,7 +1260,9 @@ static cudaError_t launchOverlapped(void (*kernel)(Params...), dim3 grid, dim3 b
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();  // the caller's to report, not the next launch check's
+    return e;
 }
 
 cudaError_t rmdLaunchGuideInfer(const Context &ctx, const PathPool &pool, Counters *cnt, uint32_t cur,

@@ -9,7 +9,7 @@ from raymond_b200._abi import SceneDesc
 W, H, SPP, POOL = 64, 48, 64, 64  # 3,072 pools of paths
 
 
-def _render(fake, call, see_counters):
+def _render(fake, call, see_counters, also=lambda *call: 0):
     api = fake.api
     desc = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
     ctx = api.Context(0)
@@ -33,6 +33,7 @@ def _render(fake, call, see_counters):
         elif fake.is_counters(name, size):
             fake.counter(ptr, ERRORS, 32).value = 0  # the kernel that clears them does nothing here
             see_counters(ptr, iterations[0])
+        return also(name, ptr, size, stream)
 
     with fake.on(see):
         run()
@@ -60,3 +61,20 @@ def test_the_end_is_seen_soon(fake, call, ends):
         fake.counter(ptr, PATHS_DONE).value = W * H * SPP if iterations >= ends else 0
 
     assert ends <= _render(fake, call, play) <= ends + 6
+
+
+@pytest.mark.parametrize("call", ["render", "guided", "noalloc", "batch"])
+def test_a_failed_launch_is_reported_once(fake, call):
+    """The error of a launch that fails is its call's; the next calls succeed."""
+    launches = 0
+
+    def see(name, ptr, size, stream):
+        nonlocal launches
+        if name.startswith("launch:"):
+            launches += 1
+            return 98 if launches == 6 else 0  # cudaErrorInvalidDeviceFunction
+
+    with pytest.raises(fake.api.RmdError, match="CUDA error 98"):
+        _render(fake, call, lambda ptr, iterations: None, also=see)
+    desc = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
+    fake.api.Scene(fake.api.Context(0), desc).close()
