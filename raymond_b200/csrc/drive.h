@@ -10,6 +10,18 @@
 
 namespace rmdhost {
 
+// Waits for a stream when a call returns early: an object's end does not wait,
+// so a call that fails leaves no work behind.  done(): the call has waited.
+struct WaitOnReturn {
+    cudaStream_t stream;
+    bool waits = true;
+    explicit WaitOnReturn(cudaStream_t s) : stream(s) {}
+    ~WaitOnReturn() {
+        if (waits) cudaStreamSynchronize(stream);
+    }
+    void done() { waits = false; }
+};
+
 // Enqueues iterations until `check` ends the loop.  iterate(cur, paths)
 // enqueues one iteration of parity cur with at most `paths` active paths (what
 // its grids need to cover); check(counters, iterations) returns whether the

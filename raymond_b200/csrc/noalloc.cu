@@ -131,6 +131,7 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
     const int tb = v.smCount * 8;
     const int rb = (int)std::min<uint32_t>((P + 255) / 256, (uint32_t)v.smCount * 8);
 
+    rmdhost::WaitOnReturn unfinished(st);
     if ((e = rmdLaunchFrameInit(pool, cnt, firstPath, firstPath + numPaths, st)) != cudaSuccess)
         return cudaFail(e, "frame init");
     const uint64_t maxIters = ((numPaths + P - 1) / P + 1) * ((uint64_t)s->max_depth + 1) + 16;
@@ -150,6 +151,7 @@ extern "C" rmd_status rmd_render_noalloc(rmd_scene *scene, const rmd_camera *cam
     };
     e = rmdhost::driveWavefront(cnt, numPaths, P, v.loop->counters, v.loop->events, st, iterate, check);
     if (e != cudaSuccess) return cudaFail(e, "wavefront");
+    unfinished.done();
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cudaFail(e, "synchronize");
     if (status != RMD_OK) return status;
     return RMD_OK;

@@ -1254,6 +1254,7 @@ rmd_status rmd_render(rmd_renderer *r, const rmd_render_settings *s) {
     uint64_t trainSteps = 0;
 
     enum { STAGE_FILM, STAGE_TRACE, STAGE_GUIDE, STAGE_SHADE, STAGE_SHADOW, STAGE_TRAIN, STAGES };
+    rmdhost::WaitOnReturn unfinished(st);
     RMD_CUDA(cudaEventRecord(r->ev[0], st));
     RMD_CUDA(rmdLaunchFrameInit(pool, cnt, firstPath, firstPath + numPaths, st));
     // every path needs at most max_depth iterations after it is generated and two to reach the film, and
@@ -1327,6 +1328,7 @@ rmd_status rmd_render(rmd_renderer *r, const rmd_render_settings *s) {
     }
     RMD_CUDA(cudaEventRecord(r->ev[1], st));
     RMD_CUDA(cudaEventSynchronize(r->ev[1]));
+    unfinished.done();
     if (status != RMD_OK) return status;
     float ms = 0;
     cudaEventElapsedTime(&ms, r->ev[0], r->ev[1]);
@@ -2017,6 +2019,7 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
     const uint64_t allPaths = std::min<uint64_t>(numPaths, b->capacity);
     if (maxIters > 0xffffffffull) return fail(RMD_ERROR_INVALID_ARGUMENT, "render too long for one call");
 
+    rmdhost::WaitOnReturn unfinished(st);
     RMD_CUDA(cudaEventRecord(b->ev[0], st));
     RMD_CUDA(rmdLaunchFrameInit(pool, cnt, firstPath, firstPath + numPaths, st));
     uint64_t iterations = 0, trainSteps = 0;
@@ -2097,13 +2100,11 @@ rmd_status rmd_batch_render(rmd_batch *b, const rmd_render_settings *s) {
                 if (e != RMD_OK) return e;
             }
         }
-        if (status != RMD_OK) {
-            cudaStreamSynchronize(st);
-            return status;
-        }
+        if (status != RMD_OK) return status;
     }
     RMD_CUDA(cudaEventRecord(b->ev[1], st));
     RMD_CUDA(cudaEventSynchronize(b->ev[1]));
+    unfinished.done();
     float ms = 0;
     cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
     const Counters &h = last;

@@ -78,3 +78,36 @@ def test_a_failed_launch_is_reported_once(fake, call):
         _render(fake, call, lambda ptr, iterations: None, also=see)
     desc = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
     fake.api.Scene(fake.api.Context(0), desc).close()
+
+
+@pytest.mark.parametrize("call", ["render", "guided", "trained", "noalloc", "batch", "graph"])
+def test_a_failed_call_leaves_no_work_behind(fake, call):
+    """When a launch fails, what was enqueued before has ended on return: the objects may go at once."""
+    api = fake.api
+    desc = SceneDesc(scenes.cornell(seed=1, envmap_exponent=2))
+    ctx = api.Context(0)
+    if call in ("batch", "graph"):
+        x = api.Batch(ctx, [desc], [{"scene": 0, "width": W, "height": H}], pool_size=POOL, graph=call == "graph")
+    else:
+        scene, film = api.Scene(ctx, desc), np.zeros((H, W, 4), np.float32)
+        x = api.Renderer(scene, W, H, pool_size=POOL)
+        if call in ("guided", "trained"):
+            x.set_guide(sampling=call == "guided", training=call == "trained")
+    streams, launches = set(), 0
+
+    def see(name, ptr, size, stream):
+        nonlocal launches
+        if stream:
+            streams.add(stream)
+        if name.startswith("launch:") or name == "cudaGraphLaunch":
+            launches += 1
+            if launches == (2 if call == "graph" else 12):
+                return 98  # cudaErrorInvalidDeviceFunction
+
+    with fake.on(see), pytest.raises(api.RmdError, match="CUDA error 98"):
+        if call == "noalloc":
+            api.render_noalloc(scene, desc.scene["camera"], W, H, film.ctypes.data, spp=SPP, first_sample=0, max_depth=4)
+        else:
+            x.render(spp=SPP, max_depth=4, first_sample=0)
+    assert streams and [fake.lib.fake_pending(s) for s in streams] == [0] * len(streams)
+    x.close()
