@@ -2,6 +2,7 @@
 first renders with new settings; a host program may at any time): a wait for the
 whole device is refused then and spoils the capture."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -70,7 +71,9 @@ def test_batches_beside_renderers_that_go(gpu_ctx):
     t = threading.Thread(target=objects)
     t.start()
     try:
-        films = [(d, render(d)) for _ in range(60) for d in (2, 3, 4, 5)]
+        films, until = [], time.monotonic() + 120  # the other thread may have to compile its module first
+        while (len(films) < 240 or made[0] < 4) and not failed and time.monotonic() < until:
+            films += [(d, render(d)) for d in (2, 3, 4, 5)]
     finally:
         stop.set()
         t.join()

@@ -1,5 +1,6 @@
 """Contexts made while rmd_render_noalloc renders."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -89,7 +90,9 @@ def test_contexts_beside_a_render(gpu_ctx):
     t = threading.Thread(target=contexts)
     t.start()
     try:
-        films = [render() for _ in range(300)]
+        films, until = [], time.monotonic() + 60
+        while (len(films) < 300 or made[0] < 20) and not failed and time.monotonic() < until:
+            films.append(render())
     finally:
         stop.set()
         t.join()
